@@ -13,14 +13,24 @@ static __device__ __forceinline__ bool image_culled(const Params& P, int x, int 
     return lay_texel(P.img.dt[P.img.cur], P, x, y) > (float)P.distTransCull;
 }
 
+// The wrap of an angle difference beyond +-pi/2 (:430-434), which the
+// reference forms in double: theta > M_PI_2 exactly if theta >= the float
+// above it, and theta - M_PI in float, in two parts, rounds as the double
+// difference does for every float from pi/2 up to 7.
+static __device__ __forceinline__ float fold_angle(float theta) {
+    const float pio2 = 0x1.921fb6p+0f, pi_hi = 0x1.921fb6p+1f, pi_lo = -0x1.777a5cp-24f;
+    const float a = fabsf(theta);
+    if (!(a >= pio2)) return theta;
+    if (a > 7.0f) return theta > 0.0f ? (float)((double)theta - 3.14159265358979323846) : (float)(3.14159265358979323846 + (double)theta);
+    const float r = (a - pi_hi) - pi_lo;
+    return theta > 0.0f ? r : -r;
+}
+
 // screenToExemplarAngle, :425-436
 static __device__ __forceinline__ float screen_to_exemplar_angle(const Params& P, int x, int y, float ex, float ey,
                                                           int layer) {
     if (P.orientationEnabled) {
-        float theta = ex_point_orient(P.ex, ex, ey, layer) - lvl_texel(P.img.orient, x, y);
-        if ((double)theta > 1.57079632679489661923) return (float)((double)theta - 3.14159265358979323846);
-        if ((double)theta < -1.57079632679489661923) return (float)(3.14159265358979323846 + (double)theta);
-        return theta;
+        return fold_angle(ex_point_orient(P.ex, ex, ey, layer) - lvl_texel(P.img.orient, x, y));
     }
     return 0.0f;
 }
@@ -310,6 +320,9 @@ static __device__ float test_offset(const Params& P, int x, int y, const Patch& 
 // calculatePropagateOffset, :956-982 (pixelWrap with the level-0 size,
 // cudaImageBuffer.h:81-87)
 static __device__ __forceinline__ size_t pixel_wrap_index(const Params& P, int tx, int ty) {
+    // (inside the image the wrap is the identity: tx / W < 1 and tx is exact)
+    if ((unsigned)tx < (unsigned)P.W && (unsigned)ty < (unsigned)P.H && P.W < (1 << 24) && P.H < (1 << 24))
+        return (size_t)ty * P.W + tx;
     int wx = (int)((float)tx - (float)P.W * floorf((float)tx / (float)P.W));
     int wy = (int)((float)ty - (float)P.H * floorf((float)ty / (float)P.H));
     return (size_t)wy * P.W + wx;

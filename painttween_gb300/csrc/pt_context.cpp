@@ -154,12 +154,26 @@ Params make_params(pt_ctx* c, int level) {
         P.earlyExit = nonneg ? 1 : 0;
     }
     if (P.r <= 4) {
-        // taps by descending weight (the weights as the kernels form them)
+        // (volatile: product and sum each rounded, as in the kernels)
+        volatile float sw = 0.0f;
+        for (int i = 0; i < 2 * P.r + 1; i++)
+            for (int j = 0; j < 2 * P.r + 1; j++) {
+                volatile float w = P.gauss[i] * P.gauss[j];
+                sw = sw + w;
+            }
+        P.sumW = sw;
+        // the 3 x 3 in the middle, then the others, each by descending weight
+        // (the weights as the kernels form them)
         const int n = 2 * P.r + 1, K = n * n;
         std::vector<std::pair<float, int>> order;
         for (int t = 0; t < K; t++) order.push_back(std::make_pair(P.gauss[t / n] * P.gauss[t % n], t));
-        std::stable_sort(order.begin(), order.end(),
-                         [](const std::pair<float, int>& a, const std::pair<float, int>& b) { return a.first > b.first; });
+        auto outer = [&](int t) { return std::abs(t / n - P.r) > 1 || std::abs(t % n - P.r) > 1; };
+        // (the middle tap before all, whatever the weights' ties)
+        auto rank = [&](int t) { return t == K / 2 ? 0 : outer(t) ? 2 : 1; };
+        std::stable_sort(order.begin(), order.end(), [&](const std::pair<float, int>& a, const std::pair<float, int>& b) {
+            const int ra = rank(a.second), rb = rank(b.second);
+            return ra != rb ? ra < rb : a.first > b.first;
+        });
         for (int k = 0; k < K; k++) P.tapOrder[k] = (uint8_t)order[k].second;
     }
     P.jitter = p.advectionJitter;
@@ -168,6 +182,11 @@ Params make_params(pt_ctx* c, int level) {
     P.orientationEnabled = p.orientationEnabled;
     P.lumShiftEnable = p.lumShiftEnable;
     P.distTransCull = p.distTransCull;
+    {
+        const double cull = (double)p.distTransCull * 1.25;  // (exact)
+        P.exCull = (float)cull;
+        if ((double)P.exCull > cull) P.exCull = std::nextafterf(P.exCull, -INFINITY);
+    }
     P.direction = p.direction;
     P.scatterSamples = p.scatterSamplesCount;
     P.colorspace = p.colorspace;
@@ -187,6 +206,7 @@ Params make_params(pt_ctx* c, int level) {
         P.ex.orient = c->ex->orient;
         P.ex.dt = c->ex->dt;
         P.ex.ids = c->ex->ids;
+        P.ex.flags = c->ex->flags;
         P.ex.w = c->ex->w;
         P.ex.h = c->ex->h;
         P.ex.ns = c->NS;
@@ -318,7 +338,8 @@ static pt_status refresh_textures(pt_ctx* c, ExLevel* L) {
 // after its planes were written
 pt_status refresh_interleaved(pt_ctx* c, ExLevel* L) {
     if (L->bo_stale && L->bo && L->base) {
-        LN(pt::launch_interleave_texels(L->base, L->out, L->bo, (size_t)L->w * L->h * c->NS, c->stream));
+        LN(pt::launch_interleave_texels(L->base, L->out, L->dt, L->bo, L->flags, (size_t)L->w * L->h * c->NS,
+                                        c->stream));
         L->bo_stale = false;
     }
     if (c->params.filterMode == PT_FILTER_TEXTURE) TRY(refresh_textures(c, L));
@@ -510,19 +531,18 @@ static bool plane_map(pt_ctx* c, const void* p, int pitch, int w, int h, int tw,
 }
 
 // the tensor maps of the planes a tiled kernel of mode tm stages
-static void tile_maps(pt_ctx* c, const Params& P, int tm, TileMaps* M) {
+static void tile_maps(pt_ctx* c, const Params& P, int tm, int tile_h, TileMaps* M) {
     memset(M, 0, sizeof(*M));
     M->err = c->tma_err;
     if (!c->use_tma || !c->tma_err) return;
-    const int tw = ptk::kTileW + 2 * P.r, th = ptk::kTileH + 2 * P.r;
+    const int tw = ptk::kTileW + 2 * P.r, th = tile_h + 2 * P.r;
     const Arr<float4>& ib = P.img.base[P.img.cur];
     bool ok = plane_map(c, ib.p, ib.w, P.lw, P.lh, tw, th, &M->base) &&
               plane_map(c, P.canvas, P.W, P.lw, P.lh, tw, th, &M->canvas);
     if (ok && tm) {
         const AdvView& A = P.adv[tm == 1 ? 0 : 1];
         ok = plane_map(c, A.base, P.W, P.lw, P.lh, tw, th, &M->pbase) &&
-             plane_map(c, A.out, P.W, P.lw, P.lh, tw, th, &M->pout) &&
-             plane_map(c, A.off.B, P.W, P.lw, P.lh, tw, th, &M->prec);
+             plane_map(c, A.out, P.W, P.lw, P.lh, tw, th, &M->pout);
     }
     M->on = ok ? 1 : 0;
 }
@@ -537,16 +557,21 @@ static void tile_maps(pt_ctx* c, const Params& P, int tm, TileMaps* M) {
 static std::mutex g_tune_mutex;
 static std::map<std::tuple<int, int, int, int, int>, int> g_tune;  // (device, shape) -> choice
 
-static std::tuple<int, int, int, int> tune_key(pt_ctx* c, const Params& P, int tm, int* blocks) {
+static int sm_count(pt_ctx* c) {
     if (!c->sm_count) {
         if (cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
             cudaGetLastError();
             c->sm_count = 152;
         }
     }
+    return c->sm_count;
+}
+
+static std::tuple<int, int, int, int> tune_key(pt_ctx* c, const Params& P, int tm, int* blocks) {
+    const int sms = sm_count(c);
     *blocks = ((P.lw + ptk::kTileW - 1) / ptk::kTileW) * ((P.lh + ptk::kTileH - 1) / ptk::kTileH);
     int cls = 0;
-    while (cls < 6 && 4 * (long long)*blocks > ((long long)c->sm_count << cls)) cls++;
+    while (cls < 6 && 4 * (long long)*blocks > ((long long)sms << cls)) cls++;
     return std::make_tuple(P.r, tm, P.ex.hw, cls);
 }
 
@@ -601,10 +626,10 @@ cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work,
     if (!tiled_usable(c)) return cudaSuccess;
     int tm = temporal_mode(c);
     if (P.r < 2 || P.r > 4) return cudaSuccess;
-    TileMaps M;
-    tile_maps(c, P, tm, &M);
     int probe = -1;
     const int wide = kind == 0 ? propagate_variant(c, P, tm, &probe) : 0;
+    TileMaps M;
+    tile_maps(c, P, tm, kind == 0 ? ptk::kPropH : ptk::kTileH, &M);
     int blocks = 0;
     pt_ctx::Tune* t = probe >= 0 ? &c->tune[tune_key(c, P, tm, &blocks)] : nullptr;
     if (t) cudaEventRecord(t->ev[2 * probe], c->stream);
@@ -991,13 +1016,14 @@ pt_status pt_initialize_exemplars(pt_ctx* c, int w, int h, int ns) {
     size_t n = (size_t)w * h * ns;
     if (n > c->ex_cap) {
         dfree_t(c, c->up_ex.base); dfree_t(c, c->up_ex.out); dfree_t(c, c->up_ex.bo);
-        dfree_t(c, c->up_ex.orient); dfree_t(c, c->up_ex.dt); dfree_t(c, c->up_ex.ids);
+        dfree_t(c, c->up_ex.orient); dfree_t(c, c->up_ex.dt); dfree_t(c, c->up_ex.ids); dfree_t(c, c->up_ex.flags);
         TRY(dalloc_t(c, &c->up_ex.base, n));
         TRY(dalloc_t(c, &c->up_ex.out, n));
         TRY(dalloc_t(c, &c->up_ex.bo, 2 * n));
         TRY(dalloc_t(c, &c->up_ex.orient, n));
         TRY(dalloc_t(c, &c->up_ex.dt, n));
         TRY(dalloc_t(c, &c->up_ex.ids, n));
+        TRY(dalloc_t(c, &c->up_ex.flags, (size_t)2));
         c->ex_cap = n;
     }
     c->up_ex.w = w;
@@ -1107,6 +1133,7 @@ pt_status pt_upload_image_float(pt_ctx* c, int level, int layer, const float* da
         if (!c->ex || c->ex != &c->up_ex || w != c->up_ex.w || h != c->up_ex.h || style < 0 || style >= c->NS)
             return fail(c, PT_ERR_INVALID, "exemplar upload does not match pt_initialize_exemplars");
         float* dst = (layer == PT_LAYER_EXEMPLAR_ORIENTATION ? c->up_ex.orient : c->up_ex.dt) + n * style;
+        if (layer == PT_LAYER_EXEMPLAR_DIST_TRANS) c->up_ex.bo_stale = true;
         return h2d(c, dst, data, n * sizeof(float));
     }
     if (level < 0 || w != (c->W >> level) || h != (c->H >> level))

@@ -78,6 +78,7 @@ struct ExLevel {  // one exemplar pyramid level, all styles (base and output pla
     float* orient = nullptr;
     float* dt = nullptr;
     int* ids = nullptr;
+    int* flags = nullptr;  // ExView::flags, rebuilt with `bo`
     int w = 0, h = 0;
     int transparent = -1;  // -1 unknown, 0/1
 };

@@ -434,6 +434,23 @@ __device__ __forceinline__ float ex_sample_out_alpha(const ExView& e, float u, f
     return bl1(b, __ldg(r0 + 4 * b.x0 + 3), __ldg(r0 + 4 * b.x1 + 3),
                __ldg(r1 + 4 * b.x0 + 3), __ldg(r1 + 4 * b.x1 + 3));
 }
+// What the exemplar level's texels can do (k_interleave_texels): whether any
+// output alpha is below 0.995, so that a filtered one may be below
+// kAlphaThreshold, and whether any distance transform texel is above `cull`.
+__device__ __forceinline__ bool exemplar_transparent(const ExView& e) { return __ldg(e.flags) != 0; }
+__device__ __forceinline__ bool exemplar_culls(const ExView& e, float cull) {
+    return __int_as_float(__ldg(e.flags + 1)) > cull;
+}
+// the output alpha of the tiled kernels (sample2's fetch with HW)
+template <int HW>
+__device__ __forceinline__ float ex_out_alpha(const ExView& e, float u, float v, int layer) {
+    if (HW) {
+        u = fminf(fmaxf(u, 0.0f), (float)(e.w - 1));
+        v = fminf(fmaxf(v, 0.0f), (float)(e.h - 1));
+        return tex2DLayered<float4>(e.tout, u + 0.5f, v + 0.5f, ex_layer(e, layer)).w;
+    }
+    return ex_sample_out_alpha(e, u, v, layer);
+}
 // the mask of keyframe layer `key` at pixel (x, y): the key's output alpha
 // (PYRAMID_FETCH_LAYER(gExemplarOutput, x, y, keyIndex)); -1 without a key
 __device__ __forceinline__ float keymask_alpha(const ExView& e, int x, int y, int key) {

@@ -253,7 +253,7 @@ static pt_status random_level_keyed(pt_ctx* c, int level, int frame, Arr<float4>
     glibc_state((uint32_t)(frame * level), s0);
     CU(cudaMemcpyAsync(c->states, s0, sizeof(s0), cudaMemcpyHostToDevice, c->stream));
     CU(cudaStreamSynchronize(c->stream));
-    ExView ex{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS};
+    ExView ex{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS, 0, 0, 0, c->ex->flags};
     const int nk = (int)c->key_sub.size(), first_key = key_full_index(c, c->key_sub.front());
     LN(pt::launch_random_level_keys(lw, lh, mx, my, c->params.transparencyOk, c->params.orientationEnabled, rgba,
                                     orient, ex, c->rnd, c->states, nk, first_key, c->stream));

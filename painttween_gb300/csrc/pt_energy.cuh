@@ -17,6 +17,7 @@
 //    are then no-ops -- are left out.
 #pragma once
 
+#include <atomic>
 #include <climits>
 
 #include "pt_common.cuh"
@@ -26,21 +27,32 @@ namespace ptk {
 
 constexpr int kTileThreads = kTileW * kTileH;
 
+// Propagate's blocks per SM, which set its registers: the kernel waits for its
+// fetches, so more warps help until they spill.  Measured (summed launches):
+// without temporal terms three blocks of two candidates a lane (80 registers)
+// 11.6 ms against 13.8 with two (1024x1024 still); with them two blocks (128)
+// 167 against 174 ms (two 1080p frames); with the exact filter, whose samples
+// hold eight texels, two 50 against 70 ms (640x360, radius 4).
+template <int CPL, int TM, int HW>
+struct PropShape {
+    static constexpr int kBlocks = (HW == 0 || TM) ? (CPL == 1 ? 1 : 2) : (CPL == 1 ? 2 : 3);
+};
+
 enum { TM_NONE = 0, TM_FWD = 1, TM_BWD = 2 };
 
 // The staged planes start on 128-byte boundaries (tensor copies write
 // there); a tile row is TW texels, as a tensor copy's box row is.
-template <int R, int TM>
+template <int R, int TM, int H = kTileH>
 struct TileSmem {
     static constexpr int TW = kTileW + 2 * R;
-    static constexpr int TH = kTileH + 2 * R;
+    static constexpr int TH = H + 2 * R;
     static constexpr int N = TW * TH;
     alignas(128) float4 base[N];
     alignas(128) float4 canvas[N];
     alignas(128) float4 pbase[TM ? N : 1];
     alignas(128) float4 pout[TM ? N : 1];
-    alignas(128) float4 prec[TM ? N : 1];  // the advected records' B plane (.x: hysteresis, the validity)
-    unsigned long long bar;                // completion barrier of the tensor copies
+    unsigned long long bar;          // completion barrier of the tensor copies
+    uint8_t pvalid[TM ? N : 1];      // the advected record is valid (hysteresis > 0)
 };
 
 // both colours of one exemplar texel: a 32-byte record of the interleaved
@@ -227,7 +239,7 @@ __device__ __forceinline__ float energy_taps(const Params& P, const TileSmem<R, 
                         float r = ssdp(sub4p(base, pbase), sub4p(tb, peb)) * P.tdIn;
                         r = fmaf(ssdp(sub4p(canvas, pout), sub4p(to, peo)), P.tdOut, r);
                         r = fmaf(ssdp(pout, to), P.tc, r);
-                        res = (T.prec[s].x > 0) ? res + r : res;
+                        res = T.pvalid[s] ? res + r : res;
                     }
                 }
                 if (i == 0 && j == 0) {
@@ -316,20 +328,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 }
 
 // Stages the tile (and halo) of the pixel-side inputs and fills the
-// per-pixel state.  Returns false for threads whose pixel is outside the
-// level rectangle (and for the threads of a block of NT > kTileThreads
-// threads past the tile's pixels, which only evaluate candidates).  A tile whose halo lies inside the level rectangle, where
+// state of pixel `pid` of the tile (several threads of a block of NT >
+// kTileThreads threads may ask for the same pixel).  Returns false for
+// threads whose pixel is outside the level rectangle.  A tile whose halo lies inside the level rectangle, where
 // the clamps are no-ops, is copied by tensor copies when the maps are on
 // (one thread issues them; the texture mode's flush of subnormal input
 // colours follows in shared memory); the others load texel by texel with
 // the clamp rules.  *abort is set (for the whole block) when the copies did
 // not complete within two bounded waits; the block must then return.
-template <int R, int TM, int NT = kTileThreads>
-__device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, TileSmem<R, TM>& T, PixT* px,
-                                           bool* abort) {
-    constexpr int TW = TileSmem<R, TM>::TW, TH = TileSmem<R, TM>::TH, N = TileSmem<R, TM>::N;
+template <int R, int TM, int NT = kTileThreads, int H = kTileH>
+__device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, TileSmem<R, TM, H>& T, int pid,
+                                           PixT* px, bool* abort) {
+    constexpr int TW = TileSmem<R, TM, H>::TW, TH = TileSmem<R, TM, H>::TH, N = TileSmem<R, TM, H>::N;
     const int tid = threadIdx.x + threadIdx.y * kTileW;
-    const int x0 = blockIdx.x * kTileW - R, y0 = blockIdx.y * kTileH - R;
+    const int lx = pid % kTileW, ly = pid / kTileW;
+    const int x0 = blockIdx.x * kTileW - R, y0 = blockIdx.y * H - R;
     *abort = false;
     const bool interior = M.on && x0 >= 0 && y0 >= 0 && x0 + TW <= P.lw && y0 + TH <= P.lh;  // (block-uniform)
     if (interior) {
@@ -340,7 +353,7 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
         }
         __syncthreads();
         if (tid == 0) {
-            const uint32_t bytes = (uint32_t)(N * sizeof(float4)) * (TM ? 5u : 2u);
+            const uint32_t bytes = (uint32_t)(N * sizeof(float4)) * (TM ? 4u : 2u);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
             // x in FLOAT32 elements: 4 per texel, so x * 4 bytes is a multiple of 16
             tma_load_2d(T.base, &M.base, 4 * x0, y0, bar);
@@ -348,7 +361,6 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
             if (TM) {
                 tma_load_2d(T.pbase, &M.pbase, 4 * x0, y0, bar);
                 tma_load_2d(T.pout, &M.pout, 4 * x0, y0, bar);
-                tma_load_2d(T.prec, &M.prec, 4 * x0, y0, bar);
             }
         }
     } else {
@@ -363,21 +375,29 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
                 const AdvView& A = P.adv[TM == TM_FWD ? 0 : 1];
                 T.pbase[q] = __ldg(A.base + k);
                 T.pout[q] = __ldg(A.out + k);
-                T.prec[q] = __ldg(A.off.B + k);
             }
+        }
+    }
+    if (TM) {
+        const PatchPlanes& O = P.adv[TM == TM_FWD ? 0 : 1].off;
+        for (int q = tid; q < N; q += NT) {
+            const int gx = clampi(x0 + q % TW, 0, P.lw - 1), gy = clampi(y0 + q / TW, 0, P.lh - 1);
+            T.pvalid[q] = __ldg(&O.B[(size_t)gy * P.W + gx].x) > 0;
         }
     }
     // the per-pixel state reads global memory only: with tensor copies it is
     // computed while they are in flight
-    const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
-    const bool in = tid < kTileThreads && x < P.lw && y < P.lh;  // (threads past the tile's pixels only evaluate)
+    const int x = blockIdx.x * kTileW + lx, y = blockIdx.y * H + ly;
+    const bool in = x < P.lw && y < P.lh;
     if (in) {
         px->x = x;
         px->y = y;
-        px->sidx = (threadIdx.y + R) * TW + threadIdx.x + R;
+        px->sidx = (ly + R) * TW + lx + R;
         px->imin = max(-R, -x); px->imax = min(R, P.lw - 1 - x);
         px->jmin = max(-R, -y); px->jmax = min(R, P.lh - 1 - y);
-        {
+        if (px->imin == -R && px->imax == R && px->jmin == -R && px->jmax == R) {
+            px->sumW = P.sumW;
+        } else {
             float sw = 0.0f;
 #pragma unroll 1
             for (int i = -R; i <= R; i++)
@@ -487,7 +507,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_residual(const Params P, c
     }
     PixT px;
     bool abort;
-    if (!stage_tile<R, TM>(P, M, T, &px, &abort)) return;
+    if (!stage_tile<R, TM>(P, M, T, threadIdx.x + threadIdx.y * kTileW, &px, &abort)) return;
     if (!need) return;
     const size_t k = (size_t)px.y * P.W + px.x;
     if (image_culled(P, px.x, px.y)) { out[k] = 0.0f; return; }
@@ -498,28 +518,17 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_residual(const Params P, c
 }
 
 // ---------------------------------------------------------------------------
-// Lane cursors.  In the kernels below every lane evaluates one candidate at
-// a time, one column of 2R+1 taps per step, and takes its next candidate as
-// soon as the current one is finished or stopped early, instead of waiting
-// for the slowest lane of its warp.  Propagate and residual take their
-// candidates from a queue in shared memory, so any lane may evaluate any
-// pixel of the tile (the pixel-side context is in shared memory too);
-// scatter's lanes each follow their own pixel's chain.  A candidate's sum
-// still runs over its taps in the reference's order, so every energy is
-// bit-identical to a separate evaluation.
+// Lane cursors.  Scatter's lanes each follow their own pixel's chain, one
+// column of 2R+1 taps per step, and take the next candidate as soon as the
+// current one is finished or stopped early.  A candidate's sum runs over its
+// taps in the reference's order, so every energy is bit-identical to a
+// separate evaluation.
 // ---------------------------------------------------------------------------
 
 constexpr unsigned kFull = 0xffffffffu;
 // (1 -/+ 2^-17): bounds of the rounding of a reference-order sum of <= 81 terms
 constexpr float kBoundLo = 1.0f - 1.0f / 131072.0f;
 constexpr float kBoundHi = 1.0f + 1.0f / 131072.0f;
-// Propagate takes no bound pass: its candidates come from coherent
-// neighbours, so their energies are mostly close to the best and a bound
-// pass rarely rejects them before its end (measured: 1 or 2 groups of 2R+1
-// taps +45-53 %, the full pass +20 % propagate time); scatter's
-// random-search candidates are rejected after a few heavy taps (full bound
-// pass: -45 % scatter time).
-
 // pixel side of an evaluation
 struct LanePix {
     int x, y, sidx;
@@ -578,28 +587,29 @@ __device__ __forceinline__ LanePix lane_pix(const Params& P, const PixT& px) {
     return q;
 }
 
-// the pixel contexts of a tile in shared memory
+// the pixel contexts of a tile of NP pixels in shared memory
+template <int NP = kTileThreads>
 struct PixShared {
-    float4 a[kTileThreads];  // sum0, sumW, prev x, prev y
-    float4 b[kTileThreads];  // prev basis
-    int bits[kTileThreads];  // window bounds + R (4 bits each), temporal, prev_fast, prev layer
+    float4 a[NP];  // sum0, sumW, prev x, prev y
+    float4 b[NP];  // prev basis
+    int bits[NP];  // window bounds + R (4 bits each), temporal, prev_fast, prev layer
 };
 
-template <int R>
-__device__ __forceinline__ void put_pix(PixShared& S, int pid, const LanePix& q) {
+template <int R, int NP>
+__device__ __forceinline__ void put_pix(PixShared<NP>& S, int pid, const LanePix& q) {
     S.a[pid] = make_float4(q.sum0, q.sumW, q.prevx, q.prevy);
     S.b[pid] = make_float4(q.pb0.x, q.pb0.y, q.pb1.x, q.pb1.y);
     S.bits[pid] = (q.imin + R) | ((q.imax + R) << 4) | ((q.jmin + R) << 8) | ((q.jmax + R) << 12) |
                   (q.temporal ? 1 << 16 : 0) | (q.prev_fast ? 1 << 17 : 0) | (q.prevlayer << 18);
 }
 
-template <int R, int TM>
-__device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared& S, int pid) {
+template <int R, int TM, int NP>
+__device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>& S, int pid) {
     constexpr int TW = TileSmem<R, TM>::TW;
     LanePix q;
     const int lx = pid % kTileW, ly = pid / kTileW;
     q.x = blockIdx.x * kTileW + lx;
-    q.y = blockIdx.y * kTileH + ly;
+    q.y = blockIdx.y * (NP / kTileW) + ly;
     q.sidx = (ly + R) * TW + lx + R;
     const float4 a = S.a[pid], b = S.b[pid];
     const int bits = S.bits[pid];
@@ -681,7 +691,7 @@ __device__ __forceinline__ float tap_finish(const Params& P, const TileSmem<R, T
             float r = ssdp(sub4p(base, pbase), sub4p(tb, t.peb)) * P.tdIn;
             r = fmaf(ssdp(sub4p(canvas, pout), sub4p(to, t.peo)), P.tdOut, r);
             r = fmaf(ssdp(pout, to), P.tc, r);
-            res = (T.prec[s].x > 0) ? res + r : res;
+            res = T.pvalid[s] ? res + r : res;
         }
     }
     if (j == 0 && i == 0) {
@@ -865,210 +875,568 @@ __device__ __forceinline__ bool lane_step_uni(const Params& P, const TileSmem<R,
     return true;
 }
 
-// a lane's index in a shared queue: warp-aggregated atomic on *next
-__device__ __forceinline__ int queue_take(bool want, int* next) {
-    const unsigned m = __ballot_sync(kFull, want);
-    const int lane = (int)lane_id();
-    const int leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(next, __popc(m));
-    base = __shfl_sync(kFull, base, leader);
-    return base + __popc(m & ((1u << lane) - 1u));
+// ---------------------------------------------------------------------------
+// Candidate evaluation in two parts.
+//
+// Nineteen of twenty candidates lose, so a candidate is first held against a
+// lower bound of its energy over the taps in the order of their weight.  The
+// reference forms its sum in tap order with round-to-nearest fmaf over at
+// most 81 non-negative terms, which is at least (1 - 2^-17) times the exact
+// sum of those terms, plus its start sum (the hysteresis term, <= 0) scaled by
+// at most (1 + 2^-17).  So once (1 - 2^-17) * bound + that start-sum share
+// reaches thr2 = best * sumW rounded up, the reference-order
+// energy is >= best and the strict "<" rejects the candidate; the bound is
+// formed with round-down products and sums, in any order.  Only where the
+// threshold is so small (|thr2| < 2^-100) that subnormal rounding could
+// matter, or is none at all, no candidate is rejected by it.
+//  * The front pass (front_taps) takes the heaviest taps, the 3 x 3 in the
+//    middle, for all of a lane's candidates of its pixel at once: the
+//    pixel-side texels and the previous frame's samples of a tap are read
+//    once for them.  Measured over the taps that reject: 82-90 % of the
+//    candidates end here at radius 2, 66-68 % at radius 3, 46 % at radius 4.
+//  * The survivors of a warp are packed into a queue of its own (WarpQueue),
+//    from which groups of eight lanes take one candidate each (eval_queue):
+//    eight further taps at a time in the order of their weight, the bound
+//    tested after each eight.  Every tap's value is kept, so that a candidate
+//    that no bound rejects (5-8 %) has its energy summed from them in the
+//    reference's order: no tap is fetched again for the exact sum.
+// Before this, each candidate was summed in the reference's order from the
+// first column on, whose taps are the lightest, and left at the threshold:
+// 15.7 / 28.4 / 48.1 taps fetched per candidate at radius 2 / 3 / 4 (now 7.5 /
+// 12.0 / 24.6), each with its own read of the pixel side.  Measured, summed
+// launches: propagate of a 1024x1024 still (radius 2) 21.5 -> 11.6 ms, of two
+// 1080p frames (radius 3) 288 -> 167 ms, of a 128x128 still 5.5 -> 2.5 ms.
+// What bounds it now: the texture unit's share of its peak fell from 74 to
+// 27 % while the fetches fell 2.4 times, and warps wait for the fetches of one
+// tap at a time (5.3 of 10.4 cycles per instruction); hence as many warps as
+// the registers allow (PropShape).  Groups of 4 lanes measured the same, of 16
+// 7 % slower; a front of 5 taps 1-7 % slower than 9.
+// ---------------------------------------------------------------------------
+
+constexpr int kFront = 9;   // taps of the front pass: the 3 x 3 in the middle
+constexpr int kGroup = 8;   // lanes that evaluate one surviving candidate
+constexpr int kGroups = 32 / kGroup;
+
+// One tap of the weight order: its place (i, j), weight and index in the
+// reference's (column-major) order.
+struct Tap {
+    float fi, fj, w;
+    int code;  // (i + R) | (j + R) << 4 | t << 8
+};
+template <int R>
+struct TapList {
+    Tap tap[(2 * R + 1) * (2 * R + 1)];
+};
+template <int R>
+__device__ __forceinline__ void load_tap_list(const Params& P, TapList<R>& L, int tid) {
+    constexpr int n = 2 * R + 1, K = n * n;
+    if (tid < K) {
+        const int t = P.tapOrder[tid], i = t / n, j = t % n;
+        Tap a;
+        a.fi = (float)(i - R);
+        a.fj = (float)(j - R);
+        a.w = P.gauss[i] * P.gauss[j];
+        a.code = i | (j << 4) | (t << 8);
+        L.tap[tid] = a;
+    }
 }
 
-// candidates of a propagate tile
-struct PropQueue {
-    float4 ca[kTileThreads * 4];     // x, y, theta, su; x holds the energy once evaluated
-    float2 cb[kTileThreads * 4];     // sv, layer bits
-    uint16_t list[kTileThreads * 4];  // pid * 4 + slot
-    float thr[kTileThreads];          // the pixel's residual
-    int slots[kTileThreads];          // per candidate (3 bits each): slot + 3, or 0 skipped, 1 repeat, 2 rejected
-    int count[kTileH], next[kTileH];  // per warp: its row's candidates (list[128 * warp ...])
+// the candidate side of an evaluation
+struct CandPos {
+    float x, y;
+    float2 b0, b1;
+    int layer;
 };
 
-// propagate_kernel with lane cursors over the tile's candidates.  WIDE
-// warps per tile row: with WIDE = 2 the block has twice the tile's threads
-// and the second half only takes candidates from the rows' queues (the same
-// candidates and results, evaluated by twice the lanes: for the coarse
-// levels, whose few tiles leave most of the GPU idle).
-template <int R, int TM, int HW, int WIDE>
-__global__ void __launch_bounds__(kTileThreads * WIDE, WIDE == 1 ? 2 : 1)
-    kt_propagate_q(const Params P, const __grid_constant__ TileMaps M, PatchPlanes work, int jump) {
-    const int pid = threadIdx.x + threadIdx.y * kTileW;
-    __shared__ TileSmem<R, TM> T;
-    __shared__ PixShared S;
-    __shared__ PropQueue Q;
+// exemplar samples of one tap
+struct ExSample {
+    float4 tb, to;
+};
+
+template <int HW>
+__device__ __forceinline__ ExSample cand_fetch(const Params& P, const CandPos& c, float fi, float fj, bool fast,
+                                               float* ptx, float* pty) {
+    const size_t lsz = (size_t)P.ex.w * P.ex.h;
+    const int li = ex_layer(P.ex, c.layer);
+    const float hw = (float)P.histW, hh = (float)P.histH;
+    float tx = c.x + fmaf(fi, c.b0.x, fj * c.b1.x);
+    float ty = c.y + fmaf(fi, c.b0.y, fj * c.b1.y);
+    if (!fast) {
+        if (tx >= hw) tx -= hw; else if (tx < 0) tx += hw;
+        if (ty >= hh) ty -= hh; else if (ty < 0) ty += hh;
+    }
+    ExSample s;
+    sample2<true, HW>(P.ex, li, P.ex.bo + 2 * (size_t)li * lsz, tx, ty, &s.tb, &s.to, fast);
+    *ptx = tx;
+    *pty = ty;
+    return s;
+}
+
+// the previous frame's samples of one tap (temporal passes)
+template <int HW>
+__device__ __forceinline__ ExSample prev_fetch(const Params& P, const LanePix& q, float fi, float fj, bool fastp) {
+    const size_t lsz = (size_t)P.ex.w * P.ex.h;
+    const float x = q.prevx + fmaf(fi, q.pb0.x, fj * q.pb1.x);
+    const float y = q.prevy + fmaf(fi, q.pb0.y, fj * q.pb1.y);
+    ExSample s;
+    sample2<true, HW>(P.ex, q.prevlayer, P.ex.bo + 2 * (size_t)q.prevlayer * lsz, x, y, &s.tb, &s.to, fastp);
+    return s;
+}
+
+// the pixel side of one tap
+struct PixSample {
+    float4 base, canvas, pbase, pout;
+    bool prev;  // the temporal terms apply at this tap
+};
+template <int R, int TM, int H>
+__device__ __forceinline__ PixSample pix_sample(const TileSmem<R, TM, H>& T, const LanePix& q, int s) {
+    PixSample p;
+    p.base = T.base[s];
+    p.canvas = T.canvas[s];
+    p.prev = false;
+    if (TM && q.temporal) {
+        p.pbase = T.pbase[s];
+        p.pout = T.pout[s];
+        p.prev = T.pvalid[s] != 0;
+    }
+    return p;
+}
+
+// calculateResidual's value at one tap before its Gaussian weight
+// (texSynth_kernel.cu:537-659), without the terms of the middle tap;
+// `center`: the middle tap, which leaves out the canvas term
+template <int TM>
+__device__ __forceinline__ float tap_terms(const Params& P, const PixSample& p, const ExSample& c, const ExSample& v,
+                                           bool center) {
+    float res = ssd_ap(p.base, c.tb, P.alphaWeight) * P.inputAnalogyWeight;
+    if (TM) {
+        float r = ssdp(sub4p(p.base, p.pbase), sub4p(c.tb, v.tb)) * P.tdIn;
+        r = fmaf(ssdp(sub4p(p.canvas, p.pout), sub4p(c.to, v.to)), P.tdOut, r);
+        r = fmaf(ssdp(p.pout, c.to), P.tc, r);
+        res = p.prev ? res + r : res;
+    }
+    return center ? res : fmaf(ssd_ap(p.canvas, c.to, P.alphaWeight), P.canvasOutputWeight, res);
+}
+
+// the terms of the middle tap added to its value: distance transform,
+// histogram, object ids (texSynth_kernel.cu:640-655)
+template <int HW>
+__device__ __forceinline__ float center_terms(const Params& P, const LanePix& q, int layer, float sv, float tx,
+                                              float ty, float res) {
+    if (P.distTransWeight > 0.f) {
+        float de = ex_sample_dt(ex_mode<HW>(P.ex), tx, ty, layer) / sv;
+        float di = lay_texel(P.img.dt[P.img.cur], P, q.x, q.y);
+        float diff = fmaxf(0.0f, fminf(fabsf(de - di), 10.0f));  // clamp(diff, 0, 10): a NaN difference gives 10
+        res = res + diff * P.distTransWeight;
+    }
+    {
+        int Lh = clampi(layer, 0, PT_MAX_STYLES - 1);
+        float sh = (float)(P.histH / P.numStyles);
+        int hx = clampi((int)tx, 0, P.histPitch - 1);
+        int hy = clampi((int)(ty + sh * (float)layer), 0, P.histRows - 1);
+        float h = __ldg(P.hist + (size_t)hy * P.histPitch + hx);
+        float thr = P.histThreshold[Lh];
+        res = res + ((h > thr) ? (h - thr) * P.histSlope[Lh] : 0.0f);
+    }
+    if (P.styleObjIdWeight > 0.f) {
+        int imgID = lvl_texel(P.img.ids, q.x, q.y);
+        int styleID = ex_point_id(P.ex, tx, ty, layer);
+        res = res + ((imgID != styleID) ? P.styleObjIdWeight : 0.0f);
+    }
+    return res;
+}
+
+// thr2 and the bound pass's threshold of a pixel whose energy to beat is
+// `best` (see exit_threshold): the latter is NaN, which rejects nothing,
+// where the bound is not used
+struct Threshold {
+    float thr2, bound;
+};
+__device__ __forceinline__ Threshold threshold_of(const Params& P, const LanePix& q, float best) {
+    Threshold t;
+    t.thr2 = (P.earlyExit && q.sumW >= kEpsilon) ? __fmul_ru(best, q.sumW) : kNoBest;
+    // the start sum's share of the reference-order sum, from below
+    const float s0lo = q.sum0 >= 0.0f ? __fmul_rd(q.sum0, kBoundLo) : __fmul_rd(q.sum0, kBoundHi);
+    // (thr2 - s0lo) / (1 - 2^-17) from above: 1 / (1 - 2^-17) < 1 + 2^-16
+    const float need = __fsub_ru(t.thr2, s0lo);
+    t.bound = fabsf(t.thr2) >= 0x1p-100f ? (need > 0.0f ? __fmul_ru(need, 1.0f + 1.0f / 65536.0f) : need) : kNoBest;
+    return t;
+}
+
+// The surviving candidates of one warp.
+template <int CAP>
+struct WarpQueue {
+    float4 a[CAP];     // x, y, b0
+    float4 b[CAP];     // b1, the bound so far, layer bits
+    float v0[CAP];     // the middle tap's value
+    uint16_t id[CAP];  // pid * 4 + slot | fast << 15
+};
+
+// The front pass over NC candidates of pixel q (bit c of `alive`: candidate c
+// is evaluated), the warp's lanes together.  Returns the candidates still
+// alive; their bounds are in sum[], the middle tap's values in v0[].
+template <int R, int TM, int HW, int NC, int H>
+__device__ __forceinline__ unsigned front_taps(const Params& P, const TileSmem<R, TM, H>& T, const TapList<R>& L,
+                                               const LanePix& q, const Threshold& th, const CandPos (&c)[NC],
+                                               float sv, unsigned alive, float (&sum)[NC],
+                                               float (&v0)[NC]) {
+    constexpr int TW = TileSmem<R, TM>::TW;
+    bool in = true;  // every footprint of the lane inside the exemplar
+#pragma unroll
+    for (int k = 0; k < NC; k++) {
+        in = in && (!((alive >> k) & 1) || footprint_inside<R>(c[k].x, c[k].y, c[k].b0, c[k].b1, P.ex.w, P.ex.h));
+        sum[k] = 0.0f;
+        v0[k] = 0.0f;
+    }
+    const bool fast = __all_sync(kFull, in);
+    const bool fastp = TM ? __all_sync(kFull, !alive || !q.temporal || q.prev_fast) : true;
+    const bool bounded = th.bound == th.bound;
+    unsigned taps = 0;
+#pragma unroll 1
+    for (int t = 0; t < kFront; t++) {
+        const unsigned on = (t == 0 || bounded) ? alive : 0u;
+        if (!__any_sync(kFull, on)) break;
+        const Tap tp = L.tap[t];
+        const int i = (tp.code & 15) - R, j = ((tp.code >> 4) & 15) - R;
+        const bool valid = (i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax);
+        if (!on || !valid) continue;
+        const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + j * TW + i);
+        ExSample s[NC], v;
+        float tx[NC], ty[NC];
+        if (TM && p.prev) v = prev_fetch<HW>(P, q, tp.fi, tp.fj, fastp);
+#pragma unroll
+        for (int k = 0; k < NC; k++)
+            if ((on >> k) & 1) s[k] = cand_fetch<HW>(P, c[k], tp.fi, tp.fj, fast, &tx[k], &ty[k]);
+#pragma unroll
+        for (int k = 0; k < NC; k++)
+            if ((on >> k) & 1) {
+                float r = tap_terms<TM>(P, p, s[k], v, t == 0);
+                if (t == 0) {
+                    r = center_terms<HW>(P, q, c[k].layer, sv, tx[k], ty[k], r);
+                    v0[k] = r;
+                }
+                sum[k] = __fmaf_rd(r, tp.w, sum[k]);
+                if (sum[k] >= th.bound) alive &= ~(1u << k);
+            }
+        taps += __popc(on);
+    }
+    if (P.counters) count_taps(P, taps, q.temporal);
+    return alive;
+}
+
+// The lane's surviving candidates appended to its warp's queue; returns the
+// queue's length (the same for every lane).
+template <int R, int NC, int CAP>
+__device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& Q, int pid, int slot0, unsigned alive,
+                                               const CandPos (&c)[NC], const float (&sum)[NC], const float (&v0)[NC]) {
+    const int n = __popc(alive);
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, o);
+        if ((int)lane_id() >= o) incl += v;
+    }
+    int w = incl - n;
+#pragma unroll
+    for (int k = 0; k < NC; k++)
+        if ((alive >> k) & 1) {
+            const bool in = footprint_inside<R>(c[k].x, c[k].y, c[k].b0, c[k].b1, P.ex.w, P.ex.h);
+            Q.a[w] = make_float4(c[k].x, c[k].y, c[k].b0.x, c[k].b0.y);
+            Q.b[w] = make_float4(c[k].b1.x, c[k].b1.y, sum[k], __int_as_float(c[k].layer));
+            Q.v0[w] = v0[k];
+            Q.id[w] = (uint16_t)((pid * 4 + slot0 + k) | (in ? 1 << 15 : 0));
+            w++;
+        }
+    __syncwarp();
+    return __shfl_sync(kFull, incl, 31);
+}
+
+// Evaluates the first n candidates of the warp's queue, a group of kGroup
+// lanes each; energies of those that no bound rejects into energy[pid * 4 +
+// slot].  thr: the energy to beat of each pixel of the tile; V: (2R+1)^2
+// values of each of the warp's groups.
+template <int R, int TM, int HW, int H, int CAP>
+__device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM, H>& T,
+                                           const PixShared<kTileW * H>& S, const TapList<R>& L,
+                                           const WarpQueue<CAP>& Q, int n, const float* thr,
+                                           float* V, float* energy) {
+    constexpr int TW = TileSmem<R, TM>::TW, n1 = 2 * R + 1, K = n1 * n1;
+    constexpr int kRest = (K - kFront + kGroup - 1) / kGroup;        // steps past the front
+    constexpr int kLast = kRest + (kFront - 1 + kGroup - 1) / kGroup;  // and of the front's other taps
+    const int lane = (int)lane_id(), g = lane / kGroup, l = lane % kGroup;
+    float* val = V + g * K;
+    bool act = false, cfast = false;
+    int next = 0, step = 0, id = 0;
+    float sum = 0.0f;
+    LanePix q;
+    CandPos c;
+    Threshold th;
+    q.temporal = false;
+    q.prev_fast = true;
+#pragma unroll 1
+    while (true) {
+        const unsigned idle = __ballot_sync(kFull, !act);
+        if (!act) {
+            const int t = next + __popc(idle & ((1u << (g * kGroup)) - 1u)) / kGroup;
+            if (t < n) {
+                const float4 a = Q.a[t], b = Q.b[t];
+                id = Q.id[t];
+                cfast = (id >> 15) & 1;
+                id &= 1023;
+                c.x = a.x; c.y = a.y;
+                c.b0 = make_float2(a.z, a.w);
+                c.b1 = make_float2(b.x, b.y);
+                c.layer = __float_as_int(b.w);
+                sum = b.z;
+                q = get_pix<R, TM>(P, S, id >> 2);
+                th = threshold_of(P, q, thr[id >> 2]);
+                if (l == 0) val[K / 2] = Q.v0[t];
+                step = 0;
+                act = true;
+            }
+        }
+        next += __popc(idle) / kGroup;
+        if (!__any_sync(kFull, act)) break;
+        const bool fast = __all_sync(kFull, !act || cfast);
+        const bool fastp = TM ? __all_sync(kFull, !act || !q.temporal || q.prev_fast) : true;
+        // steps 0 .. kRest-1: the taps past the front; then the front's other
+        // taps, for the exact sum
+        float part = 0.0f;
+        const int pos = step < kRest ? kFront + step * kGroup + l : 1 + (step - kRest) * kGroup + l;
+        if (act && pos < (step < kRest ? K : kFront)) {
+            const Tap tp = L.tap[pos];
+            const int i = (tp.code & 15) - R, j = ((tp.code >> 4) & 15) - R;
+            if ((i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax)) {
+                const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + j * TW + i);
+                ExSample v;
+                float tx, ty;
+                if (TM && p.prev) v = prev_fetch<HW>(P, q, tp.fi, tp.fj, fastp);
+                const ExSample s = cand_fetch<HW>(P, c, tp.fi, tp.fj, fast, &tx, &ty);
+                const float r = tap_terms<TM>(P, p, s, v, false);
+                val[tp.code >> 8] = r;
+                if (step < kRest) part = __fmul_rd(r, tp.w);
+            }
+            if (P.counters) count_taps(P, 1u, q.temporal);
+        }
+#pragma unroll
+        for (int o = 1; o < kGroup; o <<= 1) part = __fadd_rd(part, __shfl_xor_sync(kFull, part, o));
+        const bool last = act && step == kLast - 1;
+        sum = __fadd_rd(sum, part);
+        step++;
+        if (act && !last && sum >= th.bound) act = false;
+        if (__any_sync(kFull, last)) {
+            __syncwarp();
+            if (last) {
+                // the exact sum, in the reference's order
+                float e = q.sum0;
+#pragma unroll 1
+                for (int i = -R; i <= R; i++) {
+                    const float gi = P.gauss[i + R];
+                    const bool cvalid = (i >= q.imin) && (i <= q.imax);
+#pragma unroll
+                    for (int j = -R; j <= R; j++) {
+                        const bool valid = cvalid && (j >= q.jmin) && (j <= q.jmax);
+                        const float w = gi * P.gauss[j + R];
+                        const float v = val[(i + R) * n1 + j + R];
+                        e = valid ? fmaf(v, w, e) : e;
+                    }
+                }
+                if (l == 0)
+                    energy[id] = (q.sumW < kEpsilon) ? kBigResidual : (e >= th.thr2) ? INFINITY : e / q.sumW;
+                act = false;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// the energy phase's shared state of a block of NW warps over NP pixels, each
+// warp with up to CAP surviving candidates
+template <int R, int NW, int NP, int CAP>
+struct EvalSmem {
+    PixShared<NP> S;
+    WarpQueue<CAP> Q[NW];
+    TapList<R> L;
+    float V[NW][kGroups * (2 * R + 1) * (2 * R + 1)];
+    float thr[NP];                    // the energy each pixel has to beat
+    alignas(16) float energy[NP * 4];  // per candidate: its energy, +inf where it lost or is none
+};
+
+// calculatePropagateOffset, texSynth_kernel.cu:956-982 (propagate_offset), for
+// CPL of a pixel's sources at once, in steps whose loads do not wait for one
+// another: the sources' records and scales, the exemplar orientations under
+// the moved offsets, then the angles and bases.
+struct PropCand {
+    CandPos c;
+    float theta;
+};
+template <int CPL>
+__device__ __forceinline__ void propagate_candidates(const Params& P, int x, int y, int slot0, int jump,
+                                                     float2 scale, PropCand (&o)[CPL]) {
+    float4 a[CPL];
+    float2 sc[CPL];
+    float dx[CPL], dy[CPL];
+#pragma unroll
+    for (int i = 0; i < CPL; i++) {
+        int tx, ty;
+        propagate_source(slot0 + i, x, y, jump, &tx, &ty);
+        dx[i] = (float)x - (float)tx;
+        dy[i] = (float)y - (float)ty;
+        a[i] = __ldg(P.off.A + pixel_wrap_index(P, tx, ty));
+        sc[i] = lvl_texel_lin(P.img.scale, tx, ty, P.hwFilter);
+    }
+    float eo[CPL];
+#pragma unroll
+    for (int i = 0; i < CPL; i++) {
+        float2 b0, b1;
+        basis(a[i].z, P.scaleWU * sc[i].x, P.scaleWV * sc[i].y, &b0, &b1);
+        CandPos& c = o[i].c;
+        new_coord(dx[i], dy[i], a[i].x, a[i].y, b0, b1, &c.x, &c.y);
+        clamp_to_exemplar(&c.x, &c.y, P.ex.w, P.ex.h);
+        c.layer = __float_as_int(a[i].w);
+        eo[i] = P.orientationEnabled ? ex_point_orient(P.ex, c.x, c.y, c.layer) : 0.0f;
+    }
+    const float io = P.orientationEnabled ? lvl_texel(P.img.orient, x, y) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < CPL; i++) {
+        o[i].theta = P.orientationEnabled ? fold_angle(eo[i] - io) : 0.0f;
+        basis(o[i].theta, P.scaleWU * scale.x, P.scaleWV * scale.y, &o[i].c.b0, &o[i].c.b1);
+    }
+}
+
+// propagate_kernel, texSynth_kernel.cu:956-982,1112-1219, over tiles of 32 x H
+// pixels.  A lane takes CPL of its pixel's four candidates (a warp covers
+// 8 * CPL pixels), and a warp goes through its candidates alone, from the
+// front pass to its pixels' results, without a barrier of the block.
+template <int R, int TM, int HW, int CPL, int H>
+__global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::kBlocks)
+    kt_propagate(const Params P, const __grid_constant__ TileMaps M, PatchPlanes work, int jump) {
+    constexpr int NP = kTileW * H, NT = NP * 4 / CPL, NW = NT / 32, PPW = 8 * CPL;  // PPW: pixels per warp
+    using Tile = TileSmem<R, TM, H>;
+    using Eval = EvalSmem<R, NW, NP, 32 * CPL>;
+    extern __shared__ __align__(128) unsigned char dyn[];
+    Tile& T = *reinterpret_cast<Tile*>(dyn);
+    Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    const int tid = threadIdx.x + threadIdx.y * kTileW, warp = tid / 32, lane = tid % 32;
+    const int pid = warp * PPW + lane % PPW, slot0 = lane / PPW * CPL;  // the lane's pixel and first candidate
+    const bool head = slot0 == 0;                                      // the lane that writes its pixel
     // Change tracking: a candidate whose source record and whose target's
     // patch window are unchanged since the previous pass with this jump was
-    // rejected there against the same residual and is skipped (bit cdx of
+    // rejected there against the same residual and is skipped (bit i of
     // `skip`); a pass without a previous one skips nothing.
     unsigned skip = 0;
     if (P.inc.on) {
-        const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
-        const bool in = pid < kTileThreads && x < P.lw && y < P.lh;
+        const int x = blockIdx.x * kTileW + pid % kTileW, y = blockIdx.y * H + pid / kTileW;
+        const bool in = x < P.lw && y < P.lh;
         const size_t k = (size_t)y * P.W + x;
         bool need = in;
-        if (in && P.inc.prev != INT_MIN && __ldg(P.inc.win + k) < P.inc.prev) {
+        if (in && P.inc.prev != INT_MIN) {
+            int last[CPL];
 #pragma unroll
-            for (int cdx = 0; cdx < 4; cdx++) {
+            for (int i = 0; i < CPL; i++) {
                 int tx, ty;
-                propagate_source(cdx, x, y, jump, &tx, &ty);
-                if (__ldg(P.inc.last + pixel_wrap_index(P, tx, ty)) < P.inc.prev) skip |= 1u << cdx;
+                propagate_source(slot0 + i, x, y, jump, &tx, &ty);
+                last[i] = __ldg(P.inc.last + pixel_wrap_index(P, tx, ty));
             }
-            need = skip != 0xFu && !image_culled(P, x, y);
+            if (__ldg(P.inc.win + k) < P.inc.prev) {
+#pragma unroll
+                for (int i = 0; i < CPL; i++)
+                    if (last[i] < P.inc.prev) skip |= 1u << i;
+                need = skip != (1u << CPL) - 1u && !image_culled(P, x, y);
+            }
         }
-        if (block_idle(P, work, need, in, k)) return;
+        if (block_idle(P, work, need, in && head, k)) return;
     }
-    if (pid < kTileH) { Q.count[pid] = 0; Q.next[pid] = 0; }
+    load_tap_list<R>(P, E.L, tid);
     PixT px;
     bool abort;
-    const bool in = stage_tile<R, TM, kTileThreads * WIDE>(P, M, T, &px, &abort);  // (synchronises the block)
+    const bool in = stage_tile<R, TM, NT, H>(P, M, T, pid, &px, &abort);  // (synchronises the block)
     if (abort) return;
-    // phase 1: each pixel builds its candidates (the reference's order,
-    // repeats and test_offset rejections resolved here) and queues them
-    int n = 0;
-    bool culled = false;
+    const int x = px.x, y = px.y;
+    const size_t k = in ? (size_t)y * P.W + x : 0;
+    // the candidates, in the reference's order (repeats and test_offset
+    // rejections resolved here)
+    CandPos c[CPL];
+    float2 scale = make_float2(1.f, 1.f);
+    unsigned alive = 0;
+    bool own = false;
+    LanePix q;
+    Threshold th;
+    q.temporal = false;
+    q.prev_fast = true;
+    th.thr2 = th.bound = kNoBest;
+    float best = 0.0f;
     if (in) {
-        const int x = px.x, y = px.y;
-        const size_t k = (size_t)y * P.W + x;
-        culled = image_culled(P, x, y);
-        if (culled) {
-            const Patch z = make_patch(0, 0, 0, 0, 0, 1.f, 1.f);
-            if (P.inc.on) P.inc.chg[k] = same_record(z, load_patch(P.off, k)) ? 0 : 1;
-            store_patch(work, k, z);
+        if (image_culled(P, x, y)) {
+            if (head) {
+                const Patch z = make_patch(0, 0, 0, 0, 0, 1.f, 1.f);
+                if (P.inc.on) P.inc.chg[k] = same_record(z, load_patch(P.off, k)) ? 0 : 1;
+                store_patch(work, k, z);
+            }
         } else {
+            own = true;
+            best = __ldg(P.res + k);
+            scale = lvl_texel_lin(P.img.scale, x, y, P.hwFilter);
+            PropCand pc[CPL];
+            propagate_candidates<CPL>(P, x, y, slot0, jump, scale, pc);
+            const bool opaque = P.transparencyOk || !exemplar_transparent(P.ex);
+            const bool culls = exemplar_culls(P.ex, P.exCull);
             const float ia = T.base[px.sidx].w;
-            uint32_t kx[4], ky[4], kt[4];
-            int kl[4];
-            int codes = 0;
 #pragma unroll
-            for (int cdx = 0; cdx < 4; cdx++) {
-                kx[cdx] = ky[cdx] = kt[cdx] = 0u;
-                kl[cdx] = 0;
-                int code = 2;  // rejected before the energy
-                if (skip & (1u << cdx)) {
-                    code = 0;
-                } else {
-                    int tx, ty;
-                    propagate_source(cdx, x, y, jump, &tx, &ty);
-                    Patch t = propagate_offset(P, tx, ty, x, y);
-                    kx[cdx] = __float_as_uint(t.x);
-                    ky[cdx] = __float_as_uint(t.y);
-                    kt[cdx] = __float_as_uint(t.theta);
-                    kl[cdx] = t.layer;
-                    bool dup = false;
+            for (int i = 0; i < CPL; i++) {
+                c[i] = pc[i].c;
+                float e = INFINITY;  // skipped, a repeat, or lost: rejected by "<"
+                bool dup = false;
 #pragma unroll
-                    for (int q = 0; q < cdx; q++)
-                        dup |= !(skip & (1u << q)) && kx[q] == kx[cdx] && ky[q] == ky[cdx] && kt[q] == kt[cdx] &&
-                               kl[q] == kl[cdx];
-                    if (dup) {
-                        code = 1;
+                for (int h = 0; h < i; h++)
+                    dup |= !((skip >> h) & 1) && __float_as_uint(c[h].x) == __float_as_uint(c[i].x) &&
+                           __float_as_uint(c[h].y) == __float_as_uint(c[i].y) &&
+                           __float_as_uint(pc[h].theta) == __float_as_uint(pc[i].theta) && c[h].layer == c[i].layer;
+                if (!((skip >> i) & 1) && !dup) {
+                    bool ok = !culls || !(ex_texel_dt(ex_mode<HW>(P.ex), (int)c[i].x, (int)c[i].y, c[i].layer) > P.exCull);
+                    if (ok && !opaque && ia > kAlphaThreshold)
+                        ok = !(ex_out_alpha<HW>(P.ex, c[i].x, c[i].y, c[i].layer) < kAlphaThreshold);
+                    if (ok) {
+                        alive |= 1u << i;
+                        if (P.counters) count_eval(P, x, y, px.temporal, false);
                     } else {
-                        float dte = ex_texel_dt(ex_mode<HW>(P.ex), (int)t.x, (int)t.y, t.layer);
-                        bool ok = !((double)dte > (double)P.distTransCull * 1.25);
-                        if (ok && !P.transparencyOk) {
-                            float ea = ex_sample_out_alpha(ex_mode<HW>(P.ex), t.x, t.y, t.layer);
-                            ok = !(ea < kAlphaThreshold && ia > kAlphaThreshold);
-                        }
-                        if (ok) {
-                            if (P.counters) count_eval(P, x, y, px.temporal, false);
-                            Q.ca[pid * 4 + n] = make_float4(t.x, t.y, t.theta, t.su);
-                            Q.cb[pid * 4 + n] = make_float2(t.sv, __int_as_float(t.layer));
-                            code = n + 3;
-                            n++;
-                        }
+                        e = kBigResidual;  // rejected before the energy: competes with 1e31
                     }
                 }
-                codes |= code << (3 * cdx);
+                E.energy[pid * 4 + slot0 + i] = e;
             }
-            Q.slots[pid] = codes;
-            Q.thr[pid] = __ldg(P.res + k);
-            put_pix<R>(S, pid, lane_pix<R>(P, px));
-        }
-    }
-    if (pid < kTileThreads) {  // (whole warps)
-        // queue this pixel's n candidates
-        const unsigned lane = lane_id();
-        int incl = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int v = __shfl_up_sync(kFull, incl, o);
-            if ((int)lane >= o) incl += v;
-        }
-        // each warp queues its own row's candidates, so that its lanes
-        // gather from neighbouring exemplar regions (a coherent field maps
-        // neighbouring pixels to neighbouring texels)
-        const int warp = pid / kTileW;
-        if (lane == 31) Q.count[warp] = incl;
-        for (int j = 0; j < n; j++) Q.list[warp * 4 * kTileW + incl - n + j] = (uint16_t)(pid * 4 + j);
-    }
-    __syncthreads();
-    // phase 2: lane cursors over the queue
-    {
-        LanePix q;
-        LaneEval e;
-        bool act = false, more = true;
-        int cur = 0;
-        const int warp = (pid / kTileW) % kTileH;  // the row whose queue this warp takes from
-        const int count = Q.count[warp];
-#pragma unroll 1
-        while (true) {
-            const bool want = !act && more;
-            if (__any_sync(kFull, want)) {
-                const int t = queue_take(want, &Q.next[warp]);
-                if (want) {
-                    if (t < count) {
-                        cur = Q.list[warp * 4 * kTileW + t];
-                        const int op = cur >> 2;
-                        q = get_pix<R, TM>(P, S, op);
-                        const float4 a = Q.ca[cur];
-                        const float2 b = Q.cb[cur];
-                        lane_start<R>(P, q, a.x, a.y, a.z, a.w, b.x, __float_as_int(b.y), Q.thr[op], &e);
-                        act = true;
-                    } else {
-                        more = false;
-                    }
-                }
-            }
-            if (!__any_sync(kFull, act)) break;
-            const bool fast = __all_sync(kFull, !act || e.fast);
-            const bool fastp = TM ? __all_sync(kFull, !act || !q.temporal || q.prev_fast) : true;
-            if (act) {
-                float r;
-                if (lane_step<R, TM, HW, true, false>(P, T, q, e, fast, fastp, &r)) {
-                    Q.ca[cur].x = r;
-                    act = false;
-                }
+            q = lane_pix<R>(P, px);
+            th = threshold_of(P, q, best);
+            if (head) {
+                E.thr[pid] = best;
+                put_pix<R>(E.S, pid, q);
             }
         }
     }
-    __syncthreads();
-    // phase 3: each pixel takes the first candidate, in the reference's
-    // order, that beats its running best
-    if (in && !culled) {
-        const int x = px.x, y = px.y;
-        const size_t k = (size_t)y * P.W + x;
-        const int codes = Q.slots[pid];
-        float best = Q.thr[pid];
+    float sum[CPL], v0[CPL];
+    alive = front_taps<R, TM, HW, CPL, H>(P, T, E.L, q, th, c, scale.y, alive, sum, v0);
+    const int n = queue_survivors<R, CPL>(P, E.Q[warp], pid, slot0, alive, c, sum, v0);
+    eval_queue<R, TM, HW, H>(P, T, E.S, E.L, E.Q[warp], n, E.thr, E.V[warp], E.energy);
+    __syncwarp();
+    // each pixel takes the first candidate, in the reference's order, that
+    // beats its running best
+    if (own && head) {
         int win = -1;
+        const float4 e4 = *reinterpret_cast<const float4*>(&E.energy[pid * 4]);
+        const float e[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
-        for (int cdx = 0; cdx < 4; cdx++) {
-            const int code = (codes >> (3 * cdx)) & 7;
-            // a skipped candidate or a repeat is rejected by "<"; one that
-            // test_offset rejected before the energy competes with 1e31
-            if (code < 2) continue;
-            const float r = code == 2 ? kBigResidual : Q.ca[pid * 4 + code - 3].x;
-            if (r < best) { best = r; win = cdx; }
-        }
+        for (int cdx = 0; cdx < 4; cdx++)
+            if (e[cdx] < best) { best = e[cdx]; win = cdx; }
+        const Patch old = load_patch(P.off, k);
         if (win >= 0) {
             int tx, ty;
             propagate_source(win, x, y, jump, &tx, &ty);
             const Patch ow = propagate_offset(P, tx, ty, x, y);
-            if (P.inc.on) P.inc.chg[k] = same_record(ow, load_patch(P.off, k)) ? 0 : 1;
+            if (P.inc.on) P.inc.chg[k] = same_record(ow, old) ? 0 : 1;
             store_patch(work, k, ow);
         } else {
             if (P.inc.on) P.inc.chg[k] = 0;
-            store_patch(work, k, load_patch(P.off, k));
+            store_patch(work, k, old);
         }
     }
 }
@@ -1096,7 +1464,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_scatter_q(const Params P, 
     load_tap_table<R>(P, TT);
     PixT px;
     bool abort;
-    const bool in = stage_tile<R, TM>(P, M, T, &px, &abort);  // (synchronises the block)
+    const bool in = stage_tile<R, TM>(P, M, T, threadIdx.x + threadIdx.y * kTileW, &px, &abort);  // (synchronises the block)
     if (abort) return;
     const int x = px.x, y = px.y;
     const size_t k = (size_t)y * P.W + x;
@@ -1252,7 +1620,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_residual_inc(const Params 
                                                                         float* out) {
     constexpr int TW = TileSmem<R, TM>::TW, N = TileSmem<R, TM>::N, K = (2 * R + 1) * (2 * R + 1);
     __shared__ TileSmem<R, TM> T;
-    __shared__ PixShared S;
+    __shared__ PixShared<> S;
     __shared__ float4 CA[kTileThreads];  // own record: x, y, sv, layer bits | fast << 30
     __shared__ float4 CB[kTileThreads];  // its basis
     __shared__ uint16_t list[kTileThreads * K];  // pid << 7 | tap
@@ -1293,7 +1661,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_residual_inc(const Params 
     if (!__syncthreads_or(need)) return;
     PixT px;
     bool abort;
-    stage_tile<R, TM>(P, M, T, &px, &abort);  // (synchronises the block)
+    stage_tile<R, TM>(P, M, T, pid, &px, &abort);  // (synchronises the block)
     if (abort) return;
     bool mine = false;
     int nt = 0;
@@ -1402,16 +1770,42 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_residual_inc(const Params 
     }
 }
 
+// Kernels with more shared memory than a static array may have: the
+// attribute that allows it is set once per kernel and device.
+template <class F>
+static cudaError_t allow_smem(F* kernel, size_t smem, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || (dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1))) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
+    return e;
+}
+
+template <int R, int TM, int HW, int CPL, int H>
+static cudaError_t launch_propagate_t(const Params& P, const TileMaps& M, PatchPlanes work, int jump,
+                                      cudaStream_t s) {
+    constexpr int NP = kTileW * H, NT = NP * 4 / CPL;
+    constexpr size_t smem =
+        (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(EvalSmem<R, NT / 32, NP, 32 * CPL>);
+    static std::atomic<uint64_t> done{0};
+    const cudaError_t e = allow_smem(kt_propagate<R, TM, HW, CPL, H>, smem, done);
+    if (e != cudaSuccess) return e;
+    const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
+    kt_propagate<R, TM, HW, CPL, H><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, work, jump);
+    return cudaGetLastError();
+}
+
 template <int R>
 cudaError_t launch_tiled_r(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
                            uint32_t pass_id, float* out, int wide, cudaStream_t s) {
-    dim3 b(kTileW, kTileH), bw(kTileW, 2 * kTileH), g((P.lw + kTileW - 1) / kTileW, (P.lh + kTileH - 1) / kTileH);
+    dim3 b(kTileW, kTileH), g((P.lw + kTileW - 1) / kTileW, (P.lh + kTileH - 1) / kTileH);
     // the texture-unit kernels fetch through the exemplar's textures, which
     // must be bound
     if (P.ex.hw && (!P.ex.tbase || !P.ex.tout)) return cudaErrorInvalidValue;
 #define PT_TILED_DISPATCH(TMV, HWV)                                                                   \
-    if (kind == 0 && wide) kt_propagate_q<R, TMV, HWV, 2><<<g, bw, 0, s>>>(P, M, work, arg);          \
-    else if (kind == 0) kt_propagate_q<R, TMV, HWV, 1><<<g, b, 0, s>>>(P, M, work, arg);             \
+    if (kind == 0 && wide) return launch_propagate_t<R, TMV, HWV, 1, kPropH>(P, M, work, arg, s);     \
+    else if (kind == 0) return launch_propagate_t<R, TMV, HWV, 2, kPropH>(P, M, work, arg, s);        \
     else if (kind == 1) kt_scatter_q<R, TMV, HWV><<<g, b, 0, s>>>(P, M, work, arg, pass_id);         \
     else if (P.inc.on || P.inc.fill) kt_residual_inc<R, TMV, HWV><<<g, b, 0, s>>>(P, M, out);        \
     else kt_residual<R, TMV, HWV><<<g, b, 0, s>>>(P, M, out);

@@ -64,7 +64,7 @@ pt_status pt_set_style(pt_ctx* c, int style, int w, int h, const float* base, co
     if ((int)c->style_levels.size() != nlev || c->style_levels[0].w != w || c->style_levels[0].h != h) {
         for (auto& L : c->style_levels) {
             dfree_t(c, L.base); dfree_t(c, L.out); dfree_t(c, L.bo); dfree_t(c, L.orient); dfree_t(c, L.dt);
-            dfree_t(c, L.ids);
+            dfree_t(c, L.ids); dfree_t(c, L.flags);
             free_textures(c, &L);
         }
         c->style_levels.assign(nlev, ExLevel());
@@ -79,6 +79,7 @@ pt_status pt_set_style(pt_ctx* c, int style, int w, int h, const float* base, co
             TRY(dalloc_t(c, &L.orient, n));
             TRY(dalloc_t(c, &L.dt, n));
             TRY(dalloc_t(c, &L.ids, n));
+            TRY(dalloc_t(c, &L.flags, (size_t)2));
         }
         c->style_set.assign(c->NS, 0);
     }

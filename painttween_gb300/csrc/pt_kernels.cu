@@ -152,12 +152,27 @@ __global__ void __launch_bounds__(128) k_residual(const Params P, float* out) {
 }
 
 // base and output exemplar texels interleaved into 32-byte records (the
-// tiled kernels fetch a texel's two colours with one 256-bit load)
-__global__ void k_interleave_texels(const float4* base, const float4* out, float4* bo, size_t n) {
+// tiled kernels fetch a texel's two colours with one 256-bit load), and what
+// they can do in ExView::flags (zeroed before): the candidate tests of a level
+// that is opaque, or whose distance transform culls nothing, need no gather.
+__global__ void k_interleave_texels(const float4* base, const float4* out, const float* dt, float4* bo, int* flags,
+                                    size_t n) {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    bo[2 * t] = base[t];
-    bo[2 * t + 1] = out[t];
+    bool transparent = false;
+    int far = 0;
+    if (t < n) {
+        const float4 o = out[t];
+        bo[2 * t] = base[t];
+        bo[2 * t + 1] = o;
+        transparent = !(o.w >= 0.995f);
+        far = max(__float_as_int(fmaxf(dt[t], 0.0f)), 0);  // (NaN: 0, it culls nothing)
+    }
+    transparent = __any_sync(0xffffffffu, transparent);
+    far = __reduce_max_sync(0xffffffffu, far);
+    if ((threadIdx.x & 31) == 0) {
+        if (transparent && !*(volatile int*)flags) atomicOr(flags, 1);
+        if (far > *(volatile int*)(flags + 1)) atomicMax(flags + 1, far);
+    }
 }
 
 // offsetsToOutput, :263-274
@@ -738,11 +753,14 @@ cudaError_t launch_random_level(int mode, int w, int h, int mx, int my, int tran
     }
     LAUNCH_CHECK();
 }
-cudaError_t launch_interleave_texels(const float4* base, const float4* out, float4* bo, size_t n, cudaStream_t s) {
+cudaError_t launch_interleave_texels(const float4* base, const float4* out, const float* dt, float4* bo, int* flags,
+                                     size_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
+    const cudaError_t e = cudaMemsetAsync(flags, 0, 2 * sizeof(int), s);
+    if (e != cudaSuccess) return e;
     const int threads = 256;
     const unsigned blocks = (unsigned)((n + threads - 1) / threads);
-    k_interleave_texels<<<blocks, threads, 0, s>>>(base, out, bo, n);
+    k_interleave_texels<<<blocks, threads, 0, s>>>(base, out, dt, bo, flags, n);
     LAUNCH_CHECK();
 }
 cudaError_t launch_any_transparent(const float4* out, size_t n, int* flag, cudaStream_t s) {

@@ -29,7 +29,7 @@ pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<fl
     int mx = (c->SW >> level) - 1, my = (c->SH >> level) - 1;
     if (mx < 1 || my < 1) return fail(c, PT_ERR_INVALID, "style too small for level %d", level);
     if (!c->rnd) TRY(dalloc_t(c, &c->rnd, (size_t)c->W * c->H));
-    ExView ex{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS};
+    ExView ex{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS, 0, 0, 0, c->ex->flags};
     int mode;
     uint32_t seed = (uint32_t)(frame * level);
     if (c->params.rngMode == PT_RNG_COUNTER) {

@@ -13,6 +13,7 @@ namespace ptk {
 constexpr int kMaxRadius = 15;  // taps per axis <= 31
 constexpr int kTileW = 32;      // pixel tile of the tiled kernels
 constexpr int kTileH = 8;
+constexpr int kPropH = 4;       // tile height of propagate
 
 // Offset field in three planes (SoA of the 36-byte PatchXF):
 //   A = (x, y, theta, layer as int bits), B = (hysteresis, scaleU, scaleV,
@@ -46,6 +47,8 @@ struct ExView {
     // the tiled kernels fetch through
     int hw;
     cudaTextureObject_t tbase, tout;
+    // [0]: some output alpha is below 0.995; [1]: the largest distance transform value (0 or more), its bits
+    const int* flags;
 };
 
 // A 2-D array of one pyramid level.  Image-side "layered" inputs (colour,
@@ -118,6 +121,7 @@ struct Params {
     int level, lw, lh;   // level and its size
     int r;               // patch radius
     float gauss[2 * kMaxRadius + 1];
+    float sumW;          // the weights of a whole window summed in the kernels' order (radius <= 4)
     float scaleWU, scaleWV;
     float alphaWeight, inputAnalogyWeight, canvasOutputWeight;
     float distTransWeight, styleObjIdWeight, coherenceWeight;
@@ -129,6 +133,7 @@ struct Params {
     int numStyles;
     int transparencyOk, orientationEnabled, lumShiftEnable;
     int distTransCull;
+    float exCull;        // an exemplar texel with a larger distance is culled: distTransCull * 1.25, rounded down
     int direction;
     int scatterSamples;
     int firstKey, lastKey;     // first and last keyframe layer (keyframe interpolation)
@@ -147,8 +152,8 @@ struct Params {
     AdvView adv[2];            // [0] = forward, [1] = backward
     unsigned long long* counters;  // profiling: energy evaluations, taps, temporal taps (null = off)
     int earlyExit;             // every per-tap term is >= 0 (all weights >= 0): candidates may stop early
-    // the taps of a patch window of radius <= 4 by descending weight (ties in
-    // the reference's order), tap t = (i + r) * (2r + 1) + (j + r)
+    // the taps of a patch window of radius <= 4, the 3 x 3 in the middle and
+    // then the others, each by descending weight; tap t = (i + r) * (2r + 1) + (j + r)
     uint8_t tapOrder[81];
     IncView inc;
 };
@@ -161,13 +166,13 @@ struct ConvKernel {
 // Tensor maps of the pixel-side planes a tiled kernel stages (each a float4
 // plane read as a FLOAT32 tensor of 4 * level width x level height, boxes of
 // one tile with its halo): the input colour, the canvas and, for temporal
-// passes, the advected colours and the advected records' B plane.  With
+// passes, the advected colours.  With
 // `on`, blocks whose tile and halo lie inside the level rectangle stage them
 // with tensor copies; the others (and every block without `on`) load them
 // with the clamp rules.  `err` is set when a block's wait for its copies
 // runs out.
 struct TileMaps {
-    CUtensorMap base, canvas, pbase, pout, prec;
+    CUtensorMap base, canvas, pbase, pout;
     int* err;
     int on;
 };
