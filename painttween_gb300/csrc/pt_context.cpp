@@ -620,6 +620,16 @@ static int propagate_variant(pt_ctx* c, const Params& P, int tm, int* probe) {
     return fallback;
 }
 
+// Scatter's lanes per pixel: four (1) for levels whose pixels leave the GPU
+// short of warps, two (0) for the others, whose warps then hold fewer
+// candidates that a win before them makes useless.  The line lies between the
+// sizes measured (summed launches, four / two lanes): all levels of a 128x128
+// still 0.44 / 0.64 ms, of four 512x512 frames 16.1 / 17.3 ms, of a 1024x1024
+// still 3.66 / 3.07 ms, of two 1080p frames 55.8 / 50.8 ms.
+static int scatter_wide(pt_ctx* c, const Params& P) {
+    return (long long)P.lw * P.lh <= 2048ll * sm_count(c);
+}
+
 cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,
                          float* out, bool* done) {
     *done = false;
@@ -627,9 +637,9 @@ cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work,
     int tm = temporal_mode(c);
     if (P.r < 2 || P.r > 4) return cudaSuccess;
     int probe = -1;
-    const int wide = kind == 0 ? propagate_variant(c, P, tm, &probe) : 0;
+    const int wide = kind == 0 ? propagate_variant(c, P, tm, &probe) : kind == 1 ? scatter_wide(c, P) : 0;
     TileMaps M;
-    tile_maps(c, P, tm, kind == 0 ? ptk::kPropH : ptk::kTileH, &M);
+    tile_maps(c, P, tm, kind == 2 ? ptk::kTileH : kind == 0 ? ptk::kPropH : wide ? ptk::kScatHWide : ptk::kScatH, &M);
     int blocks = 0;
     pt_ctx::Tune* t = probe >= 0 ? &c->tune[tune_key(c, P, tm, &blocks)] : nullptr;
     if (t) cudaEventRecord(t->ev[2 * probe], c->stream);

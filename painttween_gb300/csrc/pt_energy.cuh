@@ -517,14 +517,6 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_residual(const Params P, c
     out[k] = energy_tiled<R, TM, HW, false>(P, T, px, c, kNoBest);
 }
 
-// ---------------------------------------------------------------------------
-// Lane cursors.  Scatter's lanes each follow their own pixel's chain, one
-// column of 2R+1 taps per step, and take the next candidate as soon as the
-// current one is finished or stopped early.  A candidate's sum runs over its
-// taps in the reference's order, so every energy is bit-identical to a
-// separate evaluation.
-// ---------------------------------------------------------------------------
-
 constexpr unsigned kFull = 0xffffffffu;
 // (1 -/+ 2^-17): bounds of the rounding of a reference-order sum of <= 81 terms
 constexpr float kBoundLo = 1.0f - 1.0f / 131072.0f;
@@ -552,25 +544,6 @@ struct LaneEval {
     float thr2;  // exit threshold (see exit_threshold)
     float s0lo;  // lower bound of the start sum's share of the reference-order sum
 };
-
-// The taps of the window by descending weight, with their weights, for the
-// bound pass; filled once per block from Params::tapOrder.
-template <int R>
-struct TapTable {
-    uint8_t ij[(2 * R + 1) * (2 * R + 1)];  // (i + R) | (j + R) << 4
-    float w[(2 * R + 1) * (2 * R + 1)];
-};
-template <int R>
-__device__ __forceinline__ void load_tap_table(const Params& P, TapTable<R>& TT) {
-    constexpr int n = 2 * R + 1, K = n * n;
-    const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-    if (tid < K) {
-        const int t = P.tapOrder[tid];
-        const int i = t / n, j = t % n;
-        TT.ij[tid] = (uint8_t)(i | (j << 4));
-        TT.w[tid] = P.gauss[i] * P.gauss[j];
-    }
-}
 
 template <int R>
 __device__ __forceinline__ LanePix lane_pix(const Params& P, const PixT& px) {
@@ -729,150 +702,6 @@ __device__ __forceinline__ float tap_value(const Params& P, const TileSmem<R, TM
     TapSample t;
     tap_fetch<R, TM, HW>(P, q, e, i, j, fast, fastp, &t);
     return tap_finish<R, TM, HW>(P, T, q, e, i, j, t);
-}
-
-// the taps of column e.col added to e.sum in the reference's order.  ROLL
-// keeps the column's taps in a loop (a smaller body: faster for scatter,
-// whose chain code competes for the instruction cache; propagate unrolls).
-// EE: a lane leaves the column as soon as its sum reaches e.thr2 (the sum
-// only grows, so stopping at any tap gives the decision of stopping at the
-// column's end), and the loads of its remaining taps are not issued.
-// With the texture unit each tap's fetches are issued before the previous
-// tap's sum and exit test (one tap ahead), so two taps' fetch latencies
-// overlap; a lane that exits has fetched one tap more than it uses.
-template <int R, int TM, int HW, bool ROLL, bool EE>
-__device__ __forceinline__ float lane_column(const Params& P, const TileSmem<R, TM>& T, const LanePix& q,
-                                             const LaneEval& e, bool fast, bool fastp) {
-    const int i = e.col;
-    const bool cvalid = (i >= q.imin) && (i <= q.imax);
-    const float gi = P.gauss[i + R];
-    float sum = e.sum;
-    if constexpr (HW && !ROLL) {
-        TapSample cur, nxt;
-        tap_fetch<R, TM, HW>(P, q, e, i, -R, fast, fastp, &cur);
-#pragma unroll
-        for (int j = -R; j <= R; j++) {
-            if (j < R) tap_fetch<R, TM, HW>(P, q, e, i, j + 1, fast, fastp, &nxt);
-            const bool valid = cvalid && (j >= q.jmin) && (j <= q.jmax);
-            const float res = tap_finish<R, TM, HW>(P, T, q, e, i, j, cur);
-            const float w = gi * P.gauss[j + R];
-            sum = valid ? fmaf(res, w, sum) : sum;
-            if (EE && sum >= e.thr2) break;
-            cur = nxt;
-        }
-        return sum;
-    } else {
-#pragma unroll(ROLL ? 1 : 2 * R + 1)
-        for (int j = -R; j <= R; j++) {
-            const bool valid = cvalid && (j >= q.jmin) && (j <= q.jmax);
-            const float res = tap_value<R, TM, HW>(P, T, q, e, i, j, fast, fastp);
-            const float w = gi * P.gauss[j + R];
-            sum = valid ? fmaf(res, w, sum) : sum;
-            if (EE && sum >= e.thr2) break;
-        }
-        return sum;
-    }
-}
-
-// taps of the first `cols` columns inside the level rectangle
-template <int R>
-__device__ __forceinline__ unsigned lane_taps(const LanePix& q, int cols) {
-    const int last = min(-R + cols - 1, q.imax);
-    return last < q.imin ? 0u : (unsigned)((last - q.imin + 1) * (q.jmax - q.jmin + 1));
-}
-
-// One step of a lane: the next column (2R+1 taps) of its candidate in the
-// reference's order; returns true when the candidate is finished, with its
-// energy in *r (kBigResidual where the tap weights sum below kEpsilon, +inf
-// where it was rejected early).  The sum is formed as calculateResidual forms
-// it (texSynth_kernel.cu:537-659), exiting early on it.  (Propagate's
-// candidates come from coherent neighbours and mostly tie with the best, so
-// it takes this exact pass alone; scatter's chains take a bound pass first,
-// lane_step_uni below.)
-template <int R, int TM, int HW, bool EE, bool ROLL>
-__device__ __forceinline__ bool lane_step(const Params& P, const TileSmem<R, TM>& T, const LanePix& q, LaneEval& e,
-                                          bool fast, bool fastp, float* r) {
-    if (!e.exact) {
-        e.exact = true;
-        e.col = -R;
-        e.sum = q.sum0;
-    }
-    e.sum = lane_column<R, TM, HW, ROLL, EE>(P, T, q, e, fast, fastp);
-    e.col++;
-    const bool stop = EE && e.sum >= e.thr2;
-    if (!stop && e.col <= R) return false;
-    if (P.counters) count_taps(P, lane_taps<R>(q, e.col + R), q.temporal);
-    *r = (q.sumW < kEpsilon) ? kBigResidual : stop ? INFINITY : e.sum / q.sumW;
-    return true;
-}
-
-// One step of a lane of scatter's chains: with an exit threshold a
-// candidate first takes a bound pass, its taps by descending weight (TT),
-// accumulating a lower bound of the weighted sum with round-down products and
-// sums.  The reference forms its sum in tap order with round-to-nearest fmaf
-// over at most 81 non-negative terms, which is at least (1 - 2^-17) times the
-// exact sum of those terms, plus its start sum (the hysteresis term, <= 0)
-// scaled by at most (1 + 2^-17).  So once (1 - 2^-17) * bound + that
-// start-sum share, rounded down, reaches thr2 = best * sumW rounded up, the
-// reference-order energy is >= best and the strict "<" rejects the
-// candidate.  The heavy central taps come first, so a rejection needs a few
-// taps instead of several columns.  A candidate the bound pass does not
-// reject (a winner or a near tie) then takes the exact pass, lane_step's.
-// Both passes share one loop body: a step is up to 2R+1 taps, by descending
-// weight (bound pass: round-down products and sums, the bound test) or the
-// next column in the reference's order (exact pass: fmaf, the exact test),
-// chosen per lane by data, so the lanes of a warp in different passes issue
-// the same instructions instead of the two passes' code in turn.
-template <int R, int TM, int HW>
-__device__ __forceinline__ bool lane_step_uni(const Params& P, const TileSmem<R, TM>& T, const TapTable<R>& TT,
-                                              const LanePix& q, LaneEval& e, bool fast, bool fastp, float* r) {
-    constexpr int K = (2 * R + 1) * (2 * R + 1);
-    const bool bound = !e.exact;
-    bool hit = false;  // the pass's test reached its threshold
-#pragma unroll 1
-    for (int k = 0; k < 2 * R + 1; k++) {
-        const int pos = e.col + k;
-        if (bound && pos >= K) break;
-        int i, j;
-        float w;
-        if (bound) {
-            const int ij = TT.ij[pos];
-            i = (ij & 15) - R;
-            j = (ij >> 4) - R;
-            w = TT.w[pos];
-        } else {
-            i = e.col;
-            j = k - R;
-            w = P.gauss[i + R] * P.gauss[j + R];
-        }
-        const bool valid = (i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax);
-        const float res = tap_value<R, TM, HW>(P, T, q, e, i, j, fast, fastp);
-        const float sb = __fadd_rd(e.sum, __fmul_rd(res, w));
-        const float sx = fmaf(res, w, e.sum);
-        e.sum = valid ? (bound ? sb : sx) : e.sum;
-        hit = bound ? (__fadd_rd(__fmul_rd(e.sum, kBoundLo), e.s0lo) >= e.thr2) : (e.sum >= e.thr2);
-        if (hit) break;
-    }
-    if (bound) {
-        e.col += 2 * R + 1;
-        if (hit) {
-            if (P.counters) count_taps(P, (unsigned)min(e.col, K), q.temporal);
-            *r = INFINITY;
-            return true;
-        }
-        if (e.col >= K) {  // not rejected: the exact pass
-            if (P.counters) count_taps(P, (unsigned)K, q.temporal);
-            e.exact = true;
-            e.col = -R;
-            e.sum = q.sum0;
-        }
-        return false;
-    }
-    e.col++;
-    if (!hit && e.col <= R) return false;
-    if (P.counters) count_taps(P, lane_taps<R>(q, e.col + R), q.temporal);
-    *r = (q.sumW < kEpsilon) ? kBigResidual : hit ? INFINITY : e.sum / q.sumW;
-    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1069,7 +898,7 @@ struct WarpQueue {
     float4 a[CAP];     // x, y, b0
     float4 b[CAP];     // b1, the bound so far, layer bits
     float v0[CAP];     // the middle tap's value
-    uint16_t id[CAP];  // pid * 4 + slot | fast << 15
+    uint16_t id[CAP];  // pid * CH + slot | fast << 15
 };
 
 // The front pass over NC candidates of pixel q (bit c of `alive`: candidate c
@@ -1078,7 +907,7 @@ struct WarpQueue {
 template <int R, int TM, int HW, int NC, int H>
 __device__ __forceinline__ unsigned front_taps(const Params& P, const TileSmem<R, TM, H>& T, const TapList<R>& L,
                                                const LanePix& q, const Threshold& th, const CandPos (&c)[NC],
-                                               float sv, unsigned alive, float (&sum)[NC],
+                                               const float (&sv)[NC], unsigned alive, float (&sum)[NC],
                                                float (&v0)[NC]) {
     constexpr int TW = TileSmem<R, TM>::TW;
     bool in = true;  // every footprint of the lane inside the exemplar
@@ -1112,7 +941,7 @@ __device__ __forceinline__ unsigned front_taps(const Params& P, const TileSmem<R
             if ((on >> k) & 1) {
                 float r = tap_terms<TM>(P, p, s[k], v, t == 0);
                 if (t == 0) {
-                    r = center_terms<HW>(P, q, c[k].layer, sv, tx[k], ty[k], r);
+                    r = center_terms<HW>(P, q, c[k].layer, sv[k], tx[k], ty[k], r);
                     v0[k] = r;
                 }
                 sum[k] = __fmaf_rd(r, tp.w, sum[k]);
@@ -1127,7 +956,7 @@ __device__ __forceinline__ unsigned front_taps(const Params& P, const TileSmem<R
 // The lane's surviving candidates appended to its warp's queue; returns the
 // queue's length (the same for every lane).
 template <int R, int NC, int CAP>
-__device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& Q, int pid, int slot0, unsigned alive,
+__device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& Q, int id0, unsigned alive,
                                                const CandPos (&c)[NC], const float (&sum)[NC], const float (&v0)[NC]) {
     const int n = __popc(alive);
     int incl = n;
@@ -1144,7 +973,7 @@ __device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& 
             Q.a[w] = make_float4(c[k].x, c[k].y, c[k].b0.x, c[k].b0.y);
             Q.b[w] = make_float4(c[k].b1.x, c[k].b1.y, sum[k], __int_as_float(c[k].layer));
             Q.v0[w] = v0[k];
-            Q.id[w] = (uint16_t)((pid * 4 + slot0 + k) | (in ? 1 << 15 : 0));
+            Q.id[w] = (uint16_t)((id0 + k) | (in ? 1 << 15 : 0));
             w++;
         }
     __syncwarp();
@@ -1152,10 +981,10 @@ __device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& 
 }
 
 // Evaluates the first n candidates of the warp's queue, a group of kGroup
-// lanes each; energies of those that no bound rejects into energy[pid * 4 +
+// lanes each; energies of those that no bound rejects into energy[pid * CH +
 // slot].  thr: the energy to beat of each pixel of the tile; V: (2R+1)^2
 // values of each of the warp's groups.
-template <int R, int TM, int HW, int H, int CAP>
+template <int R, int TM, int HW, int H, int CAP, int CH>
 __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM, H>& T,
                                            const PixShared<kTileW * H>& S, const TapList<R>& L,
                                            const WarpQueue<CAP>& Q, int n, const float* thr,
@@ -1182,14 +1011,14 @@ __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM
                 const float4 a = Q.a[t], b = Q.b[t];
                 id = Q.id[t];
                 cfast = (id >> 15) & 1;
-                id &= 1023;
+                id &= 0x7fff;
                 c.x = a.x; c.y = a.y;
                 c.b0 = make_float2(a.z, a.w);
                 c.b1 = make_float2(b.x, b.y);
                 c.layer = __float_as_int(b.w);
                 sum = b.z;
-                q = get_pix<R, TM>(P, S, id >> 2);
-                th = threshold_of(P, q, thr[id >> 2]);
+                q = get_pix<R, TM>(P, S, id / CH);
+                th = threshold_of(P, q, thr[id / CH]);
                 if (l == 0) val[K / 2] = Q.v0[t];
                 step = 0;
                 act = true;
@@ -1252,14 +1081,14 @@ __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM
 
 // the energy phase's shared state of a block of NW warps over NP pixels, each
 // warp with up to CAP surviving candidates
-template <int R, int NW, int NP, int CAP>
+template <int R, int NW, int NP, int CAP, int CH>
 struct EvalSmem {
     PixShared<NP> S;
     WarpQueue<CAP> Q[NW];
     TapList<R> L;
     float V[NW][kGroups * (2 * R + 1) * (2 * R + 1)];
     float thr[NP];                    // the energy each pixel has to beat
-    alignas(16) float energy[NP * 4];  // per candidate: its energy, +inf where it lost or is none
+    alignas(16) float energy[NP * CH];  // per candidate (CH a pixel): its energy, +inf where it lost or is none
 };
 
 // calculatePropagateOffset, texSynth_kernel.cu:956-982 (propagate_offset), for
@@ -1313,7 +1142,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     kt_propagate(const Params P, const __grid_constant__ TileMaps M, PatchPlanes work, int jump) {
     constexpr int NP = kTileW * H, NT = NP * 4 / CPL, NW = NT / 32, PPW = 8 * CPL;  // PPW: pixels per warp
     using Tile = TileSmem<R, TM, H>;
-    using Eval = EvalSmem<R, NW, NP, 32 * CPL>;
+    using Eval = EvalSmem<R, NW, NP, 32 * CPL, 4>;
     extern __shared__ __align__(128) unsigned char dyn[];
     Tile& T = *reinterpret_cast<Tile*>(dyn);
     Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
@@ -1357,7 +1186,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     // the candidates, in the reference's order (repeats and test_offset
     // rejections resolved here)
     CandPos c[CPL];
-    float2 scale = make_float2(1.f, 1.f);
+    float sv[CPL];
     unsigned alive = 0;
     bool own = false;
     LanePix q;
@@ -1376,7 +1205,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
         } else {
             own = true;
             best = __ldg(P.res + k);
-            scale = lvl_texel_lin(P.img.scale, x, y, P.hwFilter);
+            const float2 scale = lvl_texel_lin(P.img.scale, x, y, P.hwFilter);
             PropCand pc[CPL];
             propagate_candidates<CPL>(P, x, y, slot0, jump, scale, pc);
             const bool opaque = P.transparencyOk || !exemplar_transparent(P.ex);
@@ -1385,6 +1214,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
 #pragma unroll
             for (int i = 0; i < CPL; i++) {
                 c[i] = pc[i].c;
+                sv[i] = scale.y;
                 float e = INFINITY;  // skipped, a repeat, or lost: rejected by "<"
                 bool dup = false;
 #pragma unroll
@@ -1414,9 +1244,9 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
         }
     }
     float sum[CPL], v0[CPL];
-    alive = front_taps<R, TM, HW, CPL, H>(P, T, E.L, q, th, c, scale.y, alive, sum, v0);
-    const int n = queue_survivors<R, CPL>(P, E.Q[warp], pid, slot0, alive, c, sum, v0);
-    eval_queue<R, TM, HW, H>(P, T, E.S, E.L, E.Q[warp], n, E.thr, E.V[warp], E.energy);
+    alive = front_taps<R, TM, HW, CPL, H>(P, T, E.L, q, th, c, sv, alive, sum, v0);
+    const int n = queue_survivors<R, CPL>(P, E.Q[warp], pid * 4 + slot0, alive, c, sum, v0);
+    eval_queue<R, TM, HW, H, 32 * CPL, 4>(P, T, E.S, E.L, E.Q[warp], n, E.thr, E.V[warp], E.energy);
     __syncwarp();
     // each pixel takes the first candidate, in the reference's order, that
     // beats its running best
@@ -1441,51 +1271,77 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     }
 }
 
-// scatter_kernel + averageOffset, texSynth_kernel.cu:841-952, each lane
-// running its own pixel's chain with a lane cursor
-template <int R, int TM, int HW>
-__global__ void __launch_bounds__(kTileThreads, 2) kt_scatter_q(const Params P, const __grid_constant__ TileMaps M,
-                                                                     PatchPlanes work, int write_all,
-                                                               uint32_t pass_id) {
-    __shared__ TileSmem<R, TM> T;
+// scatter_kernel + averageOffset, texSynth_kernel.cu:841-952, over tiles of
+// 32 x H pixels.  A pixel's chain is up to 25 candidates around its running
+// best offset, then the average of its neighbours.  Few of them win, so LPP
+// lanes of the pixel's own take the next LPP * NC of them at once, as they
+// follow if none of those before wins; the first, in the chain's order, that
+// beats the best is taken, and the chain goes on behind it from there.  Their
+// energies go the way of propagate's candidates (front pass, then the warp's
+// queue).
+// Before this, a lane ran its pixel's chain one candidate after the other, so
+// a launch took as long as the longest chains of its warps.  Measured, summed
+// launches: 128x128 still 1.90 -> 0.44 ms, 1024x1024 still 5.6 -> 3.1 ms, two
+// 1080p frames 67 -> 49 ms.  Eight lanes a pixel measured 41-55 % slower than
+// four, tiles of eight rows 5-9 % slower than four with two lanes, three
+// blocks an SM (80 registers) 9-30 % slower than two.
+template <int R, int TM, int HW, int LPP, int H>
+__global__ void __launch_bounds__(kTileW * H * LPP, 2)
+    kt_scatter(const Params P, const __grid_constant__ TileMaps M, PatchPlanes work, int write_all,
+               uint32_t pass_id) {
+    constexpr int NC = 2, CH = NC * LPP;
+    constexpr int NP = kTileW * H, NT = NP * LPP, NW = NT / 32, PPW = 32 / LPP;
+    using Tile = TileSmem<R, TM, H>;
+    using Eval = EvalSmem<R, NW, NP, 32 * NC, CH>;
+    extern __shared__ __align__(128) unsigned char dyn[];
+    Tile& T = *reinterpret_cast<Tile*>(dyn);
+    Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    const int tid = threadIdx.x + threadIdx.y * kTileW, warp = tid / 32, lane = tid % 32;
+    const int pid = warp * PPW + lane % PPW, sub = lane / PPW;
+    const bool head = sub == 0;  // the lane that writes its pixel
     // Change tracking: with the reference's generator a pixel's candidates
     // follow from its own record and its 3x3 neighbours, so a pixel whose
     // patch window is unchanged since the previous scatter of the loop had
     // every candidate rejected there against the same residual, and again now.
     bool stable = false;
     if (P.inc.on) {
-        const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
+        const int x = blockIdx.x * kTileW + pid % kTileW, y = blockIdx.y * H + pid / kTileW;
         const bool in = x < P.lw && y < P.lh;
         const size_t k = (size_t)y * P.W + x;
         stable = in && P.inc.prev != INT_MIN && __ldg(P.inc.win + k) < P.inc.prev;
-        if (block_idle(P, work, in && !stable, in, k, write_all != 0)) return;
+        if (block_idle(P, work, in && !stable, in && head, k, write_all != 0)) return;
     }
-    __shared__ TapTable<R> TT;
-    load_tap_table<R>(P, TT);
+    load_tap_list<R>(P, E.L, tid);
     PixT px;
     bool abort;
-    const bool in = stage_tile<R, TM>(P, M, T, threadIdx.x + threadIdx.y * kTileW, &px, &abort);  // (synchronises the block)
+    const bool in = stage_tile<R, TM, NT, H>(P, M, T, pid, &px, &abort);  // (synchronises the block)
     if (abort) return;
     const int x = px.x, y = px.y;
-    const size_t k = (size_t)y * P.W + x;
+    const size_t k = in ? (size_t)y * P.W + x : 0;
     bool own = false;
     if (in) {
         if (stable || image_culled(P, x, y)) {
-            if (write_all) store_patch(work, k, load_patch(P.off, k));
-            if (P.inc.on) P.inc.chg[k] = 0;
+            if (head) {
+                if (write_all) store_patch(work, k, load_patch(P.off, k));
+                if (P.inc.on) P.inc.chg[k] = 0;
+            }
         } else {
             own = true;
         }
     }
-    // chain state (the reference's loop, :896-937)
+    // chain state (the reference's loop, :896-937), the same in all of the
+    // pixel's lanes
+    const float closest = 10.f, factor = 0.9f;
     const float cached = own ? __ldg(P.res + k) : 0.0f;
     float best = (float)((double)cached + 10e-7);
     float owx = 0.f, owy = 0.f, owt = 0.f;  // running best offset
     int wkind = 0;                           // 0: the pixel's own, 1: a chain candidate, 2: the average
     float ia = 0.f, dist = 0.f;
-    float2 sc = make_float2(0.f, 0.f);
-    float avgx = 0.f, avgy = 0.f, avgt = 0.f;
+    float2 sc = make_float2(1.f, 1.f);
+    float avgx = 0.f, avgy = 0.f;
     LanePix q;
+    q.temporal = false;
+    q.prev_fast = true;
     if (own) {
         const float4 a = __ldg(P.off.A + k);
         owx = a.x; owy = a.y;
@@ -1494,10 +1350,12 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_scatter_q(const Params P, 
         sc = lvl_texel_lin(P.img.scale, x, y, P.hwFilter);
         // averageOffset of the base field (:841-861)
         int na = 0;
+#pragma unroll
         for (int i = -1; i <= 1; i++)
+#pragma unroll
             for (int j = -1; j <= 1; j++) {
                 if (!in_rect(P, x + i, y + j) || (i == 0 && j == 0)) continue;
-                float4 nb = __ldg(P.off.A + (size_t)(y + j) * P.W + (x + i));
+                const float4 nb = __ldg(P.off.A + (size_t)(y + j) * P.W + (x + i));
                 if (__float_as_int(nb.w) != 0) continue;
                 avgx = avgx + nb.x;
                 avgy = avgy + nb.y;
@@ -1505,43 +1363,57 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_scatter_q(const Params P, 
             }
         avgx = avgx / (float)na;
         avgy = avgy / (float)na;
-        avgt = screen_to_exemplar_angle(P, x, y, avgx, avgy, 0);
         q = lane_pix<R>(P, px);
+        if (head) put_pix<R>(E.S, pid, q);
     }
-    const float closest = 10.f, factor = 0.9f;
+    const bool opaque = P.transparencyOk || !exemplar_transparent(P.ex) || !(ia > kAlphaThreshold);
+    const bool culls = exemplar_culls(P.ex, P.exCull);
     uint32_t lastx = 0xffffffffu, lasty = 0xffffffffu;
-    int i = 0;
-    bool avg_pending = true;
-    LaneEval e;
-    bool act = false, more = own;
-    bool cur_avg = false;
-    float cur_t = 0.f;
+    int next = 0;                 // the chain's next candidate
+    bool avg_pending = true, more = own;
 #pragma unroll 1
-    while (true) {
-        if (!act && more) {
-            // the next candidate that needs an energy; one that test_offset
-            // rejects first competes with 1e31 right here
+    while (__any_sync(kFull, more)) {
+        // the next CH candidates; the lane keeps its own NC
+        CandPos c[NC];
+        float sv[NC], theta[NC], cdist[NC];
+        int kind[NC], cnext[NC];  // 0: none; where the chain goes on behind the candidate
+#pragma unroll
+        for (int s = 0; s < NC; s++) {
+            c[s] = CandPos{0.f, 0.f, make_float2(0.f, 0.f), make_float2(0.f, 0.f), 0};
+            sv[s] = 1.f;
+            theta[s] = cdist[s] = 0.f;
+            kind[s] = cnext[s] = 0;
+        }
+        const uint32_t lastx0 = lastx, lasty0 = lasty;
+        bool any = false;
+        if (more) {
 #pragma unroll 1
-            while (true) {
+            for (int s = 0; s < CH; s++) {
                 bool have = false;
                 float ex = 0.f, ey = 0.f;
 #pragma unroll 1
-                while (i < P.scatterSamples && dist * factor >= closest) {
-                    float dmin = dist * factor;
+                while (next < P.scatterSamples && dist * factor >= closest) {
+                    const float dmin = dist * factor;
                     if (P.rngMode == PT_RNG_COUNTER) {
-                        float rr = counter_u01(P.rngSeed, pass_id, x, y, 2 * i);
-                        float th = counter_u01(P.rngSeed, pass_id, x, y, 2 * i + 1) * 6.28318530717958647692f;
-                        float sn, cs;
-                        sincos_poly(th, &sn, &cs);
-                        float len = fmaf(rr, dist - dmin, dmin);
-                        ex = fmaf(cs, len, owx);
-                        ey = fmaf(sn, len, owy);
-                    } else {
-                        ex = owx + dmin;
-                        ey = owy + 0.0f;
+                        if (s / NC == sub) {
+                            const float rr = counter_u01(P.rngSeed, pass_id, x, y, 2 * next);
+                            const float th = counter_u01(P.rngSeed, pass_id, x, y, 2 * next + 1) * 6.28318530717958647692f;
+                            float sn, cs;
+                            sincos_poly(th, &sn, &cs);
+                            const float len = fmaf(rr, dist - dmin, dmin);
+                            ex = fmaf(cs, len, owx);
+                            ey = fmaf(sn, len, owy);
+                            clamp_to_exemplar(&ex, &ey, P.ex.w, P.ex.h);
+                        }
+                        next++;
+                        dist *= factor;
+                        have = true;
+                        break;
                     }
+                    ex = owx + dmin;
+                    ey = owy + 0.0f;
                     clamp_to_exemplar(&ex, &ey, P.ex.w, P.ex.h);
-                    i++;
+                    next++;
                     dist *= factor;
                     // an exact repeat of the previous candidate has its energy
                     // and is rejected by the strict "<"
@@ -1551,52 +1423,89 @@ __global__ void __launch_bounds__(kTileThreads, 2) kt_scatter_q(const Params P, 
                     have = true;
                     break;
                 }
-                float cx, cy, ct, csu, csv;
-                if (have) {
-                    cx = ex; cy = ey; ct = screen_to_exemplar_angle(P, x, y, ex, ey, 0);
-                    csu = sc.x; csv = sc.y;
-                } else if (avg_pending) {
-                    cx = avgx; cy = avgy; ct = avgt; csu = 1.f; csv = 1.f;
+                int kd = 1;
+                if (!have) {
+                    if (!avg_pending) break;
                     avg_pending = false;
-                } else {
-                    more = false;
-                    break;
+                    kd = 2;
+                    ex = avgx;
+                    ey = avgy;
                 }
-                bool ok = !((double)ex_texel_dt(ex_mode<HW>(P.ex), (int)cx, (int)cy, 0) > (double)P.distTransCull * 1.25);
-                if (ok && !P.transparencyOk) {
-                    float ea = ex_sample_out_alpha(ex_mode<HW>(P.ex), cx, cy, 0);
-                    ok = !(ea < kAlphaThreshold && ia > kAlphaThreshold);
-                }
-                if (!ok) {
-                    if (kBigResidual < best) {
-                        best = kBigResidual;
-                        owx = cx; owy = cy; owt = ct; wkind = have ? 1 : 2;
+                any = true;
+#pragma unroll
+                for (int z = 0; z < NC; z++)
+                    if (s == sub * NC + z) {
+                        c[z].x = ex;
+                        c[z].y = ey;
+                        kind[z] = kd;
+                        cnext[z] = next;
+                        cdist[z] = dist;
                     }
-                    continue;
-                }
-                if (P.counters) count_eval(P, x, y, px.temporal, false);
-                lane_start<R>(P, q, cx, cy, ct, csu, csv, 0, best, &e);
-                cur_avg = !have;
-                cur_t = ct;
-                act = true;
-                break;
             }
         }
-        if (!__any_sync(kFull, act)) break;
-        const bool fast = __all_sync(kFull, !act || e.fast);
-        const bool fastp = TM ? __all_sync(kFull, !act || !q.temporal || q.prev_fast) : true;
-        if (act) {
-            float r;
-            if (lane_step_uni<R, TM, HW>(P, T, TT, q, e, fast, fastp, &r)) {
-                if (r < best) {
-                    best = r;
-                    owx = e.cx; owy = e.cy; owt = cur_t; wkind = cur_avg ? 2 : 1;
+        unsigned alive = 0;
+#pragma unroll
+        for (int z = 0; z < NC; z++) {
+            float e = INFINITY;
+            if (kind[z]) {
+                theta[z] = screen_to_exemplar_angle(P, x, y, c[z].x, c[z].y, 0);
+                const float su = kind[z] == 1 ? sc.x : 1.f;
+                sv[z] = kind[z] == 1 ? sc.y : 1.f;
+                basis(theta[z], P.scaleWU * su, P.scaleWV * sv[z], &c[z].b0, &c[z].b1);
+                bool ok = !culls || !(ex_texel_dt(ex_mode<HW>(P.ex), (int)c[z].x, (int)c[z].y, 0) > P.exCull);
+                if (ok && !opaque) ok = !(ex_out_alpha<HW>(P.ex, c[z].x, c[z].y, 0) < kAlphaThreshold);
+                if (ok) {
+                    alive |= 1u << z;
+                    if (P.counters) count_eval(P, x, y, px.temporal, false);
+                } else {
+                    e = kBigResidual;  // rejected before the energy: competes with 1e31
                 }
-                act = false;
+            }
+            if (more) E.energy[pid * CH + sub * NC + z] = e;
+        }
+        const Threshold th = threshold_of(P, q, more ? best : kNoBest);
+        if (more && head) E.thr[pid] = best;
+        float sum[NC], v0[NC];
+        alive = front_taps<R, TM, HW, NC, H>(P, T, E.L, q, th, c, sv, alive, sum, v0);
+        const int n = queue_survivors<R, NC>(P, E.Q[warp], pid * CH + sub * NC, alive, c, sum, v0);
+        eval_queue<R, TM, HW, H, 32 * NC, CH>(P, T, E.S, E.L, E.Q[warp], n, E.thr, E.V[warp], E.energy);
+        __syncwarp();
+        // the first candidate that beats the best, if any
+        int win = -1;
+        if (more) {
+#pragma unroll
+            for (int s = CH - 1; s >= 0; s--) {
+                const float r = E.energy[pid * CH + s];
+                win = r < best ? s : win;
             }
         }
+        const int src = (win < 0 ? sub : win / NC) * PPW + lane % PPW;
+        float wx = 0.f, wy = 0.f, wt = 0.f, wd = 0.f;
+        int wn = 0, wk = 0;
+#pragma unroll
+        for (int z = 0; z < NC; z++) {
+            const float tx = __shfl_sync(kFull, c[z].x, src), ty = __shfl_sync(kFull, c[z].y, src);
+            const float tt = __shfl_sync(kFull, theta[z], src), td = __shfl_sync(kFull, cdist[z], src);
+            const int tn = __shfl_sync(kFull, cnext[z], src), tk = __shfl_sync(kFull, kind[z], src);
+            if (win % NC == z) { wx = tx; wy = ty; wt = tt; wd = td; wn = tn; wk = tk; }
+        }
+        if (more) {
+            if (win >= 0) {
+                best = E.energy[pid * CH + win];
+                owx = wx; owy = wy; owt = wt;
+                wkind = wk;
+                next = wn;
+                dist = wd;
+                avg_pending = wk != 2;
+                lastx = __float_as_uint(wx);
+                lasty = __float_as_uint(wy);
+                if (wk == 2) { lastx = lastx0; lasty = lasty0; }
+            }
+            more = any && (avg_pending || next < P.scatterSamples && dist * factor >= closest);
+        }
+        __syncwarp();
     }
-    if (!own) return;
+    if (!own || !head) return;
     const Patch off = load_patch(P.off, k);
     Patch ow = off;
     if (wkind == 1) ow = make_patch(owx, owy, owt, 0.0f, 0, sc.x, sc.y);
@@ -1787,12 +1696,26 @@ static cudaError_t launch_propagate_t(const Params& P, const TileMaps& M, PatchP
                                       cudaStream_t s) {
     constexpr int NP = kTileW * H, NT = NP * 4 / CPL;
     constexpr size_t smem =
-        (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(EvalSmem<R, NT / 32, NP, 32 * CPL>);
+        (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(EvalSmem<R, NT / 32, NP, 32 * CPL, 4>);
     static std::atomic<uint64_t> done{0};
     const cudaError_t e = allow_smem(kt_propagate<R, TM, HW, CPL, H>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
     kt_propagate<R, TM, HW, CPL, H><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, work, jump);
+    return cudaGetLastError();
+}
+
+template <int R, int TM, int HW, int LPP, int H>
+static cudaError_t launch_scatter_t(const Params& P, const TileMaps& M, PatchPlanes work, int write_all,
+                                    uint32_t pass_id, cudaStream_t s) {
+    constexpr int NP = kTileW * H, NT = NP * LPP;
+    constexpr size_t smem =
+        (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(EvalSmem<R, NT / 32, NP, 64, 2 * LPP>);
+    static std::atomic<uint64_t> done{0};
+    const cudaError_t e = allow_smem(kt_scatter<R, TM, HW, LPP, H>, smem, done);
+    if (e != cudaSuccess) return e;
+    const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
+    kt_scatter<R, TM, HW, LPP, H><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, work, write_all, pass_id);
     return cudaGetLastError();
 }
 
@@ -1806,7 +1729,9 @@ cudaError_t launch_tiled_r(int kind, int tm, const Params& P, const TileMaps& M,
 #define PT_TILED_DISPATCH(TMV, HWV)                                                                   \
     if (kind == 0 && wide) return launch_propagate_t<R, TMV, HWV, 1, kPropH>(P, M, work, arg, s);     \
     else if (kind == 0) return launch_propagate_t<R, TMV, HWV, 2, kPropH>(P, M, work, arg, s);        \
-    else if (kind == 1) kt_scatter_q<R, TMV, HWV><<<g, b, 0, s>>>(P, M, work, arg, pass_id);         \
+    else if (kind == 1 && wide)                                                                        \
+        return launch_scatter_t<R, TMV, HWV, 4, kScatHWide>(P, M, work, arg, pass_id, s);             \
+    else if (kind == 1) return launch_scatter_t<R, TMV, HWV, 2, kScatH>(P, M, work, arg, pass_id, s);  \
     else if (P.inc.on || P.inc.fill) kt_residual_inc<R, TMV, HWV><<<g, b, 0, s>>>(P, M, out);        \
     else kt_residual<R, TMV, HWV><<<g, b, 0, s>>>(P, M, out);
     if (P.ex.hw) {

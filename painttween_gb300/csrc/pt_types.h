@@ -14,6 +14,8 @@ constexpr int kMaxRadius = 15;  // taps per axis <= 31
 constexpr int kTileW = 32;      // pixel tile of the tiled kernels
 constexpr int kTileH = 8;
 constexpr int kPropH = 4;       // tile height of propagate
+constexpr int kScatH = 4;       // of scatter with two lanes per pixel
+constexpr int kScatHWide = 2;   // and with four
 
 // Offset field in three planes (SoA of the 36-byte PatchXF):
 //   A = (x, y, theta, layer as int bits), B = (hysteresis, scaleU, scaleV,
