@@ -111,6 +111,7 @@ struct PixCtx {
     Patch prevF, prevB;
     float2 fb0, fb1, bb0, bb1;
     float hyst;
+    float sumW;  // the weights of the window's taps inside the level rectangle, in tap order
 };
 
 // hysteresisTerm, :506-535
@@ -145,6 +146,21 @@ static __device__ void make_pixctx(const Params& P, int x, int y, PixCtx* pc) {
         basis(a, P.scaleWU * pc->prevB.su, P.scaleWV * pc->prevB.sv, &pc->bb0, &pc->bb1);
     }
     pc->hyst = pc->validF ? hysteresis_term(P, x, y) : 0.0f;
+    const int i0 = max(-P.r, -x), i1 = min(P.r, P.lw - 1 - x), j0 = max(-P.r, -y), j1 = min(P.r, P.lh - 1 - y);
+    float sw = 0.0f;
+    for (int i = i0; i <= i1; i++)
+        for (int j = j0; j <= j1; j++) sw = sw + P.gauss[i + P.r] * P.gauss[j + P.r];
+    pc->sumW = sw;
+}
+
+// Early exit of a patch distance whose per-tap terms are all >= 0
+// (Params::earlyExit; the coherence term, whose range depends on its
+// parameters, goes without): the running sum never decreases, so once it
+// reaches best * sumW rounded up the energy is >= best and the strict "<"
+// rejects the candidate.  NaN, which stops nothing, otherwise.
+static __device__ __forceinline__ float energy_limit(const Params& P, const PixCtx& pc, float best) {
+    return (P.earlyExit && !(P.coherenceWeight > 0.f) && pc.sumW >= kEpsilon) ? __fmul_ru(best, pc.sumW)
+                                                                             : __int_as_float(0x7fc00000);
 }
 
 // timeDerivativeTerms, :438-469
@@ -196,10 +212,10 @@ static __device__ float coherence_term(const Params& P, int x, int y, int i, int
 
 static __device__ __forceinline__ int f2i(float v) { return (int)v; }  // cvt.rzi: saturating, NaN -> 0
 
-// calculateResidual, :537-659
-static __device__ float energy(const Params& P, int x, int y, const Patch& t, const PixCtx& pc) {
+// calculateResidual, :537-659; +inf once the sum reaches `limit` (energy_limit)
+static __device__ float energy(const Params& P, int x, int y, const Patch& t, const PixCtx& pc, float limit) {
     const int r = P.r;
-    float sumW = 0.0f, sum = 0.0f;
+    float sum = 0.0f;
     if (pc.validF) sum = sum - pc.hyst;
     float2 b0, b1;
     basis(t.theta, P.scaleWU * t.su, P.scaleWV * t.sv, &b0, &b1);
@@ -261,11 +277,11 @@ static __device__ float energy(const Params& P, int x, int y, const Patch& t, co
             }
             float w = P.gauss[i + r] * P.gauss[j + r];
             sum = fmaf(res, w, sum);
-            sumW = sumW + w;
+            if (sum >= limit) return INFINITY;
         }
     }
-    if (sumW < kEpsilon) return kBigResidual;
-    return sum / sumW;
+    if (pc.sumW < kEpsilon) return kBigResidual;
+    return sum / pc.sumW;
 }
 
 // profiling: one patch-distance evaluation and its in-rectangle taps,
@@ -304,15 +320,17 @@ static __device__ __forceinline__ void count_eval(const Params& P, int x, int y,
 }
 
 // test_offset + isExemplarPixelCulled, :200-205,695-721
-static __device__ float test_offset(const Params& P, int x, int y, const Patch& t, float image_alpha, const PixCtx& pc) {
+// (best: the energy that the result is compared with)
+static __device__ float test_offset(const Params& P, int x, int y, const Patch& t, float image_alpha, const PixCtx& pc,
+                                    float best) {
     float dte = ex_texel_dt(P.ex, f2i(t.x), f2i(t.y), t.layer);
-    if (!((double)dte > (double)P.distTransCull * 1.25)) {
+    if (!(dte > P.exCull)) {
         if (!P.transparencyOk) {
             float ea = ex_sample_out_alpha(P.ex, t.x, t.y, t.layer);
             if (ea < kAlphaThreshold && image_alpha > kAlphaThreshold) return kBigResidual;
         }
         if (P.counters) count_eval(P, x, y, pc.temporalF || pc.temporalB);
-        return energy(P, x, y, t, pc);
+        return energy(P, x, y, t, pc, energy_limit(P, pc, best));
     }
     return kBigResidual;
 }

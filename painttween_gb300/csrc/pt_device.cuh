@@ -407,8 +407,28 @@ __device__ __forceinline__ float4 bl4p(const Bl& b, float4 a, float4 c, float4 d
 
 __device__ __forceinline__ int ex_layer(const ExView& e, int layer) { return clampi(layer, 0, e.ns - 1); }
 
-// exemplar base and output at unnormalised (u, v), one footprint
+// An exemplar colour at unnormalised (u, v) through the texture unit
+// (PT_FILTER_TEXTURE, the level's textures bound).  The level sits in the
+// corner of a larger array with its edge texels repeated once beyond, so the
+// coordinate is clamped to [0, w-1] x [0, h-1] first (NaN to 0): that fetches
+// the texels, with the weights, that clamp addressing on a w x h array would.
+__device__ __forceinline__ float4 ex_tex(cudaTextureObject_t t, const ExView& e, float u, float v, int layer) {
+    u = fminf(fmaxf(u, 0.0f), (float)(e.w - 1));
+    v = fminf(fmaxf(v, 0.0f), (float)(e.h - 1));
+    return tex2DLayered<float4>(t, u + 0.5f, v + 0.5f, ex_layer(e, layer));
+}
+
+// exemplar base and output at unnormalised (u, v), one footprint.  These
+// three take the texture unit where the level's textures are bound: its
+// emulation in integer arithmetic costs some hundred instructions a channel
+// (a propagate pass with temporal terms of both neighbours over 240x180
+// pixels took 4.8 ms by it).
 __device__ __forceinline__ void ex_sample2(const ExView& e, float u, float v, int layer, float4* base, float4* out) {
+    if (e.hw && e.tbase) {
+        *base = ex_tex(e.tbase, e, u, v, layer);
+        *out = ex_tex(e.tout, e, u, v, layer);
+        return;
+    }
     Bl b = bl_setup(u, v, e.w, e.h, e.hw);
     const size_t L = (size_t)ex_layer(e, layer) * e.w * e.h;
     const size_t r0 = L + (size_t)b.y0 * e.w, r1 = L + (size_t)b.y1 * e.w;
@@ -420,6 +440,7 @@ __device__ __forceinline__ void ex_sample2(const ExView& e, float u, float v, in
     *out = bl4(b, o00, o10, o01, o11);
 }
 __device__ __forceinline__ float4 ex_sample_out(const ExView& e, float u, float v, int layer) {
+    if (e.hw && e.tout) return ex_tex(e.tout, e, u, v, layer);
     Bl b = bl_setup(u, v, e.w, e.h, e.hw);
     const size_t L = (size_t)ex_layer(e, layer) * e.w * e.h;
     const size_t r0 = L + (size_t)b.y0 * e.w, r1 = L + (size_t)b.y1 * e.w;
@@ -427,6 +448,7 @@ __device__ __forceinline__ float4 ex_sample_out(const ExView& e, float u, float 
                __ldg(e.out + r1 + b.x1));
 }
 __device__ __forceinline__ float ex_sample_out_alpha(const ExView& e, float u, float v, int layer) {
+    if (e.hw && e.tout) return ex_tex(e.tout, e, u, v, layer).w;
     Bl b = bl_setup(u, v, e.w, e.h, e.hw);
     const float* L = (const float*)(e.out + (size_t)ex_layer(e, layer) * e.w * e.h);
     const float* r0 = L + (size_t)b.y0 * e.w * 4;
@@ -440,16 +462,6 @@ __device__ __forceinline__ float ex_sample_out_alpha(const ExView& e, float u, f
 __device__ __forceinline__ bool exemplar_transparent(const ExView& e) { return __ldg(e.flags) != 0; }
 __device__ __forceinline__ bool exemplar_culls(const ExView& e, float cull) {
     return __int_as_float(__ldg(e.flags + 1)) > cull;
-}
-// the output alpha of the tiled kernels (sample2's fetch with HW)
-template <int HW>
-__device__ __forceinline__ float ex_out_alpha(const ExView& e, float u, float v, int layer) {
-    if (HW) {
-        u = fminf(fmaxf(u, 0.0f), (float)(e.w - 1));
-        v = fminf(fmaxf(v, 0.0f), (float)(e.h - 1));
-        return tex2DLayered<float4>(e.tout, u + 0.5f, v + 0.5f, ex_layer(e, layer)).w;
-    }
-    return ex_sample_out_alpha(e, u, v, layer);
 }
 // the mask of keyframe layer `key` at pixel (x, y): the key's output alpha
 // (PYRAMID_FETCH_LAYER(gExemplarOutput, x, y, keyIndex)); -1 without a key

@@ -82,7 +82,7 @@ __device__ __forceinline__ void sample2(const ExView& E, int li, const float4* L
                                         float4* out, bool fast) {
     const int w = E.w, h = E.h;
     if (HW) {
-        if (!fast) {
+        if (!fast) {  // (ex_tex's clamp)
             u = fminf(fmaxf(u, 0.0f), (float)(w - 1));
             v = fminf(fmaxf(v, 0.0f), (float)(h - 1));
         }
@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
                 if (!((skip >> i) & 1) && !dup) {
                     bool ok = !culls || !(ex_texel_dt(ex_mode<HW>(P.ex), (int)c[i].x, (int)c[i].y, c[i].layer) > P.exCull);
                     if (ok && !opaque && ia > kAlphaThreshold)
-                        ok = !(ex_out_alpha<HW>(P.ex, c[i].x, c[i].y, c[i].layer) < kAlphaThreshold);
+                        ok = !(ex_sample_out_alpha(ex_mode<HW>(P.ex), c[i].x, c[i].y, c[i].layer) < kAlphaThreshold);
                     if (ok) {
                         alive |= 1u << i;
                         if (P.counters) count_eval(P, x, y, px.temporal, false);
@@ -1453,7 +1453,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
                 sv[z] = kind[z] == 1 ? sc.y : 1.f;
                 basis(theta[z], P.scaleWU * su, P.scaleWV * sv[z], &c[z].b0, &c[z].b1);
                 bool ok = !culls || !(ex_texel_dt(ex_mode<HW>(P.ex), (int)c[z].x, (int)c[z].y, 0) > P.exCull);
-                if (ok && !opaque) ok = !(ex_out_alpha<HW>(P.ex, c[z].x, c[z].y, 0) < kAlphaThreshold);
+                if (ok && !opaque) ok = !(ex_sample_out_alpha(ex_mode<HW>(P.ex), c[z].x, c[z].y, 0) < kAlphaThreshold);
                 if (ok) {
                     alive |= 1u << z;
                     if (P.counters) count_eval(P, x, y, px.temporal, false);

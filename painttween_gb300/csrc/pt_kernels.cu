@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(128) k_propagate(const Params P, PatchPlanes w
         else if (c == 1) { s1x = kx; s1y = ky; s1t = kt; s1l = t.layer; }
         else if (c == 2) { s2x = kx; s2y = ky; s2t = kt; s2l = t.layer; }
         if (dup) continue;
-        float r = test_offset(P, x, y, t, ia, pc);
+        float r = test_offset(P, x, y, t, ia, pc, best);
         if (r < best) { ow = t; best = r; }
     }
     store_patch(work, k, ow);
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(128) k_scatter(const Params P, PatchPlanes wor
         lasty = __float_as_uint(ey);
         float ang = screen_to_exemplar_angle(P, x, y, ex, ey, 0);
         Patch t = make_patch(ex, ey, ang, 0.0f, 0, sc.x, sc.y);
-        float r = test_offset(P, x, y, t, ia, pc);
+        float r = test_offset(P, x, y, t, ia, pc, best);
         if (r < best) { ow = t; best = r; }
         dist *= factor;
     }
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128) k_scatter(const Params P, PatchPlanes wor
     avg.x = avg.x / (float)n;
     avg.y = avg.y / (float)n;
     avg.theta = screen_to_exemplar_angle(P, x, y, avg.x, avg.y, 0);
-    float r = test_offset(P, x, y, avg, ia, pc);
+    float r = test_offset(P, x, y, avg, ia, pc, best);
     if (r < best) { ow = avg; best = r; }
     if (best < cached) store_patch(work, k, ow);
     else if (write_all) store_patch(work, k, off);
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(128) k_residual(const Params P, float* out) {
     make_pixctx(P, x, y, &pc);
     Patch t = load_patch(P.off, k);
     if (P.counters) count_eval(P, x, y, pc.temporalF || pc.temporalB);
-    out[k] = energy(P, x, y, t, pc);
+    out[k] = energy(P, x, y, t, pc, __int_as_float(0x7fc00000));
 }
 
 // base and output exemplar texels interleaved into 32-byte records (the

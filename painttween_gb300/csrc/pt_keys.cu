@@ -64,7 +64,7 @@ __device__ void ribbon_candidates(const Params& P, const KeyView& K, int x, int 
                 ey = ey + rb.y;
             }
             Patch q = make_patch(ex, ey, screen_to_exemplar_angle(P, x, y, ex, ey, j), 0.f, j, 1.f, 1.f);
-            float r = test_offset(P, x, y, q, ia, pc);
+            float r = test_offset(P, x, y, q, ia, pc, *best);
             if (r < *best) {
                 *ow = q;
                 *best = r;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kKeyPix) k_propagate_keys(const Params P, Patc
         else if (c == 2) ty = y + jump;
         else ty = y - jump;
         Patch t = propagate_offset(P, tx, ty, x, y);
-        float r = test_offset(P, x, y, t, ia, pc);
+        float r = test_offset(P, x, y, t, ia, pc, best);
         if (r < best) {
             ow = t;
             best = r;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kKeyPix) k_scatter_keys(const Params P, PatchP
         clamp_to_exemplar(&ex, &ey, P.ex.w, P.ex.h);
         const int elayer = ow.layer;
         Patch t = make_patch(ex, ey, screen_to_exemplar_angle(P, x, y, ex, ey, elayer), 0.f, elayer, 1.f, 1.f);
-        float r = test_offset(P, x, y, t, ia, pc);
+        float r = test_offset(P, x, y, t, ia, pc, best);
         if (r < best) {
             ow = t;
             best = r;
