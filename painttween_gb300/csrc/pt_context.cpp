@@ -699,7 +699,7 @@ pt_status do_sync(pt_ctx* c, int level, int flags) {
 }
 
 // ---------------------------------------------------------------------------
-// glibc random(): seeding and jump-ahead (row-parallel random levels)
+// glibc random(): seeding and jump-ahead (random levels)
 // ---------------------------------------------------------------------------
 
 // state of the TYPE_3 generator after srand(seed): the 31 values
@@ -729,20 +729,32 @@ static void matmul31(const uint32_t* a, const uint32_t* b, uint32_t* out) {
             out[i * 31 + j] = s;
         }
 }
-std::vector<uint32_t> step_power(uint64_t n) {
-    // one step: s'[i] = s[i+1] (i < 30), s'[30] = s[0] + s[28]
-    std::vector<uint32_t> M(961, 0), R(961, 0), T(961);
-    for (int i = 0; i < 30; i++) M[i * 31 + i + 1] = 1;
-    M[30 * 31 + 0] = 1;
-    M[30 * 31 + 28] += 1;
-    for (int i = 0; i < 31; i++) R[i * 31 + i] = 1;
-    while (n) {
-        if (n & 1) { matmul31(R.data(), M.data(), T.data()); R.swap(T); }
-        matmul31(M.data(), M.data(), T.data());
-        M.swap(T);
-        n >>= 1;
-    }
-    return R;
+// The powers step^(segment steps * 2^b) of the generator's step, each
+// transposed: the jumps to the segments of a stream (k_glibc_states).
+// Computed once a process; streams of up to 2^31 draws need 23.
+static const int kGlibcPowers = 23;
+const std::vector<uint32_t>& glibc_powers() {
+    static const std::vector<uint32_t> all = [] {
+        // one step: s'[i] = s[i+1] (i < 30), s'[30] = s[0] + s[28]
+        std::vector<uint32_t> M(961, 0), R(961, 0), T(961), out;
+        for (int i = 0; i < 30; i++) M[i * 31 + i + 1] = 1;
+        M[30 * 31 + 0] = 1;
+        M[30 * 31 + 28] += 1;
+        for (int i = 0; i < 31; i++) R[i * 31 + i] = 1;
+        for (int n = pt::glibc_segment_steps(); n; n >>= 1) {
+            if (n & 1) { matmul31(R.data(), M.data(), T.data()); R.swap(T); }
+            matmul31(M.data(), M.data(), T.data());
+            M.swap(T);
+        }
+        for (int b = 0; b < kGlibcPowers; b++) {
+            for (int k = 0; k < 31; k++)
+                for (int i = 0; i < 31; i++) out.push_back(R[i * 31 + k]);
+            matmul31(R.data(), R.data(), T.data());
+            R.swap(T);
+        }
+        return out;
+    }();
+    return all;
 }
 
 // ---------------------------------------------------------------------------
@@ -1038,7 +1050,7 @@ pt_status pt_initialize_exemplars(pt_ctx* c, int w, int h, int ns) {
     }
     c->up_ex.w = w;
     c->up_ex.h = h;
-    c->up_ex.transparent = -1;
+    c->up_ex.transparent = c->up_ex.transparent_all = -1;
     c->up_ex.bo_stale = true;
     c->up_ex.tex_stale = true;
     c->ex = &c->up_ex;
@@ -1097,7 +1109,7 @@ pt_status pt_upload_image_color4(pt_ctx* c, int level, int layer, const float* r
                         h, style);
         float4* plane = (layer == PT_LAYER_EXEMPLAR_OUTPUT) ? c->up_ex.out : c->up_ex.base;
         TRY(h2d(c, plane + n * style, rgba, n * sizeof(float4)));
-        if (layer == PT_LAYER_EXEMPLAR_OUTPUT) c->up_ex.transparent = -1;
+        if (layer == PT_LAYER_EXEMPLAR_OUTPUT) c->up_ex.transparent = c->up_ex.transparent_all = -1;
         c->up_ex.bo_stale = true;
         c->up_ex.tex_stale = true;
         return PT_OK;

@@ -80,7 +80,8 @@ struct ExLevel {  // one exemplar pyramid level, all styles (base and output pla
     int* ids = nullptr;
     int* flags = nullptr;  // ExView::flags, rebuilt with `bo`
     int w = 0, h = 0;
-    int transparent = -1;  // -1 unknown, 0/1
+    // output texels with alpha < 0.99: of style 0, of all styles (-1 unknown)
+    int transparent = -1, transparent_all = -1;
 };
 
 struct FrameLevel {
@@ -182,8 +183,14 @@ struct pt_ctx {
     size_t stage_bytes = 0;
     float* conv_scratch = nullptr;
     size_t conv_scratch_elems = 0;
+    // random levels: the generator's matrix powers, and the scratch of one
+    // level (segment states, draws, trials, starts, how far they sufficed)
+    uint32_t* glibc_mats = nullptr;
     uint32_t* states = nullptr;
-    size_t states_cap = 0;
+    uint32_t* draws = nullptr;
+    uint8_t* trials = nullptr;
+    int* starts = nullptr;
+    size_t states_cap = 0, draws_cap = 0, starts_cap = 0;
     int* flag = nullptr;
 
     // resident working set
@@ -241,7 +248,6 @@ struct pt_ctx {
     unsigned long long* counters = nullptr;  // [kernel][evals, taps, temporal taps]
     std::vector<cudaEvent_t> ev_pool;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_pairs[PT_KERNEL_COUNT];
-    std::map<int, std::vector<uint32_t>> jump_cache;  // M^(4w)
 };
 
 
@@ -284,18 +290,19 @@ PT_HIDDEN void free_frames(pt_ctx* c);
 PT_HIDDEN void free_store(pt_ctx* c);
 PT_HIDDEN void free_textures(pt_ctx* c, ExLevel* L);
 PT_HIDDEN void glibc_state(uint32_t seed, uint32_t out[31]);
+PT_HIDDEN const std::vector<uint32_t>& glibc_powers();
 PT_HIDDEN pt_status h2d(pt_ctx* c, void* dst, const void* src, size_t bytes);
 PT_HIDDEN cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,
                                    float* out, bool* done);
 PT_HIDDEN Params make_params(pt_ctx* c, int level);
 PT_HIDDEN cudaEvent_t pool_event(pt_ctx* c);
-PT_HIDDEN pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<float> orient);
+PT_HIDDEN pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<float> orient, int nk = 0,
+                                 int first_key = 0);
 PT_HIDDEN pt_status rect_copy(pt_ctx* c, void* dst, size_t dpitch, const void* src, size_t spitch, size_t row_bytes,
                               int rows, cudaMemcpyKind kind);
 PT_HIDDEN pt_status refresh_interleaved(pt_ctx* c, ExLevel* L);
 PT_HIDDEN pt_status reset_image_slots(pt_ctx* c);
 PT_HIDDEN pt_status reset_working(pt_ctx* c);
-PT_HIDDEN std::vector<uint32_t> step_power(uint64_t n);
 PT_HIDDEN bool tiled_usable(pt_ctx* c);
 PT_HIDDEN pt_status writable_work(pt_ctx* c, int level, PatchPlanes* out, bool* was_aliased = nullptr);
 

@@ -237,28 +237,10 @@ static float key_advect_weight(const pt_ctx* c, int frame, bool forwards) {
 
 // SynthesisFrame::createRandomPyramid with setupWithKeys
 // (synthesisFrame.cpp:66-150): the glibc stream of srand(frame*level), each
-// pixel drawing its key layer first; one GPU thread walks the stream.
+// pixel drawing its key layer first.
 static pt_status random_level_keyed(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<float> orient) {
     TRY(check_ready(c, level));
-    const int lw = c->W >> level, lh = c->H >> level;
-    const int mx = (c->SW >> level) - 1, my = (c->SH >> level) - 1;
-    if (mx < 1 || my < 1) return fail(c, PT_ERR_INVALID, "style too small for level %d", level);
-    if (!c->rnd) TRY(dalloc_t(c, &c->rnd, (size_t)c->W * c->H));
-    if (c->states_cap < 31) {
-        dfree_t(c, c->states);
-        TRY(dalloc_t(c, &c->states, (size_t)31));
-        c->states_cap = 31;
-    }
-    uint32_t s0[31];
-    glibc_state((uint32_t)(frame * level), s0);
-    CU(cudaMemcpyAsync(c->states, s0, sizeof(s0), cudaMemcpyHostToDevice, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
-    ExView ex{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS, 0, 0, 0, c->ex->flags};
-    const int nk = (int)c->key_sub.size(), first_key = key_full_index(c, c->key_sub.front());
-    LN(pt::launch_random_level_keys(lw, lh, mx, my, c->params.transparencyOk, c->params.orientationEnabled, rgba,
-                                    orient, ex, c->rnd, c->states, nk, first_key, c->stream));
-    c->img.rnd = Arr<float4>{c->rnd, lw, lh};
-    return PT_OK;
+    return random_level(c, level, frame, rgba, orient, (int)c->key_sub.size(), key_full_index(c, c->key_sub.front()));
 }
 
 static pt_status synthesize_consecutive(pt_ctx* c, const pt_params& user, int frame, int level, int pass,

@@ -105,7 +105,7 @@ pt_status pt_set_style(pt_ctx* c, int style, int w, int h, const float* base, co
         CU(cudaMemcpyAsync(L.orient + n * style, por[l], n * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
         CU(cudaMemcpyAsync(L.dt + n * style, pd[l], n * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
         CU(cudaMemcpyAsync(L.ids + n * style, pi[l], n * sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
-        L.transparent = -1;
+        L.transparent = L.transparent_all = -1;
         L.bo_stale = true;
         L.tex_stale = true;
     }

@@ -71,13 +71,31 @@ cudaError_t launch_gather_level(const Params& P, const float* src, int ch, float
 cudaError_t launch_down_avg(const float* src, int w, int h, int ch, int vel, float* dst, cudaStream_t s);
 cudaError_t launch_down_vote(const int* src, int w, int h, int* dst, cudaStream_t s);
 cudaError_t launch_tensor_angle(const float* t3, int n, float* out, cudaStream_t s);
-cudaError_t launch_random_level_keys(int w, int h, int mx, int my, int transparencyOk, int orientationEnabled,
-                                     Arr<float4> img, Arr<float> iorient, ExView ex, float4* out,
-                                     const uint32_t* state31, int nk, int first_key, cudaStream_t s);
-cudaError_t launch_random_level(int mode, int w, int h, int mx, int my, int transparencyOk, int orientationEnabled,
-                                Arr<float4> img, Arr<float> iorient, ExView ex, float4* out,
-                                const uint32_t* states, uint32_t seed, cudaStream_t s);
-cudaError_t launch_any_transparent(const float4* out, size_t n, int* flag, cudaStream_t s);
+// the random level (pt_random.cu): L.nk > 0 with keyframe interpolation
+struct RandomLevel {
+    int w, h, mx, my;
+    int transparencyOk, orientationEnabled;
+    Arr<float4> img;
+    Arr<float> iorient;
+    ExView ex;
+    float4* out;
+    int nk, first_key;
+};
+using ptk::GlibcState;
+// segments of a stream of `draws` draws, and the generator's steps of one
+size_t glibc_segments(size_t draws);
+int glibc_segment_steps();
+// pixels that cannot retry: four draws each.  mats: the transposed powers
+// step^(segment steps * 2^b); states: 31 words a segment
+cudaError_t launch_random_level(const RandomLevel& L, const GlibcState& s0, const uint32_t* mats, uint32_t* states,
+                                cudaStream_t s);
+// with retries or keys, from a stream of n draws (n > 1000; what it does not
+// suffice for is drawn serially); trials: n bytes, starts: w * h, done: 2
+cudaError_t launch_random_level_retry(const RandomLevel& L, const GlibcState& s0, const uint32_t* mats,
+                                      uint32_t* states, uint32_t* draws, size_t n, uint8_t* trials, int* starts,
+                                      int* done, cudaStream_t s);
+cudaError_t launch_random_level_counter(const RandomLevel& L, uint32_t seed, cudaStream_t s);
+cudaError_t launch_count_transparent(const float4* out, size_t n, int* count, cudaStream_t s);
 cudaError_t launch_interleave_texels(const float4* base, const float4* out, const float* dt, float4* bo, int* flags,
                                      size_t n, cudaStream_t s);
 

@@ -468,165 +468,6 @@ __global__ void k_tensor_angle(const float* t3, int n, float* out) {
     out[i] = ((double)angle >= 1.57079632679489661923) ? (float)((double)angle - 3.14159265358979323846) : angle;
 }
 
-// ---------------------------------------------------------------------------
-// random-offset level (SynthesisFrame::createRandomPyramid,
-// synthesisFrame.cpp:66-150)
-// ---------------------------------------------------------------------------
-
-struct RandParams {
-    int w, h, mx, my;
-    int transparencyOk, orientationEnabled;
-    Arr<float4> img;     // level-size input colour (alpha)
-    Arr<float> iorient;  // level-size input orientation
-    ExView ex;           // exemplar level (style 0)
-    float4* out;
-};
-
-__device__ __forceinline__ float4 random_texel(const RandParams& R, int x, int y, uint32_t d0, uint32_t d1,
-                                                uint32_t d2, uint32_t d3) {
-    int ox = (int)((d0 >> 1) % (uint32_t)R.mx);
-    int oy = (int)((d1 >> 1) % (uint32_t)R.my);
-    float orient = R.orientationEnabled
-                       ? __ldg(R.iorient.p + (size_t)y * R.iorient.w + x) - __ldg(R.ex.orient + (size_t)oy * R.ex.w + ox)
-                       : 0.f;
-    float rx = (float)(d2 >> 1) / (float)2147483647;
-    float ry = (float)(d3 >> 1) / (float)2147483647;
-    return f4((float)ox + rx, (float)oy + ry, orient, 0.0f);
-}
-
-// One thread per row: the glibc additive-feedback state at the row start is
-// precomputed on the host (jump-ahead by a 31x31 matrix power over Z/2^32);
-// each thread then steps the recurrence r[i] = r[i-31] + r[i-3] in a
-// shared-memory ring.  Valid when no pixel retries (no exemplar texel with
-// alpha < 0.99, or transparency allowed).
-__global__ void k_glibc_rows(const RandParams R, const uint32_t* row_states) {
-    extern __shared__ uint32_t ring_all[];
-    int y = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t* ring = ring_all + threadIdx.x;  // stride blockDim.x: conflict-free
-    const int S = blockDim.x;
-    if (y >= R.h) return;
-    for (int i = 0; i < 31; i++) ring[i * S] = row_states[(size_t)y * 31 + i];
-    int head = 0;
-    int h28 = 28;
-    for (int x = 0; x < R.w; x++) {
-        uint32_t d[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            uint32_t v = ring[head * S] + ring[h28 * S];
-            ring[head * S] = v;
-            head = (head == 30) ? 0 : head + 1;
-            h28 = (h28 == 30) ? 0 : h28 + 1;
-            d[q] = v;
-        }
-        R.out[(size_t)y * R.w + x] = random_texel(R, x, y, d[0], d[1], d[2], d[3]);
-    }
-}
-
-// Exact serial version (one thread) with the reference's retry loop for
-// opaque pixels that drew a transparent exemplar texel.
-__global__ void k_glibc_serial(const RandParams R, const uint32_t* state31) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    uint32_t ring[31];
-    for (int i = 0; i < 31; i++) ring[i] = state31[i];
-    int head = 0;
-    auto next = [&]() -> uint32_t {
-        int h28 = head + 28;
-        if (h28 >= 31) h28 -= 31;
-        uint32_t v = ring[head] + ring[h28];
-        ring[head] = v;
-        head = (head == 30) ? 0 : head + 1;
-        return v;
-    };
-    for (int y = 0; y < R.h; y++)
-        for (int x = 0; x < R.w; x++) {
-            float ia = __ldg(R.img.p + (size_t)y * R.img.w + x).w;
-            uint32_t d0, d1;
-            int trial = 0;
-            bool again;
-            do {
-                d0 = next();
-                d1 = next();
-                trial++;
-                int ox = (int)((d0 >> 1) % (uint32_t)R.mx), oy = (int)((d1 >> 1) % (uint32_t)R.my);
-                float ea = __ldg(R.ex.out + (size_t)oy * R.ex.w + ox).w;
-                again = !R.transparencyOk && ia > kAlphaThreshold && ea < kAlphaThreshold && trial < 50;
-            } while (again);
-            uint32_t d2 = next(), d3 = next();
-            R.out[(size_t)y * R.w + x] = random_texel(R, x, y, d0, d1, d2, d3);
-        }
-}
-
-// Keyframe interpolation (createRandomPyramid with setupWithKeys,
-// synthesisFrame.cpp:94-139): each pixel first draws its key layer
-// (rand() % nk + first_key), then the offset in that layer with the retry
-// rule, then the two fractions; one thread, exact glibc order.
-__global__ void k_glibc_serial_keys(const RandParams R, const uint32_t* state31, int nk, int first_key) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    uint32_t ring[31];
-    for (int i = 0; i < 31; i++) ring[i] = state31[i];
-    int head = 0;
-    auto next = [&]() -> uint32_t {
-        int h28 = head + 28;
-        if (h28 >= 31) h28 -= 31;
-        uint32_t v = ring[head] + ring[h28];
-        ring[head] = v;
-        head = (head == 30) ? 0 : head + 1;
-        return v;
-    };
-    const size_t lsz = (size_t)R.ex.w * R.ex.h;
-    for (int y = 0; y < R.h; y++)
-        for (int x = 0; x < R.w; x++) {
-            const int style = (int)((next() >> 1) % (uint32_t)nk) + first_key;
-            const int sl = clampi(style, 0, R.ex.ns - 1);  // a layer of the uploaded exemplar
-            float ia = __ldg(R.img.p + (size_t)y * R.img.w + x).w;
-            int ox, oy, trial = 0;
-            bool again;
-            do {
-                ox = (int)((next() >> 1) % (uint32_t)R.mx);
-                oy = (int)((next() >> 1) % (uint32_t)R.my);
-                trial++;
-                float ea = __ldg(R.ex.out + sl * lsz + (size_t)oy * R.ex.w + ox).w;
-                again = !R.transparencyOk && ia > kAlphaThreshold && ea < kAlphaThreshold && trial < 50;
-            } while (again);
-            float orient = R.orientationEnabled ? __ldg(R.iorient.p + (size_t)y * R.iorient.w + x) -
-                                                      __ldg(R.ex.orient + sl * lsz + (size_t)oy * R.ex.w + ox)
-                                                : 0.f;
-            float rx = (float)(next() >> 1) / (float)2147483647;
-            float ry = (float)(next() >> 1) / (float)2147483647;
-            R.out[(size_t)y * R.w + x] = f4((float)ox + rx, (float)oy + ry, orient, (float)style);
-        }
-}
-
-// counter-based random level: four hashed draws per pixel and trial
-__global__ void k_counter_random(const RandParams R, uint32_t seed) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= R.w || y >= R.h) return;
-    float ia = __ldg(R.img.p + (size_t)y * R.img.w + x).w;
-    uint32_t base = hash32(seed ^ hash32(x * 0x85EBCA6BU ^ hash32(y * 0xC2B2AE35U)));
-    uint32_t d0, d1;
-    int trial = 0;
-    bool again;
-    do {
-        d0 = hash32(base + 4u * trial);
-        d1 = hash32(base + 4u * trial + 1u);
-        trial++;
-        int ox = (int)((d0 >> 1) % (uint32_t)R.mx), oy = (int)((d1 >> 1) % (uint32_t)R.my);
-        float ea = __ldg(R.ex.out + (size_t)oy * R.ex.w + ox).w;
-        again = !R.transparencyOk && ia > kAlphaThreshold && ea < kAlphaThreshold && trial < 50;
-    } while (again);
-    uint32_t d2 = hash32(base + 0x40000000u), d3 = hash32(base + 0x40000001u);
-    R.out[(size_t)y * R.w + x] = random_texel(R, x, y, d0, d1, d2, d3);
-}
-
-// any exemplar output texel with alpha < 0.99 (decides whether the random
-// level can be drawn row-parallel)
-__global__ void k_any_transparent(const float4* out, size_t n, int* flag) {
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    for (; i < n; i += (size_t)gridDim.x * blockDim.x)
-        if (__ldg(out + i).w < kAlphaThreshold) { atomicOr(flag, 1); return; }
-}
-
 }  // namespace ptk
 
 // ---------------------------------------------------------------------------
@@ -725,34 +566,6 @@ cudaError_t launch_tensor_angle(const float* t3, int n, float* out, cudaStream_t
     k_tensor_angle<<<(n + 255) / 256, 256, 0, s>>>(t3, n, out);
     LAUNCH_CHECK();
 }
-cudaError_t launch_random_level_keys(int w, int h, int mx, int my, int transparencyOk, int orientationEnabled,
-                                     Arr<float4> img, Arr<float> iorient, ExView ex, float4* out,
-                                     const uint32_t* state31, int nk, int first_key, cudaStream_t s) {
-    RandParams R;
-    R.w = w; R.h = h; R.mx = mx; R.my = my;
-    R.transparencyOk = transparencyOk; R.orientationEnabled = orientationEnabled;
-    R.img = img; R.iorient = iorient; R.ex = ex; R.out = out;
-    k_glibc_serial_keys<<<1, 1, 0, s>>>(R, state31, nk, first_key);
-    LAUNCH_CHECK();
-}
-cudaError_t launch_random_level(int mode, int w, int h, int mx, int my, int transparencyOk, int orientationEnabled,
-                                Arr<float4> img, Arr<float> iorient, ExView ex, float4* out,
-                                const uint32_t* states, uint32_t seed, cudaStream_t s) {
-    RandParams R;
-    R.w = w; R.h = h; R.mx = mx; R.my = my;
-    R.transparencyOk = transparencyOk; R.orientationEnabled = orientationEnabled;
-    R.img = img; R.iorient = iorient; R.ex = ex; R.out = out;
-    if (mode == 0) {  // row-parallel glibc
-        const int tb = 64;
-        k_glibc_rows<<<(h + tb - 1) / tb, tb, tb * 31 * sizeof(uint32_t), s>>>(R, states);
-    } else if (mode == 1) {  // serial glibc
-        k_glibc_serial<<<1, 1, 0, s>>>(R, states);
-    } else {
-        dim3 b(32, 4);
-        k_counter_random<<<grid2(w, h, b), b, 0, s>>>(R, seed);
-    }
-    LAUNCH_CHECK();
-}
 cudaError_t launch_interleave_texels(const float4* base, const float4* out, const float* dt, float4* bo, int* flags,
                                      size_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
@@ -763,9 +576,4 @@ cudaError_t launch_interleave_texels(const float4* base, const float4* out, cons
     k_interleave_texels<<<blocks, threads, 0, s>>>(base, out, dt, bo, flags, n);
     LAUNCH_CHECK();
 }
-cudaError_t launch_any_transparent(const float4* out, size_t n, int* flag, cudaStream_t s) {
-    k_any_transparent<<<152 * 4, 256, 0, s>>>(out, n, flag);
-    LAUNCH_CHECK();
-}
-
 }  // namespace pt

@@ -6,12 +6,26 @@
 
 static pt_status ensure_transparency_known(pt_ctx* c) {
     if (c->ex->transparent >= 0) return PT_OK;
-    CU(cudaMemsetAsync(c->flag, 0, sizeof(int), c->stream));
-    LN(pt::launch_any_transparent(c->ex->out, (size_t)c->ex->w * c->ex->h, c->flag, c->stream));
-    int f = 0;
-    CU(cudaMemcpyAsync(&f, c->flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    const size_t n = (size_t)c->ex->w * c->ex->h;
+    CU(cudaMemsetAsync(c->flag, 0, 2 * sizeof(int), c->stream));
+    LN(pt::launch_count_transparent(c->ex->out, n, c->flag, c->stream));
+    if (c->NS > 1) LN(pt::launch_count_transparent(c->ex->out + n, n * (c->NS - 1), c->flag + 1, c->stream));
+    int f[2] = {0, 0};
+    CU(cudaMemcpyAsync(f, c->flag, sizeof f, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
-    c->ex->transparent = f ? 1 : 0;
+    c->ex->transparent = f[0];
+    c->ex->transparent_all = f[0] + f[1];
+    return PT_OK;
+}
+
+// scratch of at least n elements
+template <class T>
+static pt_status ensure_scratch(pt_ctx* c, T** p, size_t* cap, size_t n) {
+    if (*cap >= n) return PT_OK;
+    dfree_t(c, *p);
+    *cap = 0;
+    TRY(dalloc_t(c, p, n));
+    *cap = n;
     return PT_OK;
 }
 
@@ -24,52 +38,64 @@ pt_status pt_create_random_level(pt_ctx* c, int level, int frame) {
     return random_level(c, level, frame, c->img.base[c->img.cur], c->img.orient);
 }
 
-pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<float> orient) {
+// (nk > 0: with setupWithKeys, each pixel drawing one of nk key layers first)
+pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<float> orient, int nk, int first_key) {
     int lw = c->W >> level, lh = c->H >> level;
     int mx = (c->SW >> level) - 1, my = (c->SH >> level) - 1;
     if (mx < 1 || my < 1) return fail(c, PT_ERR_INVALID, "style too small for level %d", level);
     if (!c->rnd) TRY(dalloc_t(c, &c->rnd, (size_t)c->W * c->H));
-    ExView ex{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS, 0, 0, 0, c->ex->flags};
-    int mode;
-    uint32_t seed = (uint32_t)(frame * level);
-    if (c->params.rngMode == PT_RNG_COUNTER) {
-        mode = 2;
-        seed = c->params.rngSeed ^ (0x9E3779B9u * (uint32_t)(frame + 1)) ^ (0x85EBCA6Bu * (uint32_t)(level + 1));
-    } else {
-        TRY(ensure_transparency_known(c));
-        mode = (c->params.transparencyOk || !c->ex->transparent) ? 0 : 1;
-        uint32_t s0[31];
-        glibc_state(seed, s0);
-        size_t need = mode == 0 ? (size_t)lh * 31 : 31;
-        if (need > c->states_cap) {
-            dfree_t(c, c->states);
-            TRY(dalloc_t(c, &c->states, need));
-            c->states_cap = need;
-        }
-        std::vector<uint32_t> host(need);
-        if (mode == 0) {
-            auto it = c->jump_cache.find(lw);
-            if (it == c->jump_cache.end()) it = c->jump_cache.emplace(lw, step_power(4ull * (uint64_t)lw)).first;
-            const std::vector<uint32_t>& A = it->second;
-            std::vector<uint32_t> s(s0, s0 + 31), t(31);
-            for (int y = 0; y < lh; y++) {
-                memcpy(&host[(size_t)y * 31], s.data(), 31 * sizeof(uint32_t));
-                for (int i = 0; i < 31; i++) {
-                    uint32_t acc = 0;
-                    for (int k = 0; k < 31; k++) acc += A[i * 31 + k] * s[k];
-                    t[i] = acc;
-                }
-                s.swap(t);
-            }
-        } else {
-            memcpy(host.data(), s0, sizeof(s0));
-        }
-        CU(cudaMemcpyAsync(c->states, host.data(), need * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
-        CU(cudaStreamSynchronize(c->stream));  // host vector goes out of scope
-    }
-    LN(pt::launch_random_level(mode, lw, lh, mx, my, c->params.transparencyOk, c->params.orientationEnabled,
-                               rgba, orient, ex, c->rnd, c->states, seed, c->stream));
+    const size_t px = (size_t)lw * lh;
+    pt::RandomLevel L;
+    L.w = lw; L.h = lh; L.mx = mx; L.my = my;
+    L.transparencyOk = c->params.transparencyOk;
+    L.orientationEnabled = c->params.orientationEnabled;
+    L.img = rgba;
+    L.iorient = orient;
+    L.ex = ExView{c->ex->base, c->ex->out, c->ex->bo, c->ex->orient, c->ex->dt, c->ex->ids, c->ex->w, c->ex->h, c->NS,
+                  0, 0, 0, c->ex->flags};
+    L.out = c->rnd;
+    L.nk = nk;
+    L.first_key = first_key;
     c->img.rnd = Arr<float4>{c->rnd, lw, lh};
+    if (nk == 0 && c->params.rngMode == PT_RNG_COUNTER) {
+        const uint32_t seed =
+            c->params.rngSeed ^ (0x9E3779B9u * (uint32_t)(frame + 1)) ^ (0x85EBCA6Bu * (uint32_t)(level + 1));
+        LN(pt::launch_random_level_counter(L, seed, c->stream));
+        return PT_OK;
+    }
+    TRY(ensure_transparency_known(c));
+    pt::GlibcState s0;
+    glibc_state((uint32_t)(frame * level), s0.s);
+    if (!c->glibc_mats) {
+        const std::vector<uint32_t>& m = glibc_powers();
+        TRY(dalloc_t(c, &c->glibc_mats, m.size()));
+        TRY(h2d(c, c->glibc_mats, m.data(), m.size() * sizeof(uint32_t)));
+    }
+    if (nk == 0 && (c->params.transparencyOk || !c->ex->transparent)) {
+        TRY(ensure_scratch(c, &c->states, &c->states_cap, 31 * pt::glibc_segments(4 * px)));
+        LN(pt::launch_random_level(L, s0, c->glibc_mats, c->states, c->stream));
+        c->launches += 2;
+        return PT_OK;
+    }
+    // the draws that the pixels take on average, and eight deviations more
+    const double texels = (double)c->ex->w * c->ex->h * (nk ? c->NS : 1);
+    const double f = std::min((double)(nk ? c->ex->transparent_all : c->ex->transparent) / texels, 0.98);
+    const double mean = (nk ? 1.0 : 0.0) + 2.0 + 2.0 / (1.0 - f), dev = 2.0 * std::sqrt(f) / (1.0 - f);
+    const double want = std::min(1.05 * mean, 64.0) * (double)px + 8.0 * dev * std::sqrt((double)px) + 4096.0;
+    const size_t n = (size_t)std::min(want, (double)(1u << 30));
+    if (n > c->draws_cap) {
+        dfree_t(c, c->draws);
+        dfree_t(c, c->trials);
+        c->draws_cap = 0;
+        TRY(dalloc_t(c, &c->draws, n));
+        TRY(dalloc_t(c, &c->trials, n));
+        c->draws_cap = n;
+    }
+    TRY(ensure_scratch(c, &c->states, &c->states_cap, 31 * pt::glibc_segments(n)));
+    TRY(ensure_scratch(c, &c->starts, &c->starts_cap, px));
+    LN(pt::launch_random_level_retry(L, s0, c->glibc_mats, c->states, c->draws, n, c->trials, c->starts, c->flag + 2,
+                                     c->stream));
+    c->launches += 5;
     return PT_OK;
 }
 

@@ -160,6 +160,11 @@ struct Params {
     IncView inc;
 };
 
+// the 31 words of glibc's TYPE_3 generator
+struct GlibcState {
+    uint32_t s[31];
+};
+
 struct ConvKernel {
     int r;
     float w[2 * kMaxRadius + 1];
