@@ -750,11 +750,12 @@ constexpr int kGroups = 32 / kGroup;
 // reference's (column-major) order.
 struct Tap {
     float fi, fj, w;
-    int code;  // (i + R) | (j + R) << 4 | t << 8
+    int code;  // (i + R) | (j + R) << 4 | t << 8 | place in a tile (j * TW + i) << 16
 };
 template <int R>
 struct TapList {
     Tap tap[(2 * R + 1) * (2 * R + 1)];
+    alignas(16) float w[(2 * R + 1) * (2 * R + 1)];  // the weights in the reference's order
 };
 template <int R>
 __device__ __forceinline__ void load_tap_list(const Params& P, TapList<R>& L, int tid) {
@@ -765,8 +766,9 @@ __device__ __forceinline__ void load_tap_list(const Params& P, TapList<R>& L, in
         a.fi = (float)(i - R);
         a.fj = (float)(j - R);
         a.w = P.gauss[i] * P.gauss[j];
-        a.code = i | (j << 4) | (t << 8);
+        a.code = i | (j << 4) | (t << 8) | (((j - R) * (kTileW + 2 * R) + i - R) * 65536);
         L.tap[tid] = a;
+        L.w[t] = a.w;
     }
 }
 
@@ -812,10 +814,18 @@ __device__ __forceinline__ ExSample prev_fetch(const Params& P, const LanePix& q
     return s;
 }
 
+// whether a tap of pixel q lies inside the level rectangle
+template <int R>
+__device__ __forceinline__ bool tap_inside(const LanePix& q, const Tap& tp) {
+    const int i = (tp.code & 15) - R, j = ((tp.code >> 4) & 15) - R;
+    return (i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax);
+}
+
 // the pixel side of one tap
 struct PixSample {
-    float4 base, canvas, pbase, pout;
-    bool prev;  // the temporal terms apply at this tap
+    float4 base, canvas, pout;
+    float4 dbase, dcanvas;  // temporal: base - pbase, canvas - pout
+    bool prev;              // the temporal terms apply at this tap
 };
 template <int R, int TM, int H>
 __device__ __forceinline__ PixSample pix_sample(const TileSmem<R, TM, H>& T, const LanePix& q, int s) {
@@ -824,9 +834,10 @@ __device__ __forceinline__ PixSample pix_sample(const TileSmem<R, TM, H>& T, con
     p.canvas = T.canvas[s];
     p.prev = false;
     if (TM && q.temporal) {
-        p.pbase = T.pbase[s];
         p.pout = T.pout[s];
         p.prev = T.pvalid[s] != 0;
+        p.dbase = sub4p(p.base, T.pbase[s]);
+        p.dcanvas = sub4p(p.canvas, p.pout);
     }
     return p;
 }
@@ -839,8 +850,8 @@ __device__ __forceinline__ float tap_terms(const Params& P, const PixSample& p, 
                                            bool center) {
     float res = ssd_ap(p.base, c.tb, P.alphaWeight) * P.inputAnalogyWeight;
     if (TM) {
-        float r = ssdp(sub4p(p.base, p.pbase), sub4p(c.tb, v.tb)) * P.tdIn;
-        r = fmaf(ssdp(sub4p(p.canvas, p.pout), sub4p(c.to, v.to)), P.tdOut, r);
+        float r = ssdp(p.dbase, sub4p(c.tb, v.tb)) * P.tdIn;
+        r = fmaf(ssdp(p.dcanvas, sub4p(c.to, v.to)), P.tdOut, r);
         r = fmaf(ssdp(p.pout, c.to), P.tc, r);
         res = p.prev ? res + r : res;
     }
@@ -909,15 +920,14 @@ __device__ __forceinline__ unsigned front_taps(const Params& P, const TileSmem<R
                                                const LanePix& q, const Threshold& th, const CandPos (&c)[NC],
                                                const float (&sv)[NC], unsigned alive, float (&sum)[NC],
                                                float (&v0)[NC]) {
-    constexpr int TW = TileSmem<R, TM>::TW;
-    bool in = true;  // every footprint of the lane inside the exemplar
+    bool fast[NC];  // all of the warp's footprints of this candidate inside the exemplar
 #pragma unroll
     for (int k = 0; k < NC; k++) {
-        in = in && (!((alive >> k) & 1) || footprint_inside<R>(c[k].x, c[k].y, c[k].b0, c[k].b1, P.ex.w, P.ex.h));
+        fast[k] = __all_sync(kFull, !((alive >> k) & 1) || footprint_inside<R>(c[k].x, c[k].y, c[k].b0, c[k].b1,
+                                                                              P.ex.w, P.ex.h));
         sum[k] = 0.0f;
         v0[k] = 0.0f;
     }
-    const bool fast = __all_sync(kFull, in);
     const bool fastp = TM ? __all_sync(kFull, !alive || !q.temporal || q.prev_fast) : true;
     const bool bounded = th.bound == th.bound;
     unsigned taps = 0;
@@ -926,16 +936,14 @@ __device__ __forceinline__ unsigned front_taps(const Params& P, const TileSmem<R
         const unsigned on = (t == 0 || bounded) ? alive : 0u;
         if (!__any_sync(kFull, on)) break;
         const Tap tp = L.tap[t];
-        const int i = (tp.code & 15) - R, j = ((tp.code >> 4) & 15) - R;
-        const bool valid = (i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax);
-        if (!on || !valid) continue;
-        const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + j * TW + i);
+        if (!on || !tap_inside<R>(q, tp)) continue;
+        const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + (tp.code >> 16));
         ExSample s[NC], v;
         float tx[NC], ty[NC];
         if (TM && p.prev) v = prev_fetch<HW>(P, q, tp.fi, tp.fj, fastp);
 #pragma unroll
         for (int k = 0; k < NC; k++)
-            if ((on >> k) & 1) s[k] = cand_fetch<HW>(P, c[k], tp.fi, tp.fj, fast, &tx[k], &ty[k]);
+            if ((on >> k) & 1) s[k] = cand_fetch<HW>(P, c[k], tp.fi, tp.fj, fast[k], &tx[k], &ty[k]);
 #pragma unroll
         for (int k = 0; k < NC; k++)
             if ((on >> k) & 1) {
@@ -982,18 +990,19 @@ __device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& 
 
 // Evaluates the first n candidates of the warp's queue, a group of kGroup
 // lanes each; energies of those that no bound rejects into energy[pid * CH +
-// slot].  thr: the energy to beat of each pixel of the tile; V: (2R+1)^2
-// values of each of the warp's groups.
+// slot].  thr: the energy to beat of each pixel of the tile; V: the tap values
+// of each of the warp's groups.
 template <int R, int TM, int HW, int H, int CAP, int CH>
 __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM, H>& T,
                                            const PixShared<kTileW * H>& S, const TapList<R>& L,
                                            const WarpQueue<CAP>& Q, int n, const float* thr,
                                            float* V, float* energy) {
-    constexpr int TW = TileSmem<R, TM>::TW, n1 = 2 * R + 1, K = n1 * n1;
+    constexpr int K = (2 * R + 1) * (2 * R + 1);
+    constexpr int kStride = (K + 3) / 4 * 4;
     constexpr int kRest = (K - kFront + kGroup - 1) / kGroup;        // steps past the front
     constexpr int kLast = kRest + (kFront - 1 + kGroup - 1) / kGroup;  // and of the front's other taps
     const int lane = (int)lane_id(), g = lane / kGroup, l = lane % kGroup;
-    float* val = V + g * K;
+    float* val = V + g * kStride;
     bool act = false, cfast = false;
     int next = 0, step = 0, id = 0;
     float sum = 0.0f;
@@ -1034,15 +1043,16 @@ __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM
         const int pos = step < kRest ? kFront + step * kGroup + l : 1 + (step - kRest) * kGroup + l;
         if (act && pos < (step < kRest ? K : kFront)) {
             const Tap tp = L.tap[pos];
-            const int i = (tp.code & 15) - R, j = ((tp.code >> 4) & 15) - R;
-            if ((i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax)) {
-                const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + j * TW + i);
+            const int t = (tp.code >> 8) & 255;
+            val[t] = 0.0f;  // (a tap outside the level rectangle adds nothing)
+            if (tap_inside<R>(q, tp)) {
+                const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + (tp.code >> 16));
                 ExSample v;
                 float tx, ty;
                 if (TM && p.prev) v = prev_fetch<HW>(P, q, tp.fi, tp.fj, fastp);
                 const ExSample s = cand_fetch<HW>(P, c, tp.fi, tp.fj, fast, &tx, &ty);
                 const float r = tap_terms<TM>(P, p, s, v, false);
-                val[tp.code >> 8] = r;
+                val[t] = r;
                 if (step < kRest) part = __fmul_rd(r, tp.w);
             }
             if (P.counters) count_taps(P, 1u, q.temporal);
@@ -1058,18 +1068,17 @@ __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM
             if (last) {
                 // the exact sum, in the reference's order
                 float e = q.sum0;
-#pragma unroll 1
-                for (int i = -R; i <= R; i++) {
-                    const float gi = P.gauss[i + R];
-                    const bool cvalid = (i >= q.imin) && (i <= q.imax);
 #pragma unroll
-                    for (int j = -R; j <= R; j++) {
-                        const bool valid = cvalid && (j >= q.jmin) && (j <= q.jmax);
-                        const float w = gi * P.gauss[j + R];
-                        const float v = val[(i + R) * n1 + j + R];
-                        e = valid ? fmaf(v, w, e) : e;
-                    }
+                for (int t = 0; t + 3 < K; t += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(val + t);
+                    const float4 w = *reinterpret_cast<const float4*>(L.w + t);
+                    e = fmaf(v.x, w.x, e);
+                    e = fmaf(v.y, w.y, e);
+                    e = fmaf(v.z, w.z, e);
+                    e = fmaf(v.w, w.w, e);
                 }
+                static_assert(K % 4 == 1, "one tap past the fours");
+                e = fmaf(val[K - 1], L.w[K - 1], e);
                 if (l == 0)
                     energy[id] = (q.sumW < kEpsilon) ? kBigResidual : (e >= th.thr2) ? INFINITY : e / q.sumW;
                 act = false;
@@ -1086,7 +1095,7 @@ struct EvalSmem {
     PixShared<NP> S;
     WarpQueue<CAP> Q[NW];
     TapList<R> L;
-    float V[NW][kGroups * (2 * R + 1) * (2 * R + 1)];
+    alignas(16) float V[NW][kGroups * (((2 * R + 1) * (2 * R + 1) + 3) / 4 * 4)];
     float thr[NP];                    // the energy each pixel has to beat
     alignas(16) float energy[NP * CH];  // per candidate (CH a pixel): its energy, +inf where it lost or is none
 };
