@@ -224,7 +224,12 @@ Params make_params(pt_ctx* c, int level) {
     P.adv[0] = c->adv[0];
     P.adv[1] = c->adv[1];
     P.inc = ptk::IncView{c->chg, c->stamp_last, c->stamp_win, c->inc_on, c->inc_pi, c->inc_prev,
-                         c->tap_cache, c->inc_fill};
+                         c->tap_cache, c->inc_fill, nullptr, nullptr, nullptr};
+    if (c->inc_on && c->inc_tiles) {
+        P.inc.rtiles = c->tile_list[2];
+        P.inc.rmark = c->tile_mark;
+        if (c->inc_tiles == 2) P.inc.tiles = c->tile_list[c->inc_kind];
+    }
     return P;
 }
 
@@ -557,7 +562,7 @@ static void tile_maps(pt_ctx* c, const Params& P, int tm, int tile_h, TileMaps* 
 static std::mutex g_tune_mutex;
 static std::map<std::tuple<int, int, int, int, int>, int> g_tune;  // (device, shape) -> choice
 
-static int sm_count(pt_ctx* c) {
+int sm_count(pt_ctx* c) {
     if (!c->sm_count) {
         if (cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
             cudaGetLastError();
@@ -626,8 +631,17 @@ static int propagate_variant(pt_ctx* c, const Params& P, int tm, int* probe) {
 // sizes measured (summed launches, four / two lanes): all levels of a 128x128
 // still 0.44 / 0.64 ms, of four 512x512 frames 16.1 / 17.3 ms, of a 1024x1024
 // still 3.66 / 3.07 ms, of two 1080p frames 55.8 / 50.8 ms.
-static int scatter_wide(pt_ctx* c, const Params& P) {
+int scatter_wide(pt_ctx* c, const Params& P) {
     return (long long)P.lw * P.lh <= 2048ll * sm_count(c);
+}
+
+// The residual's: four (1) for levels that leave the GPU short of warps, one
+// (0; the exact filter's, two) for the others.  Measured at limits of 256, 512
+// and 1024 pixels an SM: four 512x512 frames 23.8 / 22.8 / 22.8 ms, two 1080p
+// frames 48.1 / 48.1 / 47.7 ms, a 480x270 level through the steps 1.48 / 1.47 /
+// 1.25 ms; four lanes at every size 2-60 % slower from 512x512 on.
+int resid_wide(pt_ctx* c, const Params& P) {
+    return (long long)P.lw * P.lh <= 1024ll * sm_count(c);
 }
 
 cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,
@@ -637,9 +651,9 @@ cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work,
     int tm = temporal_mode(c);
     if (P.r < 2 || P.r > 4) return cudaSuccess;
     int probe = -1;
-    const int wide = kind == 0 ? propagate_variant(c, P, tm, &probe) : kind == 1 ? scatter_wide(c, P) : 0;
+    const int wide = kind == 0 ? propagate_variant(c, P, tm, &probe) : kind == 1 ? scatter_wide(c, P) : resid_wide(c, P);
     TileMaps M;
-    tile_maps(c, P, tm, kind == 2 ? ptk::kTileH : kind == 0 ? ptk::kPropH : wide ? ptk::kScatHWide : ptk::kScatH, &M);
+    tile_maps(c, P, tm, kind == 2 ? (wide ? ptk::kResidHWide : ptk::kResidH) : kind == 0 ? ptk::kPropH : wide ? ptk::kScatHWide : ptk::kScatH, &M);
     int blocks = 0;
     pt_ctx::Tune* t = probe >= 0 ? &c->tune[tune_key(c, P, tm, &blocks)] : nullptr;
     if (t) cudaEventRecord(t->ev[2 * probe], c->stream);
@@ -964,6 +978,8 @@ pt_status pt_initialize(pt_ctx* c, int iw, int ih, int sw, int sh, int ns) {
     dfree_t(c, c->chg); dfree_t(c, c->stamp_last); dfree_t(c, c->stamp_win);
     dfree_t(c, c->tap_cache);
     c->tap_cache_k = 0;
+    for (auto& t : c->tile_list) dfree_t(c, t);
+    dfree_t(c, c->tile_mark);
     free_store(c);
     c->initialized = false;
     c->W = iw; c->H = ih; c->SW = sw; c->SH = sh; c->NS = ns;

@@ -238,6 +238,12 @@ struct pt_ctx {
     int* stamp_win = nullptr;
     int inc_seq = 0;        // index of the last tracked pass
     int inc_on = 0, inc_pi = 0, inc_prev = INT_MIN;
+    // active tile lists: propagate's, scatter's (its shape of the level) and
+    // the residual's with its marks; inc_tiles: the lists of this pass
+    int* tile_list[3] = {nullptr, nullptr, nullptr};
+    int* tile_mark = nullptr;
+    int inc_tiles = 0;      // 0: none, 1: the residual's, 2: all
+    int inc_kind = 0;       // the pass runs propagate (0) or scatter (1)
     int inc_fill = 0;       // the next residual computes and stores every tap value
     float* tap_cache = nullptr;  // per-tap residual values, (2r+1)^2 planes
     int tap_cache_k = 0;         // planes allocated
@@ -304,6 +310,9 @@ PT_HIDDEN pt_status refresh_interleaved(pt_ctx* c, ExLevel* L);
 PT_HIDDEN pt_status reset_image_slots(pt_ctx* c);
 PT_HIDDEN pt_status reset_working(pt_ctx* c);
 PT_HIDDEN bool tiled_usable(pt_ctx* c);
+PT_HIDDEN int scatter_wide(pt_ctx* c, const Params& P);
+PT_HIDDEN int resid_wide(pt_ctx* c, const Params& P);
+PT_HIDDEN int sm_count(pt_ctx* c);
 PT_HIDDEN pt_status writable_work(pt_ctx* c, int level, PatchPlanes* out, bool* was_aliased = nullptr);
 
 template <class T>

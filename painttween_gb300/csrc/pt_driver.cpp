@@ -178,6 +178,27 @@ static pt_status propagate_and_scatter(pt_ctx* c, int level, int iterations, boo
             fill_after_first = true;
         }
     }
+    // Levels with more tiles than the GPU holds at once (those of the
+    // residual's narrow shape, more than 8 tiles an SM) list those that have work: a block of an idle tile ends after its checks, but keeps its place
+    // from another for the time of two or three loads.  Four fifths of a 1080p
+    // frame's tiles are culled: propagate 162 -> 149 ms, scatter 49.6 -> 48.1
+    // ms over two such frames, propagate of a 1024x1024 still 11.3 -> 10.4 ms;
+    // on levels that fit at once the lists' launches cost more than they save.
+    bool lists = false;
+    int passes = 0;
+    if (track) {
+        Params P = make_params(c, level);
+        lists = P.lw < 65536 * ptk::kTileW && P.lh < 65536 && !resid_wide(c, P);  // (the list's tiles are the narrow shape's)
+        if (lists) {
+            if (!c->tile_mark) {
+                const size_t n = (size_t)((c->W + ptk::kTileW - 1) / ptk::kTileW) * ((c->H + 1) / 2);
+                for (auto& t : c->tile_list) TRY(dalloc_t(c, &t, n + 1));
+                TRY(dalloc_t(c, &c->tile_mark, n));
+            }
+            LN(pt::launch_active_tiles(P, ptk::kPropH, c->tile_list[0], c->stream));
+            LN(pt::launch_active_tiles(P, scatter_wide(c, P) ? ptk::kScatHWide : ptk::kScatH, c->tile_list[1], c->stream));
+        }
+    }
     std::map<int, int> last_pass;  // jump (0 = scatter) -> index of its last pass
     auto run = [&](int jump) -> pt_status {
         if (fill_after_first) {
@@ -194,9 +215,15 @@ static pt_status propagate_and_scatter(pt_ctx* c, int level, int iterations, boo
             bool same = it != last_pass.end() && (jump != 0 || c->params.rngMode != PT_RNG_COUNTER);
             c->inc_prev = same ? it->second : INT_MIN;
             last_pass[jump] = c->inc_pi;
+            // the loop's first two passes write the culled pixels' records
+            // into both buffers; from then on they stay as they are
+            c->inc_tiles = lists ? (passes >= 2 ? 2 : 1) : 0;
+            c->inc_kind = jump ? 0 : 1;
         }
+        passes++;
         pt_status st = jump ? pt_propagate(c, level, jump, key) : pt_scatter(c, level, key);
         c->inc_on = 0;
+        c->inc_tiles = 0;
         c->inc_prev = INT_MIN;
         return st;
     };

@@ -38,6 +38,12 @@ struct PropShape {
     static constexpr int kBlocks = (HW == 0 || TM) ? (CPL == 1 ? 1 : 2) : (CPL == 1 ? 2 : 3);
 };
 
+// The residual's, by lanes per pixel.
+template <int LPP, int HW>
+struct ResidShape {
+    static constexpr int kBlocks = LPP == 1 ? 4 : LPP == 2 ? 2 : 3;
+};
+
 enum { TM_NONE = 0, TM_FWD = 1, TM_BWD = 2 };
 
 // The staged planes start on 128-byte boundaries (tensor copies write
@@ -167,18 +173,6 @@ __device__ __forceinline__ bool footprint_inside(float x, float y, float2 b0, fl
 // exactly sum / sumW.  A NaN thr2 (no early exit, or best = kNoBest) never
 // stops a sum, so the energy is computed in full, NaN and inf included.
 constexpr float kNoBest = __builtin_nanf("");
-__device__ __forceinline__ float exit_threshold(const Params& P, const PixT& px, float best) {
-    return (P.earlyExit && px.sumW >= kEpsilon) ? __fmul_ru(best, px.sumW) : kNoBest;
-}
-
-// taps a loop processed before it stopped: the valid taps of its first
-// `cols` columns
-template <int R>
-__device__ __forceinline__ unsigned taps_done(const PixT& px, int cols) {
-    const int last = min(-R + cols - 1, px.imax);
-    return last < px.imin ? 0u : (unsigned)((last - px.imin + 1) * (px.jmax - px.jmin + 1));
-}
-
 __device__ __forceinline__ void count_taps(const Params& P, unsigned taps, bool temporal) {
     unsigned mask = __activemask();
     unsigned tsum = __reduce_add_sync(mask, taps);
@@ -187,109 +181,6 @@ __device__ __forceinline__ void count_taps(const Params& P, unsigned taps, bool 
         atomicAdd(&P.counters[1], (unsigned long long)tsum);
         atomicAdd(&P.counters[2], (unsigned long long)ttsum);
     }
-}
-
-// One body for both cases: the single-candidate kernels (scatter in
-// particular) are instruction-cache bound, and a second, compile-time fast
-// copy of this loop measured slower there.  EE: the early-exit test is
-// compiled in (false for the residual, which always needs the full sum).
-template <int R, int TM, int HW, bool EE>
-__device__ __forceinline__ float energy_taps(const Params& P, const TileSmem<R, TM>& T, const PixT& px,
-                                             const Cand& c, float2 b0, float2 b1, float sum0, bool fast,
-                                             bool fastp, float thr2) {
-    constexpr int TW = TileSmem<R, TM>::TW;
-    const size_t lsz = (size_t)P.ex.w * P.ex.h;
-    const int li = ex_layer(P.ex, c.layer);
-    const size_t lo = (size_t)li * lsz;
-    const float4* LBO = P.ex.bo + 2 * lo;
-    const int lpi = TM ? ex_layer(P.ex, px.prev.layer) : 0;
-    const size_t lp = (size_t)lpi * lsz;
-    const float hw = (float)P.histW, hh = (float)P.histH;
-    const unsigned mask = __activemask();
-    float sum = sum0;
-    bool act = EE ? !(sum >= thr2) : true;
-    int cols = 0;
-#pragma unroll 1
-    for (int i = -R; i <= R; i++) {
-        if (EE && !__any_sync(mask, act)) break;
-        cols += act ? 1 : 0;
-        if (act) {
-#pragma unroll
-            for (int j = -R; j <= R; j++) {
-                const bool valid = (i >= px.imin) && (i <= px.imax) && (j >= px.jmin) && (j <= px.jmax);
-                const int s = px.sidx + j * TW + i;
-                float4 base = T.base[s];
-                float4 canvas = T.canvas[s];
-                float tx = c.x + fmaf((float)i, b0.x, (float)j * b1.x);
-                float ty = c.y + fmaf((float)i, b0.y, (float)j * b1.y);
-                if (!fast) {
-                    if (tx >= hw) tx -= hw; else if (tx < 0) tx += hw;
-                    if (ty >= hh) ty -= hh; else if (ty < 0) ty += hh;
-                }
-                float4 tb, to;
-                sample2<true, HW>(P.ex, li, LBO, tx, ty, &tb, &to, fast);
-                float res = ssd_ap(base, tb, P.alphaWeight) * P.inputAnalogyWeight;
-                if (TM) {
-                    if (px.temporal) {
-                        float4 pbase = T.pbase[s], pout = T.pout[s];
-                        float ptx = px.prev.x + fmaf((float)i, px.pb0.x, (float)j * px.pb1.x);
-                        float pty = px.prev.y + fmaf((float)i, px.pb0.y, (float)j * px.pb1.y);
-                        float4 peb, peo;
-                        sample2<true, HW>(P.ex, lpi, P.ex.bo + 2 * lp, ptx, pty, &peb, &peo, fastp);
-                        float r = ssdp(sub4p(base, pbase), sub4p(tb, peb)) * P.tdIn;
-                        r = fmaf(ssdp(sub4p(canvas, pout), sub4p(to, peo)), P.tdOut, r);
-                        r = fmaf(ssdp(pout, to), P.tc, r);
-                        res = T.pvalid[s] ? res + r : res;
-                    }
-                }
-                if (i == 0 && j == 0) {
-                    if (P.distTransWeight > 0.f) {
-                        float de = ex_sample_dt(ex_mode<HW>(P.ex), tx, ty, c.layer) / c.sv;
-                        float di = lay_texel(P.img.dt[P.img.cur], P, px.x, px.y);
-                        float diff = fmaxf(0.0f, fminf(fabsf(de - di), 10.0f));  // clamp(diff, 0, 10): a NaN difference gives 10
-                        res = res + diff * P.distTransWeight;
-                    }
-                    {
-                        int Lh = clampi(c.layer, 0, PT_MAX_STYLES - 1);
-                        float sh = (float)(P.histH / P.numStyles);
-                        int hx = clampi((int)tx, 0, P.histPitch - 1);
-                        int hy = clampi((int)(ty + sh * (float)c.layer), 0, P.histRows - 1);
-                        float h = __ldg(P.hist + (size_t)hy * P.histPitch + hx);
-                        float thr = P.histThreshold[Lh];
-                        res = res + ((h > thr) ? (h - thr) * P.histSlope[Lh] : 0.0f);
-                    }
-                    if (P.styleObjIdWeight > 0.f) {
-                        int imgID = lvl_texel(P.img.ids, px.x, px.y);
-                        int styleID = ex_point_id(P.ex, tx, ty, c.layer);
-                        res = res + ((imgID != styleID) ? P.styleObjIdWeight : 0.0f);
-                    }
-                } else {
-                    res = fmaf(ssd_ap(canvas, to, P.alphaWeight), P.canvasOutputWeight, res);
-                }
-                const float w = P.gauss[i + R] * P.gauss[j + R];
-                sum = valid ? fmaf(res, w, sum) : sum;
-            }
-            if (EE) act = !(sum >= thr2);
-        }
-    }
-    if (P.counters) count_taps(P, taps_done<R>(px, cols), px.temporal);
-    if (px.sumW < kEpsilon) return kBigResidual;
-    if (EE && sum >= thr2) return INFINITY;
-    return sum / px.sumW;
-}
-
-template <int R, int TM, int HW, bool EE>
-__device__ __forceinline__ float energy_tiled(const Params& P, const TileSmem<R, TM>& T, const PixT& px,
-                                           const Cand& c, float best) {
-    float sum0 = 0.0f;
-    if (px.hyst_on) sum0 = sum0 - px.hyst;
-    float2 b0, b1;
-    basis(c.theta, P.scaleWU * c.su, P.scaleWV * c.sv, &b0, &b1);
-    const unsigned mask = __activemask();
-    bool fast = __all_sync(mask, footprint_inside<R>(c.x, c.y, b0, b1, P.ex.w, P.ex.h));
-    bool fastp = TM ? __all_sync(mask, !px.temporal || px.prev_fast) : true;
-    return energy_taps<R, TM, HW, EE>(P, T, px, c, b0, b1, sum0, fast, fastp,
-                                  EE ? exit_threshold(P, px, best) : kNoBest);
 }
 
 // Tensor copies into shared memory (cp.async.bulk.tensor) completing on an
@@ -327,6 +218,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
+// The tile of this block: of a list of active tiles, or of the whole grid.
+// False past the list's end.
+__device__ __forceinline__ bool block_tile(const int* list, int2* tile) {
+    if (!list) {
+        *tile = make_int2(blockIdx.x, blockIdx.y);
+        return true;
+    }
+    const int i = blockIdx.y * gridDim.x + blockIdx.x;
+    const int n = __ldg(list), id = __ldg(list + 1 + i);  // (the list has room for every tile)
+    *tile = make_int2(id & 0xffff, id >> 16);
+    return i < n;
+}
+
 // Stages the tile (and halo) of the pixel-side inputs and fills the
 // state of pixel `pid` of the tile (several threads of a block of NT >
 // kTileThreads threads may ask for the same pixel).  Returns false for
@@ -337,12 +241,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 // the clamp rules.  *abort is set (for the whole block) when the copies did
 // not complete within two bounded waits; the block must then return.
 template <int R, int TM, int NT = kTileThreads, int H = kTileH>
-__device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, TileSmem<R, TM, H>& T, int pid,
-                                           PixT* px, bool* abort) {
+__device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, TileSmem<R, TM, H>& T, int2 tile,
+                                           int pid, PixT* px, bool* abort) {
     constexpr int TW = TileSmem<R, TM, H>::TW, TH = TileSmem<R, TM, H>::TH, N = TileSmem<R, TM, H>::N;
     const int tid = threadIdx.x + threadIdx.y * kTileW;
     const int lx = pid % kTileW, ly = pid / kTileW;
-    const int x0 = blockIdx.x * kTileW - R, y0 = blockIdx.y * H - R;
+    const int x0 = tile.x * kTileW - R, y0 = tile.y * H - R;
     *abort = false;
     const bool interior = M.on && x0 >= 0 && y0 >= 0 && x0 + TW <= P.lw && y0 + TH <= P.lh;  // (block-uniform)
     if (interior) {
@@ -387,7 +291,7 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
     }
     // the per-pixel state reads global memory only: with tensor copies it is
     // computed while they are in flight
-    const int x = blockIdx.x * kTileW + lx, y = blockIdx.y * H + ly;
+    const int x = tile.x * kTileW + lx, y = tile.y * H + ly;
     const bool in = x < P.lw && y < P.lh;
     if (in) {
         px->x = x;
@@ -468,55 +372,6 @@ __device__ __forceinline__ bool block_idle(const Params& P, PatchPlanes work, bo
     return true;
 }
 
-// updateResidualCache_kernel, texSynth_kernel.cu:661-693
-template <int R, int TM, int HW>
-__global__ void __launch_bounds__(kTileThreads, 2) kt_residual(const Params P, const __grid_constant__ TileMaps M,
-                                                                    float* out) {
-    __shared__ TileSmem<R, TM> T;
-    // Change tracking: only pixels with a changed record in their patch
-    // window get a new residual; the others keep theirs (the same inputs give
-    // the same value).  The pass stamps are updated here.
-    bool need = true;
-    if (P.inc.on) {
-        constexpr int TW = TileSmem<R, TM>::TW, N = TileSmem<R, TM>::N;
-        __shared__ uint8_t C[N];
-        const int tid = threadIdx.x + threadIdx.y * kTileW;
-        const int x0 = blockIdx.x * kTileW - R, y0 = blockIdx.y * kTileH - R;
-        for (int q = tid; q < N; q += kTileThreads) {
-            int gx = clampi(x0 + q % TW, 0, P.lw - 1);
-            int gy = clampi(y0 + q / TW, 0, P.lh - 1);
-            C[q] = P.inc.chg[(size_t)gy * P.W + gx];
-        }
-        __syncthreads();
-        const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
-        const bool in = x < P.lw && y < P.lh;
-        need = false;
-        if (in) {
-            const int c0 = threadIdx.y * TW + threadIdx.x;  // window corner
-            unsigned any = 0;
-#pragma unroll
-            for (int j = 0; j <= 2 * R; j++)
-#pragma unroll
-                for (int i = 0; i <= 2 * R; i++) any |= C[c0 + j * TW + i];
-            need = any != 0;
-            const size_t k = (size_t)y * P.W + x;
-            if (C[c0 + R * TW + R]) P.inc.last[k] = P.inc.pi;
-            if (need) P.inc.win[k] = P.inc.pi;
-        }
-        if (!__syncthreads_or(need)) return;
-    }
-    PixT px;
-    bool abort;
-    if (!stage_tile<R, TM>(P, M, T, threadIdx.x + threadIdx.y * kTileW, &px, &abort)) return;
-    if (!need) return;
-    const size_t k = (size_t)px.y * P.W + px.x;
-    if (image_culled(P, px.x, px.y)) { out[k] = 0.0f; return; }
-    Patch t = load_patch(P.off, k);
-    Cand c{t.x, t.y, t.theta, t.su, t.sv, t.layer};
-    if (P.counters) count_eval(P, px.x, px.y, px.temporal, false);
-    out[k] = energy_tiled<R, TM, HW, false>(P, T, px, c, kNoBest);
-}
-
 constexpr unsigned kFull = 0xffffffffu;
 // (1 -/+ 2^-17): bounds of the rounding of a reference-order sum of <= 81 terms
 constexpr float kBoundLo = 1.0f - 1.0f / 131072.0f;
@@ -530,19 +385,6 @@ struct LanePix {
     float prevx, prevy;
     int prevlayer;  // clamped to the exemplar's layers
     float2 pb0, pb1;
-};
-
-// candidate side of an evaluation and its cursor
-struct LaneEval {
-    float cx, cy, sv;
-    int layer;
-    float2 b0, b1;
-    bool fast;   // footprint inside the exemplar
-    bool exact;  // the reference-order pass (else the bound pass)
-    int col;     // exact pass: next column, -R..R; bound pass: next position in the weight order
-    float sum;   // exact pass: the running sum; bound pass: the lower bound of the weighted taps so far
-    float thr2;  // exit threshold (see exit_threshold)
-    float s0lo;  // lower bound of the start sum's share of the reference-order sum
 };
 
 template <int R>
@@ -577,12 +419,12 @@ __device__ __forceinline__ void put_pix(PixShared<NP>& S, int pid, const LanePix
 }
 
 template <int R, int TM, int NP>
-__device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>& S, int pid) {
+__device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>& S, int2 tile, int pid) {
     constexpr int TW = TileSmem<R, TM>::TW;
     LanePix q;
     const int lx = pid % kTileW, ly = pid / kTileW;
-    q.x = blockIdx.x * kTileW + lx;
-    q.y = blockIdx.y * (NP / kTileW) + ly;
+    q.x = tile.x * kTileW + lx;
+    q.y = tile.y * (NP / kTileW) + ly;
     q.sidx = (ly + R) * TW + lx + R;
     const float4 a = S.a[pid], b = S.b[pid];
     const int bits = S.bits[pid];
@@ -594,114 +436,6 @@ __device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>&
     q.sum0 = a.x; q.sumW = a.y; q.prevx = a.z; q.prevy = a.w;
     q.pb0 = make_float2(b.x, b.y); q.pb1 = make_float2(b.z, b.w);
     return q;
-}
-
-// best = the energy to beat (kNoBest: none, the energy is computed in full)
-template <int R>
-__device__ __forceinline__ void lane_start(const Params& P, const LanePix& q, float cx, float cy, float theta,
-                                           float su, float sv, int layer, float best, LaneEval* e) {
-    e->cx = cx; e->cy = cy; e->sv = sv; e->layer = layer;
-    basis(theta, P.scaleWU * su, P.scaleWV * sv, &e->b0, &e->b1);
-    e->fast = footprint_inside<R>(cx, cy, e->b0, e->b1, P.ex.w, P.ex.h);
-    e->thr2 = (P.earlyExit && q.sumW >= kEpsilon) ? __fmul_ru(best, q.sumW) : kNoBest;
-    // With an exit threshold, a bound pass over the taps by descending
-    // weight comes first (see lane_step); without one, or with one so small
-    // (|thr2| < 2^-100) that subnormal rounding could matter, only the exact
-    // pass.
-    e->exact = !(fabsf(e->thr2) >= 0x1p-100f);
-    e->col = e->exact ? -R : 0;
-    e->sum = e->exact ? q.sum0 : 0.0f;
-    e->s0lo = q.sum0 >= 0.0f ? __fmul_rd(q.sum0, kBoundLo) : __fmul_rd(q.sum0, kBoundHi);
-}
-
-// The exemplar samples of tap (i, j) of candidate e at pixel q (and, for a
-// temporal pixel, of its previous offset), with the sample position.
-struct TapSample {
-    float4 tb, to, peb, peo;
-    float tx, ty;
-};
-
-template <int R, int TM, int HW>
-__device__ __forceinline__ void tap_fetch(const Params& P, const LanePix& q, const LaneEval& e, int i, int j,
-                                          bool fast, bool fastp, TapSample* t) {
-    const size_t lsz = (size_t)P.ex.w * P.ex.h;
-    const int li = ex_layer(P.ex, e.layer);
-    const size_t lo = (size_t)li * lsz;
-    const float4* LBO = P.ex.bo + 2 * lo;
-    const size_t lp = TM ? (size_t)q.prevlayer * lsz : 0;
-    const float hw = (float)P.histW, hh = (float)P.histH;
-    float tx = e.cx + fmaf((float)i, e.b0.x, (float)j * e.b1.x);
-    float ty = e.cy + fmaf((float)i, e.b0.y, (float)j * e.b1.y);
-    if (!fast) {
-        if (tx >= hw) tx -= hw; else if (tx < 0) tx += hw;
-        if (ty >= hh) ty -= hh; else if (ty < 0) ty += hh;
-    }
-    sample2<true, HW>(P.ex, li, LBO, tx, ty, &t->tb, &t->to, fast);
-    t->tx = tx;
-    t->ty = ty;
-    if (TM && q.temporal) {
-        float ptx = q.prevx + fmaf((float)i, q.pb0.x, (float)j * q.pb1.x);
-        float pty = q.prevy + fmaf((float)i, q.pb0.y, (float)j * q.pb1.y);
-        sample2<true, HW>(P.ex, TM ? q.prevlayer : 0, P.ex.bo + 2 * lp, ptx, pty, &t->peb, &t->peo, fastp);
-    }
-}
-
-// calculateResidual's value at tap (i, j) of candidate e at pixel q, before
-// its Gaussian weight (texSynth_kernel.cu:537-659), from the tap's samples
-template <int R, int TM, int HW>
-__device__ __forceinline__ float tap_finish(const Params& P, const TileSmem<R, TM>& T, const LanePix& q,
-                                            const LaneEval& e, int i, int j, const TapSample& t) {
-    constexpr int TW = TileSmem<R, TM>::TW;
-    const int s = q.sidx + j * TW + i;
-    const float4 base = T.base[s];
-    const float4 canvas = T.canvas[s];
-    const float4 tb = t.tb, to = t.to;
-    const float tx = t.tx, ty = t.ty;
-    float res = ssd_ap(base, tb, P.alphaWeight) * P.inputAnalogyWeight;
-    if (TM) {
-        if (q.temporal) {
-            const float4 pbase = T.pbase[s], pout = T.pout[s];
-            float r = ssdp(sub4p(base, pbase), sub4p(tb, t.peb)) * P.tdIn;
-            r = fmaf(ssdp(sub4p(canvas, pout), sub4p(to, t.peo)), P.tdOut, r);
-            r = fmaf(ssdp(pout, to), P.tc, r);
-            res = T.pvalid[s] ? res + r : res;
-        }
-    }
-    if (j == 0 && i == 0) {
-        if (P.distTransWeight > 0.f) {
-            float de = ex_sample_dt(ex_mode<HW>(P.ex), tx, ty, e.layer) / e.sv;
-            float di = lay_texel(P.img.dt[P.img.cur], P, q.x, q.y);
-            float diff = fmaxf(0.0f, fminf(fabsf(de - di), 10.0f));  // clamp(diff, 0, 10): a NaN difference gives 10
-            res = res + diff * P.distTransWeight;
-        }
-        {
-            int Lh = clampi(e.layer, 0, PT_MAX_STYLES - 1);
-            float sh = (float)(P.histH / P.numStyles);
-            int hx = clampi((int)tx, 0, P.histPitch - 1);
-            int hy = clampi((int)(ty + sh * (float)e.layer), 0, P.histRows - 1);
-            float h = __ldg(P.hist + (size_t)hy * P.histPitch + hx);
-            float thr = P.histThreshold[Lh];
-            res = res + ((h > thr) ? (h - thr) * P.histSlope[Lh] : 0.0f);
-        }
-        if (P.styleObjIdWeight > 0.f) {
-            int imgID = lvl_texel(P.img.ids, q.x, q.y);
-            int styleID = ex_point_id(P.ex, tx, ty, e.layer);
-            res = res + ((imgID != styleID) ? P.styleObjIdWeight : 0.0f);
-        }
-    } else {
-        res = fmaf(ssd_ap(canvas, to, P.alphaWeight), P.canvasOutputWeight, res);
-    }
-    return res;
-}
-
-// calculateResidual's value at tap (i, j) of candidate e at pixel q, before
-// its Gaussian weight; fast / fastp are warp-uniform
-template <int R, int TM, int HW>
-__device__ __forceinline__ float tap_value(const Params& P, const TileSmem<R, TM>& T, const LanePix& q,
-                                           const LaneEval& e, int i, int j, bool fast, bool fastp) {
-    TapSample t;
-    tap_fetch<R, TM, HW>(P, q, e, i, j, fast, fastp, &t);
-    return tap_finish<R, TM, HW>(P, T, q, e, i, j, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -769,6 +503,27 @@ __device__ __forceinline__ void load_tap_list(const Params& P, TapList<R>& L, in
         a.code = i | (j << 4) | (t << 8) | (((j - R) * (kTileW + 2 * R) + i - R) * 65536);
         L.tap[tid] = a;
         L.w[t] = a.w;
+    }
+}
+
+// the taps in the reference's order
+template <int R>
+struct TapPlace {
+    Tap tap[(2 * R + 1) * (2 * R + 1)];
+    float w[(2 * R + 1) * (2 * R + 1)];
+};
+template <int R>
+__device__ __forceinline__ void load_tap_place(const Params& P, TapPlace<R>& L, int tid) {
+    constexpr int n = 2 * R + 1;
+    if (tid < n * n) {
+        const int i = tid / n, j = tid % n;
+        Tap a;
+        a.fi = (float)(i - R);
+        a.fj = (float)(j - R);
+        a.w = P.gauss[i] * P.gauss[j];
+        a.code = i | (j << 4) | (tid << 8) | (((j - R) * (kTileW + 2 * R) + i - R) * 65536);
+        L.tap[tid] = a;
+        L.w[tid] = a.w;
     }
 }
 
@@ -886,8 +641,23 @@ __device__ __forceinline__ float center_terms(const Params& P, const LanePix& q,
     return res;
 }
 
+// calculateResidual's value at one tap, before its weight, of record c at its
+// pixel q
+template <int R, int TM, int HW, int H>
+__device__ __forceinline__ float own_tap(const Params& P, const TileSmem<R, TM, H>& T, const LanePix& q,
+                                         const CandPos& c, float sv, const Tap& tp, bool fast, bool fastp) {
+    const PixSample p = pix_sample<R, TM, H>(T, q, q.sidx + (tp.code >> 16));
+    ExSample v;
+    float tx, ty;
+    if (TM && p.prev) v = prev_fetch<HW>(P, q, tp.fi, tp.fj, fastp);
+    const ExSample s = cand_fetch<HW>(P, c, tp.fi, tp.fj, fast, &tx, &ty);
+    const bool center = tp.fi == 0.0f && tp.fj == 0.0f;
+    const float r = tap_terms<TM>(P, p, s, v, center);
+    return center ? center_terms<HW>(P, q, c.layer, sv, tx, ty, r) : r;
+}
+
 // thr2 and the bound pass's threshold of a pixel whose energy to beat is
-// `best` (see exit_threshold): the latter is NaN, which rejects nothing,
+// `best` (see kNoBest): the latter is NaN, which rejects nothing,
 // where the bound is not used
 struct Threshold {
     float thr2, bound;
@@ -995,7 +765,7 @@ __device__ __forceinline__ int queue_survivors(const Params& P, WarpQueue<CAP>& 
 template <int R, int TM, int HW, int H, int CAP, int CH>
 __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM, H>& T,
                                            const PixShared<kTileW * H>& S, const TapList<R>& L,
-                                           const WarpQueue<CAP>& Q, int n, const float* thr,
+                                           const WarpQueue<CAP>& Q, int2 tile, int n, const float* thr,
                                            float* V, float* energy) {
     constexpr int K = (2 * R + 1) * (2 * R + 1);
     constexpr int kStride = (K + 3) / 4 * 4;
@@ -1026,7 +796,7 @@ __device__ __forceinline__ void eval_queue(const Params& P, const TileSmem<R, TM
                 c.b1 = make_float2(b.x, b.y);
                 c.layer = __float_as_int(b.w);
                 sum = b.z;
-                q = get_pix<R, TM>(P, S, id / CH);
+                q = get_pix<R, TM>(P, S, tile, id / CH);
                 th = threshold_of(P, q, thr[id / CH]);
                 if (l == 0) val[K / 2] = Q.v0[t];
                 step = 0;
@@ -1155,6 +925,9 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     extern __shared__ __align__(128) unsigned char dyn[];
     Tile& T = *reinterpret_cast<Tile*>(dyn);
     Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    int2 tile;
+    if (P.inc.rtiles && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) P.inc.rtiles[0] = 0;
+    if (!block_tile(P.inc.tiles, &tile)) return;
     const int tid = threadIdx.x + threadIdx.y * kTileW, warp = tid / 32, lane = tid % 32;
     const int pid = warp * PPW + lane % PPW, slot0 = lane / PPW * CPL;  // the lane's pixel and first candidate
     const bool head = slot0 == 0;                                      // the lane that writes its pixel
@@ -1164,7 +937,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     // `skip`); a pass without a previous one skips nothing.
     unsigned skip = 0;
     if (P.inc.on) {
-        const int x = blockIdx.x * kTileW + pid % kTileW, y = blockIdx.y * H + pid / kTileW;
+        const int x = tile.x * kTileW + pid % kTileW, y = tile.y * H + pid / kTileW;
         const bool in = x < P.lw && y < P.lh;
         const size_t k = (size_t)y * P.W + x;
         bool need = in;
@@ -1188,7 +961,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     load_tap_list<R>(P, E.L, tid);
     PixT px;
     bool abort;
-    const bool in = stage_tile<R, TM, NT, H>(P, M, T, pid, &px, &abort);  // (synchronises the block)
+    const bool in = stage_tile<R, TM, NT, H>(P, M, T, tile, pid, &px, &abort);  // (synchronises the block)
     if (abort) return;
     const int x = px.x, y = px.y;
     const size_t k = in ? (size_t)y * P.W + x : 0;
@@ -1255,7 +1028,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     float sum[CPL], v0[CPL];
     alive = front_taps<R, TM, HW, CPL, H>(P, T, E.L, q, th, c, sv, alive, sum, v0);
     const int n = queue_survivors<R, CPL>(P, E.Q[warp], pid * 4 + slot0, alive, c, sum, v0);
-    eval_queue<R, TM, HW, H, 32 * CPL, 4>(P, T, E.S, E.L, E.Q[warp], n, E.thr, E.V[warp], E.energy);
+    eval_queue<R, TM, HW, H, 32 * CPL, 4>(P, T, E.S, E.L, E.Q[warp], tile, n, E.thr, E.V[warp], E.energy);
     __syncwarp();
     // each pixel takes the first candidate, in the reference's order, that
     // beats its running best
@@ -1305,6 +1078,9 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     extern __shared__ __align__(128) unsigned char dyn[];
     Tile& T = *reinterpret_cast<Tile*>(dyn);
     Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    int2 tile;
+    if (P.inc.rtiles && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) P.inc.rtiles[0] = 0;
+    if (!block_tile(P.inc.tiles, &tile)) return;
     const int tid = threadIdx.x + threadIdx.y * kTileW, warp = tid / 32, lane = tid % 32;
     const int pid = warp * PPW + lane % PPW, sub = lane / PPW;
     const bool head = sub == 0;  // the lane that writes its pixel
@@ -1314,7 +1090,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     // every candidate rejected there against the same residual, and again now.
     bool stable = false;
     if (P.inc.on) {
-        const int x = blockIdx.x * kTileW + pid % kTileW, y = blockIdx.y * H + pid / kTileW;
+        const int x = tile.x * kTileW + pid % kTileW, y = tile.y * H + pid / kTileW;
         const bool in = x < P.lw && y < P.lh;
         const size_t k = (size_t)y * P.W + x;
         stable = in && P.inc.prev != INT_MIN && __ldg(P.inc.win + k) < P.inc.prev;
@@ -1323,7 +1099,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     load_tap_list<R>(P, E.L, tid);
     PixT px;
     bool abort;
-    const bool in = stage_tile<R, TM, NT, H>(P, M, T, pid, &px, &abort);  // (synchronises the block)
+    const bool in = stage_tile<R, TM, NT, H>(P, M, T, tile, pid, &px, &abort);  // (synchronises the block)
     if (abort) return;
     const int x = px.x, y = px.y;
     const size_t k = in ? (size_t)y * P.W + x : 0;
@@ -1477,7 +1253,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
         float sum[NC], v0[NC];
         alive = front_taps<R, TM, HW, NC, H>(P, T, E.L, q, th, c, sv, alive, sum, v0);
         const int n = queue_survivors<R, NC>(P, E.Q[warp], pid * CH + sub * NC, alive, c, sum, v0);
-        eval_queue<R, TM, HW, H, 32 * NC, CH>(P, T, E.S, E.L, E.Q[warp], n, E.thr, E.V[warp], E.energy);
+        eval_queue<R, TM, HW, H, 32 * NC, CH>(P, T, E.S, E.L, E.Q[warp], tile, n, E.thr, E.V[warp], E.energy);
         __syncwarp();
         // the first candidate that beats the best, if any
         int win = -1;
@@ -1525,164 +1301,201 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     else if (write_all) store_patch(work, k, off);
 }
 
-// updateResidualCache_kernel, texSynth_kernel.cu:661-693, inside a tracked
-// propagate/scatter loop.  The residual is the reference-order weighted sum
-// of per-tap values; each pixel keeps those values (P.inc.taps).  A tap's
-// value changes only when the pixel's own record changed (all taps) or the
-// record of the pixel under the tap changed (its canvas), so only those taps
-// are recomputed and the sum is then taken again over the stored values:
-// the same operations on the same values, so the same bits.  With `fill`
-// every tap of every pixel is computed (the loop's first residual).
-template <int R, int TM, int HW>
-__global__ void __launch_bounds__(kTileThreads, 2) kt_residual_inc(const Params P, const __grid_constant__ TileMaps M,
-                                                                        float* out) {
-    constexpr int TW = TileSmem<R, TM>::TW, N = TileSmem<R, TM>::N, K = (2 * R + 1) * (2 * R + 1);
-    __shared__ TileSmem<R, TM> T;
-    __shared__ PixShared<> S;
-    __shared__ float4 CA[kTileThreads];  // own record: x, y, sv, layer bits | fast << 30
-    __shared__ float4 CB[kTileThreads];  // its basis
-    __shared__ uint16_t list[kTileThreads * K];  // pid << 7 | tap
-    __shared__ uint8_t C[N];
-    __shared__ int count;
-    const int pid = threadIdx.x + threadIdx.y * kTileW;
-    const size_t plane = (size_t)P.W * P.H;
-    const int x0 = blockIdx.x * kTileW - R, y0 = blockIdx.y * kTileH - R;
-    if (!P.inc.fill) {
-        for (int q = pid; q < N; q += kTileThreads) {
-            int gx = clampi(x0 + q % TW, 0, P.lw - 1);
-            int gy = clampi(y0 + q / TW, 0, P.lh - 1);
-            C[q] = P.inc.chg[(size_t)gy * P.W + gx];
-        }
-    }
-    if (pid == 0) count = 0;
-    __syncthreads();
-    // tap mask of this pixel (bit t: recompute tap t) and the pass stamps
-    const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
+// updateResidualCache_kernel, texSynth_kernel.cu:661-693, over tiles of 32 x H
+// pixels.  The residual is the reference-order weighted sum of per-tap values;
+// LPP lanes of a pixel take its taps side by side, the values are kept and
+// then summed in order.
+//
+// KEEP: inside a tracked propagate/scatter loop the values stay in P.inc.taps.
+// A tap's value changes only when the pixel's own record changed (all taps) or
+// the record of the pixel under the tap changed (its canvas), so only those
+// taps are recomputed, queued per warp tap by tap so that neighbouring lanes
+// sample neighbouring texels, and the sum is then taken again over the stored
+// values: the same operations on the same values, so the same bits.  With
+// `fill` every tap of every pixel is computed (the loop's first residual).
+// Otherwise the values stay in shared memory.
+//
+// What bounds it is the time of the checks, loads and barriers around few
+// taps: most tiles have none or a handful to recompute.  So tiles come from
+// the canvas kernel's list on large levels, the changed records are a bit
+// each, from which a row of a window is a shift, and a warp queues and sums
+// alone.  Before: a lane a pixel over 32 x 8 tiles, the changed records a byte
+// each, one queue a block between barriers.  Measured, summed launches: two
+// 1080p frames 56.6 -> 47.7 ms, radius 4 at 192x160 4.8 -> 4.1 ms; without the
+// lists the same kernel took 70 ms.  ResidShape: with one lane a pixel four
+// blocks an SM 49.8, five 50.2, six 55.2 ms (two 1080p frames).
+template <int R, int NW, int NP, bool KEEP>
+struct ResidSmem {
+    static constexpr int K = (2 * R + 1) * (2 * R + 1);
+    PixShared<NP> S;
+    float4 own[NP];   // the pixel's record: x, y, basis b0
+    float4 own2[NP];  // basis b1, sv, layer bits
+    uint8_t fast[NP];  // its footprint is inside the exemplar
+    TapPlace<R> L;
+    uint16_t list[KEEP ? NW : 1][KEEP ? NP / NW * K : 1];  // pixel of the warp << 8 | tap
+    float v[KEEP ? 1 : NP][KEEP ? 1 : K];
+    unsigned long long chg[NP / kTileW + 2 * R];  // the changed records of each row of tile and halo, a bit each
+};
+
+template <int R, int TM, int HW, int LPP, int H, bool KEEP>
+__global__ void __launch_bounds__(kTileW * H * LPP, ResidShape<LPP, HW>::kBlocks)
+    kt_residual(const Params P, const __grid_constant__ TileMaps M, float* out) {
+    constexpr int NP = kTileW * H, NT = NP * LPP, NW = NT / 32, PPW = 32 / LPP;
+    constexpr int n1 = 2 * R + 1, K = n1 * n1;
+    using Tile = TileSmem<R, TM, H>;
+    using Shared = ResidSmem<R, NW, NP, KEEP>;
+    extern __shared__ __align__(128) unsigned char dyn[];
+    Tile& T = *reinterpret_cast<Tile*>(dyn);
+    Shared& E = *reinterpret_cast<Shared*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    constexpr int TW = Tile::TW, N = Tile::N;
+    int2 tile;
+    if (!block_tile(P.inc.fill ? nullptr : P.inc.rtiles, &tile)) return;
+    const int tid = threadIdx.x + threadIdx.y * kTileW, warp = tid / 32, lane = tid % 32;
+    const int lp = lane % PPW, pid = warp * PPW + lp, sub = lane / PPW;
+    const int lx = pid % kTileW, ly = pid / kTileW;
+    const int x = tile.x * kTileW + lx, y = tile.y * H + ly;
     const bool in = x < P.lw && y < P.lh;
-    const size_t k = (size_t)y * P.W + x;
-    const int c0 = threadIdx.y * TW + threadIdx.x;  // window corner in C
-    uint64_t m0 = 0, m1 = 0;                        // taps 0..63, 64..80
-    bool own = P.inc.fill != 0;
-    if (in && !P.inc.fill) {
-        own = C[c0 + R * TW + R] != 0;
-#pragma unroll
-        for (int t = 0; t < K; t++) {
-            const int i = t / (2 * R + 1), j = t % (2 * R + 1);  // column-major (reference order)
-            if (C[c0 + j * TW + i]) {
-                if (t < 64) m0 |= 1ull << t; else m1 |= 1ull << (t - 64);
+    const size_t k = in ? (size_t)y * P.W + x : 0;
+    const size_t plane = (size_t)P.W * P.H;
+    const bool dense = !KEEP || P.inc.fill;  // every tap of every pixel
+    bool own = in, any = in;
+    load_tap_place<R>(P, E.L, tid);
+    if (!dense) {
+        const int x0 = tile.x * kTileW - R, y0 = tile.y * H - R;
+        if (tid < Tile::TH) E.chg[tid] = 0;
+        __syncthreads();
+        bool some = false;
+        for (int q = tid; q < N; q += NT) {
+            const int gx = clampi(x0 + q % TW, 0, P.lw - 1), gy = clampi(y0 + q / TW, 0, P.lh - 1);
+            if (P.inc.chg[(size_t)gy * P.W + gx]) {
+                atomicOr(&E.chg[q / TW], 1ull << (q % TW));
+                some = true;
             }
         }
-        if (own) P.inc.last[k] = P.inc.pi;
-        if (m0 | m1) P.inc.win[k] = P.inc.pi;
+        if (!__syncthreads_or(some)) return;
+        unsigned all = 0;
+#pragma unroll
+        for (int j = 0; j < n1; j++) all |= (unsigned)(E.chg[ly + j] >> lx);
+        own = in && ((E.chg[ly + R] >> (lx + R)) & 1);
+        any = in && (all & ((1u << n1) - 1u));
+        if (sub == 0) {
+            if (own) P.inc.last[k] = P.inc.pi;
+            if (any) P.inc.win[k] = P.inc.pi;
+        }
     }
-    const bool need = in && (own || (m0 | m1));
-    if (!__syncthreads_or(need)) return;
     PixT px;
     bool abort;
-    stage_tile<R, TM>(P, M, T, pid, &px, &abort);  // (synchronises the block)
+    stage_tile<R, TM, NT, H>(P, M, T, tile, pid, &px, &abort);  // (synchronises the block)
     if (abort) return;
     bool mine = false;
-    int nt = 0;
-    if (need) {
+    LanePix q;
+    CandPos c;
+    float sv = 1.0f;
+    bool fast = true;
+    q.temporal = false;
+    q.prev_fast = true;
+    if (any) {
         if (image_culled(P, x, y)) {
-            out[k] = 0.0f;
+            if (sub == 0) out[k] = 0.0f;
         } else {
             mine = true;
-            const LanePix q = lane_pix<R>(P, px);
-            put_pix<R>(S, pid, q);
+            q = lane_pix<R>(P, px);
             const Patch o = load_patch(P.off, k);
-            LaneEval e;
-            lane_start<R>(P, q, o.x, o.y, o.theta, o.su, o.sv, o.layer, kNoBest, &e);
-            CA[pid] = make_float4(e.cx, e.cy, e.sv, __int_as_float(e.layer | (e.fast ? 1 << 30 : 0)));
-            CB[pid] = make_float4(e.b0.x, e.b0.y, e.b1.x, e.b1.y);
-            if (own) {  // every tap t < K
-                m0 = K >= 64 ? ~0ull : (1ull << K) - 1ull;
-                m1 = K > 64 ? (1ull << (K - 64)) - 1ull : 0ull;
+            c.x = o.x; c.y = o.y; c.layer = o.layer;
+            sv = o.sv;
+            basis(o.theta, P.scaleWU * o.su, P.scaleWV * o.sv, &c.b0, &c.b1);
+            fast = footprint_inside<R>(c.x, c.y, c.b0, c.b1, P.ex.w, P.ex.h);
+            if (sub == 0 && !dense) {
+                put_pix<R>(E.S, pid, q);
+                E.own[pid] = make_float4(c.x, c.y, c.b0.x, c.b0.y);
+                E.own2[pid] = make_float4(c.b1.x, c.b1.y, sv, __int_as_float(c.layer));
+                E.fast[pid] = fast;
             }
-            // only taps inside the level rectangle enter the sum
-#pragma unroll
-            for (int t = 0; t < K; t++) {
-                const int i = t / (2 * R + 1) - R, j = t % (2 * R + 1) - R;
-                const bool valid = (i >= q.imin) && (i <= q.imax) && (j >= q.jmin) && (j <= q.jmax);
-                if (!valid) {
-                    if (t < 64) m0 &= ~(1ull << t); else m1 &= ~(1ull << (t - 64));
-                }
-            }
-            nt = __popcll(m0) + __popcll(m1);
-            if (P.counters && own) count_eval(P, x, y, px.temporal, false);
+            if (P.counters && own && sub == 0) count_eval(P, x, y, px.temporal, false);
         }
     }
-    {
-        // queue this pixel's nt taps
-        const unsigned lane = lane_id();
-        int incl = nt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int v = __shfl_up_sync(kFull, incl, o);
-            if ((int)lane >= o) incl += v;
+    if (dense) {
+        // the lane's own pixel, every LPP-th tap
+        const bool wfast = __all_sync(kFull, !mine || fast);
+        const bool fastp = TM ? __all_sync(kFull, !mine || !q.temporal || q.prev_fast) : true;
+        unsigned taps = 0;
+#pragma unroll 2
+        for (int t = sub; t < K; t += LPP) {
+            const Tap tp = E.L.tap[t];
+            if (mine && tap_inside<R>(q, tp)) {
+                const float r = own_tap<R, TM, HW, H>(P, T, q, c, sv, tp, wfast, fastp);
+                if (KEEP) P.inc.taps[(size_t)t * plane + k] = r;
+                else E.v[pid][t] = r;
+                taps++;
+            }
         }
-        const int total = __shfl_sync(kFull, incl, 31);
-        int base = 0;
-        if (lane == 31 && total > 0) base = atomicAdd(&count, total);
-        base = __shfl_sync(kFull, base, 31);
-        int w = base + incl - nt;
-        for (int t = 0; t < K; t++) {
-            const bool b = t < 64 ? (m0 >> t) & 1 : (m1 >> (t - 64)) & 1;
-            if (mine && b && w < kTileThreads * K) list[w++] = (uint16_t)((pid << 7) | t);
-        }
-    }
-    __syncthreads();
-    // every lane takes every 256th queued tap
-    const int n = count;
+        if (P.counters) count_taps(P, taps, q.temporal);
+    } else {
+        // the warp's affected taps, tap by tap
+        int n = 0;
+        uint16_t* list = E.list[warp];
+        const unsigned cols = mine ? ((2u << (q.imax + R)) - 1u) & ~((1u << (q.imin + R)) - 1u) : 0u;
 #pragma unroll 1
-    for (int b = 0; b < n; b += kTileThreads) {
-        const int it = b + pid;
-        bool act = it < n;
-        LanePix q;
-        LaneEval e;
-        int t = 0, op = 0;
-        if (act) {
-            const int v = list[it];
-            op = v >> 7;
-            t = v & 127;
+        for (int j0 = 0; j0 < n1; j0 += LPP) {
+            const int j = j0 + sub;  // the lane's row of the window
+            unsigned bits = 0;
+            if (mine && j - R >= q.jmin && j - R <= q.jmax)
+                bits = own ? cols : (unsigned)(E.chg[ly + j] >> lx) & cols;
+            if (!__any_sync(kFull, bits)) continue;
+#pragma unroll
+            for (int i = 0; i < n1; i++) {
+                const bool b = (bits >> i) & 1;
+                const unsigned m = __ballot_sync(kFull, b);
+                if (b) list[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(lp << 8 | (i * n1 + j));
+                n += __popc(m);
+            }
         }
-        act = act && t < K && op < kTileThreads;  // (every queued entry satisfies this)
-        if (act) {
-            q = get_pix<R, TM>(P, S, op);
-            const float4 a = CA[op], bb = CB[op];
-            const int lb = __float_as_int(a.w);
-            e.cx = a.x; e.cy = a.y; e.sv = a.z;
-            e.layer = lb & ~(1 << 30);
-            e.fast = (lb >> 30) & 1;
-            e.b0 = make_float2(bb.x, bb.y);
-            e.b1 = make_float2(bb.z, bb.w);
-        }
-        const bool fast = __all_sync(kFull, !act || e.fast);
-        const bool fastp = TM ? __all_sync(kFull, !act || !q.temporal || q.prev_fast) : true;
-        if (act) {
-            const int i = t / (2 * R + 1) - R, j = t % (2 * R + 1) - R;
-            const float v = tap_value<R, TM, HW>(P, T, q, e, i, j, fast, fastp);
-            P.inc.taps[(size_t)t * plane + (size_t)q.y * P.W + q.x] = v;
+        __syncwarp();
+#pragma unroll 1
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const bool act = i0 + lane < n;
+            int t = 0, op = 0;
+            LanePix a;
+            CandPos ac;
+            float asv = 1.0f;
+            bool af = true;
+            a.temporal = false;
+            a.prev_fast = true;
+            if (act) {
+                const int v = list[i0 + lane];
+                t = v & 255;
+                op = warp * PPW + (v >> 8);
+                a = get_pix<R, TM>(P, E.S, tile, op);
+                const float4 o = E.own[op], o2 = E.own2[op];
+                ac.x = o.x; ac.y = o.y;
+                ac.b0 = make_float2(o.z, o.w);
+                ac.b1 = make_float2(o2.x, o2.y);
+                asv = o2.z;
+                ac.layer = __float_as_int(o2.w);
+                af = E.fast[op] != 0;
+            }
+            const bool wfast = __all_sync(kFull, af);
+            const bool fastp = TM ? __all_sync(kFull, !a.temporal || a.prev_fast) : true;
+            if (act)
+                P.inc.taps[(size_t)t * plane + (size_t)a.y * P.W + a.x] =
+                    own_tap<R, TM, HW, H>(P, T, a, ac, asv, E.L.tap[t], wfast, fastp);
+            if (P.counters) count_taps(P, act ? 1u : 0u, a.temporal);
         }
     }
-    if (P.counters) count_taps(P, (unsigned)nt, px.temporal);
-    __syncthreads();
-    // the residual: the stored values summed in the reference's order
-    if (mine) {
-        const LanePix q = get_pix<R, TM>(P, S, pid);
+    __syncwarp();
+    // the residual: the values summed in the reference's order
+    if (mine && sub == 0) {
         float sum = q.sum0;
+        const float* v = KEEP ? P.inc.taps + k : E.v[pid];
+        const size_t step = KEEP ? plane : 1;
+        const bool whole = q.imin == -R && q.imax == R && q.jmin == -R && q.jmax == R;
+        if (whole) {
+#pragma unroll n1
+            for (int t = 0; t < K; t++) sum = fmaf(v[t * step], E.L.w[t], sum);
+        } else {
 #pragma unroll 1
-        for (int i = -R; i <= R; i++) {
-            const float gi = P.gauss[i + R];
-            const bool cvalid = (i >= q.imin) && (i <= q.imax);
-#pragma unroll
-            for (int j = -R; j <= R; j++) {
-                const bool valid = cvalid && (j >= q.jmin) && (j <= q.jmax);
-                const int t = (i + R) * (2 * R + 1) + (j + R);
-                const float v = valid ? P.inc.taps[(size_t)t * plane + k] : 0.0f;
-                const float w = gi * P.gauss[j + R];
-                sum = valid ? fmaf(v, w, sum) : sum;
-            }
+            for (int t = 0; t < K; t++)
+                if (tap_inside<R>(q, E.L.tap[t])) sum = fmaf(v[t * step], E.L.w[t], sum);
         }
         out[k] = (q.sumW < kEpsilon) ? kBigResidual : sum / q.sumW;
     }
@@ -1728,10 +1541,21 @@ static cudaError_t launch_scatter_t(const Params& P, const TileMaps& M, PatchPla
     return cudaGetLastError();
 }
 
+template <int R, int TM, int HW, int LPP, int H, bool KEEP>
+static cudaError_t launch_residual_t(const Params& P, const TileMaps& M, float* out, cudaStream_t s) {
+    constexpr int NP = kTileW * H, NT = NP * LPP;
+    constexpr size_t smem = (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(ResidSmem<R, NT / 32, NP, KEEP>);
+    static std::atomic<uint64_t> done{0};
+    const cudaError_t e = allow_smem(kt_residual<R, TM, HW, LPP, H, KEEP>, smem, done);
+    if (e != cudaSuccess) return e;
+    const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
+    kt_residual<R, TM, HW, LPP, H, KEEP><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, out);
+    return cudaGetLastError();
+}
+
 template <int R>
 cudaError_t launch_tiled_r(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
                            uint32_t pass_id, float* out, int wide, cudaStream_t s) {
-    dim3 b(kTileW, kTileH), g((P.lw + kTileW - 1) / kTileW, (P.lh + kTileH - 1) / kTileH);
     // the texture-unit kernels fetch through the exemplar's textures, which
     // must be bound
     if (P.ex.hw && (!P.ex.tbase || !P.ex.tout)) return cudaErrorInvalidValue;
@@ -1741,8 +1565,12 @@ cudaError_t launch_tiled_r(int kind, int tm, const Params& P, const TileMaps& M,
     else if (kind == 1 && wide)                                                                        \
         return launch_scatter_t<R, TMV, HWV, 4, kScatHWide>(P, M, work, arg, pass_id, s);             \
     else if (kind == 1) return launch_scatter_t<R, TMV, HWV, 2, kScatH>(P, M, work, arg, pass_id, s);  \
-    else if (P.inc.on || P.inc.fill) kt_residual_inc<R, TMV, HWV><<<g, b, 0, s>>>(P, M, out);        \
-    else kt_residual<R, TMV, HWV><<<g, b, 0, s>>>(P, M, out);
+    else if (wide && (P.inc.on || P.inc.fill))                                                         \
+        return launch_residual_t<R, TMV, HWV, 4, kResidHWide, true>(P, M, out, s);                    \
+    else if (wide) return launch_residual_t<R, TMV, HWV, 4, kResidHWide, false>(P, M, out, s);        \
+    else if (P.inc.on || P.inc.fill)                                                                   \
+        return launch_residual_t<R, TMV, HWV, HWV ? 1 : 2, kResidH, true>(P, M, out, s);              \
+    else return launch_residual_t<R, TMV, HWV, HWV ? 1 : 2, kResidH, false>(P, M, out, s);
     if (P.ex.hw) {
         if (tm == TM_NONE) { PT_TILED_DISPATCH(TM_NONE, 1) }
         else if (tm == TM_FWD) { PT_TILED_DISPATCH(TM_FWD, 1) }

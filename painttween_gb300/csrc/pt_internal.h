@@ -53,6 +53,8 @@ cudaError_t launch_ribbon_pack(const Ribbon* src, int w, int h, float4* dst, cud
 cudaError_t launch_ribbon_down(const float4* src, int sw, float4* dst, int w, int h, cudaStream_t s);
 cudaError_t launch_residual(const Params& P, float* out, cudaStream_t s);
 cudaError_t launch_canvas(const Params& P, float4* canvas, cudaStream_t s);
+// the tiles (kTileW x tile_h) with a pixel that is not culled (IncView::tiles)
+cudaError_t launch_active_tiles(const Params& P, int tile_h, int* list, cudaStream_t s);
 cudaError_t launch_random_offsets(const Params& P, PatchPlanes work, cudaStream_t s);
 cudaError_t launch_upsample(const Params& P, PatchPlanes work, PatchPlanes border_src, int copy_border,
                             float* res_out, cudaStream_t s);

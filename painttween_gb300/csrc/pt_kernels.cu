@@ -177,8 +177,25 @@ __global__ void k_interleave_texels(const float4* base, const float4* out, const
 
 // offsetsToOutput, :263-274
 __global__ void k_canvas(const Params P, float4* canvas) {
-    PIXEL_XY
-    if (P.inc.on && !P.inc.chg[k]) return;  // tracked pass left this record unchanged
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    const size_t k = (size_t)y * P.W + x;
+    bool changed = in_rect(P, x, y);
+    if (P.inc.on) {
+        changed = changed && P.inc.chg[k];  // (a tracked pass left the other records unchanged)
+        if (P.inc.rtiles) {
+            // the residual's tiles (as large as this block, no smaller than
+            // the radius): this one and those around it
+            if (!__syncthreads_or(changed)) return;
+            const int t = threadIdx.y * blockDim.x + threadIdx.x;
+            if (t < 9) {
+                const int tx = (int)blockIdx.x + t % 3 - 1, ty = (int)blockIdx.y + t / 3 - 1;
+                if (tx >= 0 && ty >= 0 && tx < (int)gridDim.x && ty < (int)gridDim.y &&
+                    atomicExch(&P.inc.rmark[ty * gridDim.x + tx], P.inc.pi) != P.inc.pi)
+                    P.inc.rtiles[1 + atomicAdd(&P.inc.rtiles[0], 1)] = tx | ty << 16;
+            }
+        }
+    }
+    if (!changed) return;
     float4 a = __ldg(P.off.A + k);
     float lumy = __ldg(&P.off.B[k].w), luma = __ldg(P.off.C + k);
     float4 c = ex_sample_out(P.ex, a.x, a.y, __float_as_int(a.w));
@@ -381,6 +398,15 @@ __global__ void k_conv(const float* src, float* dst, int w, int h, int pitch, in
     dst[(size_t)y * pitch + x] = s;
 }
 
+// The tiles of blockDim.x x blockDim.y pixels that hold a pixel that is not
+// culled, in list[1 ...], their number in list[0] (zeroed before).
+__global__ void k_active_tiles(const Params P, int* list) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    const bool active = in_rect(P, x, y) && !image_culled(P, x, y);
+    if (__syncthreads_or(active) && threadIdx.x == 0 && threadIdx.y == 0)
+        list[1 + atomicAdd(&list[0], 1)] = (int)(blockIdx.x | blockIdx.y << 16);
+}
+
 // copies of the level rectangle
 __global__ void k_copy_patch(const Params P, PatchPlanes dst, PatchPlanes src) {
     PIXEL_XY
@@ -480,6 +506,7 @@ using namespace ptk;
 
 static inline dim3 grid2(int w, int h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h + b.y - 1) / b.y); }
 static const dim3 kPix(32, 4);
+static_assert(kResidH == 4 && kTileW == 32, "the canvas kernel gathers the residual's tiles, its own blocks");
 
 #define LAUNCH_CHECK() return cudaGetLastError()
 
@@ -498,6 +525,13 @@ cudaError_t launch_residual(const Params& P, float* out, cudaStream_t s) {
 }
 cudaError_t launch_canvas(const Params& P, float4* canvas, cudaStream_t s) {
     k_canvas<<<grid2(P.lw, P.lh, kPix), kPix, 0, s>>>(P, canvas);
+    LAUNCH_CHECK();
+}
+cudaError_t launch_active_tiles(const Params& P, int tile_h, int* list, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(list, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    const dim3 b(kTileW, tile_h);
+    k_active_tiles<<<grid2(P.lw, P.lh, b), b, 0, s>>>(P, list);
     LAUNCH_CHECK();
 }
 cudaError_t launch_random_offsets(const Params& P, PatchPlanes work, cudaStream_t s) {

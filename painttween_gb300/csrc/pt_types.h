@@ -16,6 +16,8 @@ constexpr int kTileH = 8;
 constexpr int kPropH = 4;       // tile height of propagate
 constexpr int kScatH = 4;       // of scatter with two lanes per pixel
 constexpr int kScatHWide = 2;   // and with four
+constexpr int kResidH = 4;      // of the residual
+constexpr int kResidHWide = 2;  // and with four lanes per pixel
 
 // Offset field in three planes (SoA of the 36-byte PatchXF):
 //   A = (x, y, theta, layer as int bits), B = (hysteresis, scaleU, scaleV,
@@ -116,6 +118,15 @@ struct IncView {
     // pitch, tap t = (i + r) * (2r + 1) + (j + r); `fill` recomputes all
     float* taps;
     int fill;
+    // The tiles a tiled kernel has work in: [0] their number, then each as
+    // x | y << 16 (null: all).  `tiles`: propagate's and scatter's (a pass from
+    // a loop's third on: those with a pixel that is not culled); `rtiles`: the
+    // residual's (those whose window holds a changed record), gathered by the
+    // canvas kernel, which marks a tile in rmark with the pass; the pass
+    // before it empties the list.
+    const int* tiles;
+    int* rtiles;
+    int* rmark;
 };
 
 struct Params {

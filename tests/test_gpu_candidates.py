@@ -58,3 +58,33 @@ def test_candidates_match_generic_kernels(w, h, kind, r, fm):
         for f in (0, 1):
             assert_offsets_equal(got[name][f][1], got["generic"][f][1], 1.0, "%s frame %d" % (name, f))
             assert_array_equal(got[name][f][0], got["generic"][f][0], "%s output frame %d" % (name, f))
+
+
+@pytest.mark.parametrize("r", [2, 3, 4])
+@pytest.mark.parametrize("w,h", [(640, 129), (1030, 270), (512, 512)])
+def test_active_tile_lists_change_nothing(w, h, r):
+    """Levels with enough tiles for the lists, most of them culled: change
+    tracking (which uses the lists) against none."""
+    from painttween_gb300 import Synthesizer
+    p = config_params(r=r, levels=3, iterations=2)
+    p.temporalCoherenceWeight = 0.5
+    p.distTransCull = 12
+    ex, clip = _inputs(w, h, "plain")
+    got = []
+    for on in (1, 0):
+        s = Synthesizer(device=0)
+        try:
+            s.set_incremental(on)
+            s.setup(p, w, h, 44, 38, 1)
+            s.set_style(0, ex["base"], ex["output"], ex["orient_tensor"], ex["dist_trans"], ex["object_ids"])
+            for i, fr in enumerate(clip):
+                s.set_frame_dict(i, fr)
+            got.append(s.synthesize_animation(0, 1))
+            res = [s.get_frame_residual(f) for f in (0, 1)]
+            got[-1] = {f: got[-1][f] + (res[f],) for f in (0, 1)}
+        finally:
+            s.close()
+    for f in (0, 1):
+        assert_offsets_equal(got[0][f][1], got[1][f][1], 1.0, "frame %d" % f)
+        assert_array_equal(got[0][f][0], got[1][f][0], "output frame %d" % f)
+        assert_array_equal(got[0][f][2], got[1][f][2], "residual frame %d" % f)
