@@ -20,6 +20,15 @@
 
 namespace ptk {
 
+// Programmatic dependent launch: the next kernel of the stream may take its
+// place on the GPU while this one's last blocks run (launch_dependents), and
+// waits before its first access to global memory until this one has ended and
+// its writes are visible (wait).
+__device__ __forceinline__ void pdl_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr float kAlphaThreshold = 0.99f;  // types.h:39
 constexpr float kEpsilon = 0.000001f;     // types.h:38
 constexpr float kBigResidual = (float)10e30;

@@ -925,6 +925,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
     extern __shared__ __align__(128) unsigned char dyn[];
     Tile& T = *reinterpret_cast<Tile*>(dyn);
     Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    pdl_start();
     int2 tile;
     if (P.inc.rtiles && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) P.inc.rtiles[0] = 0;
     if (!block_tile(P.inc.tiles, &tile)) return;
@@ -1078,6 +1079,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     extern __shared__ __align__(128) unsigned char dyn[];
     Tile& T = *reinterpret_cast<Tile*>(dyn);
     Eval& E = *reinterpret_cast<Eval*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
+    pdl_start();
     int2 tile;
     if (P.inc.rtiles && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) P.inc.rtiles[0] = 0;
     if (!block_tile(P.inc.tiles, &tile)) return;
@@ -1348,6 +1350,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, ResidShape<LPP, HW>::kBlocks
     Tile& T = *reinterpret_cast<Tile*>(dyn);
     Shared& E = *reinterpret_cast<Shared*>(dyn + (sizeof(Tile) + 127) / 128 * 128);
     constexpr int TW = Tile::TW, N = Tile::N;
+    pdl_start();
     int2 tile;
     if (!block_tile(P.inc.fill ? nullptr : P.inc.rtiles, &tile)) return;
     const int tid = threadIdx.x + threadIdx.y * kTileW, warp = tid / 32, lane = tid % 32;
@@ -1523,8 +1526,7 @@ static cudaError_t launch_propagate_t(const Params& P, const TileMaps& M, PatchP
     const cudaError_t e = allow_smem(kt_propagate<R, TM, HW, CPL, H>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
-    kt_propagate<R, TM, HW, CPL, H><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, work, jump);
-    return cudaGetLastError();
+    return pt::launch_dependent(kt_propagate<R, TM, HW, CPL, H>, g, dim3(kTileW, NT / kTileW), smem, s, P, M, work, jump);
 }
 
 template <int R, int TM, int HW, int LPP, int H>
@@ -1537,8 +1539,7 @@ static cudaError_t launch_scatter_t(const Params& P, const TileMaps& M, PatchPla
     const cudaError_t e = allow_smem(kt_scatter<R, TM, HW, LPP, H>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
-    kt_scatter<R, TM, HW, LPP, H><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, work, write_all, pass_id);
-    return cudaGetLastError();
+    return pt::launch_dependent(kt_scatter<R, TM, HW, LPP, H>, g, dim3(kTileW, NT / kTileW), smem, s, P, M, work, write_all, pass_id);
 }
 
 template <int R, int TM, int HW, int LPP, int H, bool KEEP>
@@ -1549,8 +1550,7 @@ static cudaError_t launch_residual_t(const Params& P, const TileMaps& M, float* 
     const cudaError_t e = allow_smem(kt_residual<R, TM, HW, LPP, H, KEEP>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
-    kt_residual<R, TM, HW, LPP, H, KEEP><<<g, dim3(kTileW, NT / kTileW), smem, s>>>(P, M, out);
-    return cudaGetLastError();
+    return pt::launch_dependent(kt_residual<R, TM, HW, LPP, H, KEEP>, g, dim3(kTileW, NT / kTileW), smem, s, P, M, out);
 }
 
 template <int R>

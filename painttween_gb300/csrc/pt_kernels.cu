@@ -177,6 +177,7 @@ __global__ void k_interleave_texels(const float4* base, const float4* out, const
 
 // offsetsToOutput, :263-274
 __global__ void k_canvas(const Params P, float4* canvas) {
+    pdl_start();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     const size_t k = (size_t)y * P.W + x;
     bool changed = in_rect(P, x, y);
@@ -524,8 +525,7 @@ cudaError_t launch_residual(const Params& P, float* out, cudaStream_t s) {
     LAUNCH_CHECK();
 }
 cudaError_t launch_canvas(const Params& P, float4* canvas, cudaStream_t s) {
-    k_canvas<<<grid2(P.lw, P.lh, kPix), kPix, 0, s>>>(P, canvas);
-    LAUNCH_CHECK();
+    return launch_dependent(k_canvas, grid2(P.lw, P.lh, kPix), kPix, 0, s, P, canvas);
 }
 cudaError_t launch_active_tiles(const Params& P, int tile_h, int* list, cudaStream_t s) {
     const cudaError_t e = cudaMemsetAsync(list, 0, sizeof(int), s);
