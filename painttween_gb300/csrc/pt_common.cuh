@@ -212,9 +212,33 @@ static __device__ float coherence_term(const Params& P, int x, int y, int i, int
 
 static __device__ __forceinline__ int f2i(float v) { return (int)v; }  // cvt.rzi: saturating, NaN -> 0
 
-// calculateResidual, :537-659; +inf once the sum reaches `limit` (energy_limit)
+// The kernels that evaluate patch distances by energy() run kCoop lanes a
+// pixel: a lane takes every kCoop-th tap, and the group then adds the values in
+// the reference's order.  All else of a pixel is the same in its lanes; the
+// first writes.  Before, a lane a pixel walked its window tap by tap, each
+// waiting for its fetches.  Measured, whole clips: three 240x180 frames with
+// passes between both neighbours 84 -> 70 ms, four 160x120 keyframe frames 74 ->
+// 49 ms; with eight lanes 72 and 51 ms, with sixteen 78 and 65 ms.
+constexpr int kCoop = 4;
+constexpr int kCoopThreads = 256, kCoopW = 8, kCoopH = kCoopThreads / kCoop / kCoopW;  // pixels of a block
+// Keyframe propagate's: a group for each of the four directions, whose
+// candidates do not depend on one another; the first with the lowest energy is
+// the one that going through them in order takes (keyframe clip 49 -> 41 ms;
+// without keys, a candidate a direction and repeats among them, it measured
+// 2 % slower than one group).
+constexpr int kDirLanes = 4 * kCoop, kDirW = 4, kDirH = kCoopThreads / kDirLanes / kDirW;
+#define COOP_PIXEL_XY(LANES, PW, PH)                                                         \
+    const int coop_px = threadIdx.x / (LANES);                                               \
+    const bool head = threadIdx.x % (LANES) == 0;                                            \
+    const int x = blockIdx.x * (PW) + coop_px % (PW), y = blockIdx.y * (PH) + coop_px / (PW); \
+    if (!in_rect(P, x, y)) return;                                                           \
+    const size_t k = (size_t)y * P.W + x;
+
+// calculateResidual, :537-659, by the kCoop lanes of the pixel together; +inf
+// once the sum reaches `limit` (energy_limit)
 static __device__ float energy(const Params& P, int x, int y, const Patch& t, const PixCtx& pc, float limit) {
-    const int r = P.r;
+    const int r = P.r, l = threadIdx.x % kCoop;
+    const unsigned group = ((1u << kCoop) - 1u) << (threadIdx.x % 32 / kCoop * kCoop);
     float sum = 0.0f;
     if (pc.validF) sum = sum - pc.hyst;
     float2 b0, b1;
@@ -222,9 +246,13 @@ static __device__ float energy(const Params& P, int x, int y, const Patch& t, co
     const float hw = (float)P.histW, hh = (float)P.histH;
     const float4* imgb = P.img.base[P.img.cur].p;
     const int imgw = P.img.base[P.img.cur].w;
-    for (int i = -r; i <= r; i++) {
-        for (int j = -r; j <= r; j++) {
-            if (!in_rect(P, x + i, y + j)) continue;
+    const int i0 = max(-r, -x), i1 = min(r, P.lw - 1 - x), j0 = max(-r, -y), j1 = min(r, P.lh - 1 - y);
+    const int rows = j1 - j0 + 1, taps = (i1 - i0 + 1) * rows;
+    int i = i0 + l / rows, j = j0 + l % rows;  // the lane's tap, column by column
+#pragma unroll 1
+    for (int t0 = 0; t0 < taps; t0 += kCoop) {
+        float res = 0.0f, w = 0.0f;
+        if (t0 + l < taps) {
             size_t k = (size_t)(y + j) * P.W + (x + i);
             float4 base = lin_texel_of(__ldg(imgb + (size_t)(y + j) * imgw + (x + i)), P.hwFilter);
             float4 canvas = __ldg(P.canvas + k);
@@ -242,7 +270,7 @@ static __device__ float energy(const Params& P, int x, int y, const Patch& t, co
                 tb = rgb_to_lab(tb);
                 to = rgb_to_lab(to);
             }
-            float res = ssd_a(base, tb, P.alphaWeight) * P.inputAnalogyWeight;
+            res = ssd_a(base, tb, P.alphaWeight) * P.inputAnalogyWeight;
             if (pc.temporalF && __ldg(&P.adv[0].off.B[k].x) > 0)
                 res = res + time_derivative(P, 0, pc.prevF, pc.fb0, pc.fb1, base, tb, canvas, to, k, i, j);
             if (pc.temporalB && __ldg(&P.adv[1].off.B[k].x) > 0)
@@ -275,10 +303,19 @@ static __device__ float energy(const Params& P, int x, int y, const Patch& t, co
                     res = fmaf(c, P.coherenceWeight, res);
                 }
             }
-            float w = P.gauss[i + r] * P.gauss[j + r];
-            sum = fmaf(res, w, sum);
-            if (sum >= limit) return INFINITY;
+            w = P.gauss[i + r] * P.gauss[j + r];
+            j += kCoop;
+            while (j > j1) {
+                j -= rows;
+                i++;
+            }
         }
+#pragma unroll
+        for (int s = 0; s < kCoop; s++) {
+            const float v = __shfl_sync(group, res, s, kCoop), g = __shfl_sync(group, w, s, kCoop);
+            sum = t0 + s < taps ? fmaf(v, g, sum) : sum;
+        }
+        if (sum >= limit) return INFINITY;
     }
     if (pc.sumW < kEpsilon) return kBigResidual;
     return sum / pc.sumW;
@@ -329,7 +366,7 @@ static __device__ float test_offset(const Params& P, int x, int y, const Patch& 
             float ea = ex_sample_out_alpha(P.ex, t.x, t.y, t.layer);
             if (ea < kAlphaThreshold && image_alpha > kAlphaThreshold) return kBigResidual;
         }
-        if (P.counters) count_eval(P, x, y, pc.temporalF || pc.temporalB);
+        if (P.counters && threadIdx.x % kCoop == 0) count_eval(P, x, y, pc.temporalF || pc.temporalB);
         return energy(P, x, y, t, pc, energy_limit(P, pc, best));
     }
     return kBigResidual;
@@ -345,6 +382,16 @@ static __device__ __forceinline__ size_t pixel_wrap_index(const Params& P, int t
     int wy = (int)((float)ty - (float)P.H * floorf((float)ty / (float)P.H));
     return (size_t)wy * P.W + wx;
 }
+// the four propagate sources of pixel (x, y), in the reference's order
+static __device__ __forceinline__ void propagate_source(int cdx, int x, int y, int jump, int* tx, int* ty) {
+    *tx = x;
+    *ty = y;
+    if (cdx == 0) *tx = x + jump;
+    else if (cdx == 1) *tx = x - jump;
+    else if (cdx == 2) *ty = y + jump;
+    else *ty = y - jump;
+}
+
 static __device__ Patch propagate_offset(const Params& P, int tx, int ty, int x, int y) {
     size_t kk = pixel_wrap_index(P, tx, ty);
     float4 a = __ldg(P.off.A + kk);

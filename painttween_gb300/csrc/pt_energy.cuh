@@ -349,16 +349,6 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
     return in;
 }
 
-// the four propagate sources of pixel (x, y), in the reference's order
-__device__ __forceinline__ void propagate_source(int cdx, int x, int y, int jump, int* tx, int* ty) {
-    *tx = x;
-    *ty = y;
-    if (cdx == 0) *tx = x + jump;
-    else if (cdx == 1) *tx = x - jump;
-    else if (cdx == 2) *ty = y + jump;
-    else *ty = y - jump;
-}
-
 // A block whose pixels need no energy (change tracking skipped all their
 // candidates) copies its records and stops before staging its tile.
 // (write: the working buffer needs every record written)

@@ -26,14 +26,14 @@ namespace ptk {
 
 // propagate_kernel, :1112-1219 (advected candidates are dead code, :981)
 // With key >= 0, a pixel under the key's mask takes the key (:1137-1142).
-__global__ void __launch_bounds__(128) k_propagate(const Params P, PatchPlanes work, int jump, int key) {
-    PIXEL_XY
+__global__ void __launch_bounds__(kCoopThreads) k_propagate(const Params P, PatchPlanes work, int jump, int key) {
+    COOP_PIXEL_XY(kCoop, kCoopW, kCoopH)
     if (image_culled(P, x, y)) {
-        store_patch(work, k, make_patch(0, 0, 0, 0, 0, 1.f, 1.f));
+        if (head) store_patch(work, k, make_patch(0, 0, 0, 0, 0, 1.f, 1.f));
         return;
     }
     if (keymask_alpha(P.ex, x, y, key) > 0.0f) {
-        store_patch(work, k, make_patch((float)x, (float)y, 0.f, 1.f, key, 1.f, 1.f));
+        if (head) store_patch(work, k, make_patch((float)x, (float)y, 0.f, 1.f, key, 1.f, 1.f));
         return;
     }
     float best = __ldg(P.res + k);
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(128) k_propagate(const Params P, PatchPlanes w
         float r = test_offset(P, x, y, t, ia, pc, best);
         if (r < best) { ow = t; best = r; }
     }
-    store_patch(work, k, ow);
+    if (head) store_patch(work, k, ow);
 }
 
 // scatter_kernel + averageOffset, :841-952.  REFERENCE mode: randFloat()
@@ -73,12 +73,12 @@ __global__ void __launch_bounds__(128) k_propagate(const Params P, PatchPlanes w
 // and [0, 2pi) from a counter-based hash.  write_all: the working buffer
 // aliases base, so unchanged pixels are written too.
 // With key >= 0, a pixel under the key's mask keeps its offset (:887-892).
-__global__ void __launch_bounds__(128) k_scatter(const Params P, PatchPlanes work, int write_all, uint32_t pass_id,
+__global__ void __launch_bounds__(kCoopThreads) k_scatter(const Params P, PatchPlanes work, int write_all, uint32_t pass_id,
                                                  int key) {
-    PIXEL_XY
+    COOP_PIXEL_XY(kCoop, kCoopW, kCoopH)
     Patch off = load_patch(P.off, k);
     if (image_culled(P, x, y) || keymask_alpha(P.ex, x, y, key) > 0.0f) {
-        if (write_all || !image_culled(P, x, y)) store_patch(work, k, off);
+        if (head && (write_all || !image_culled(P, x, y))) store_patch(work, k, off);
         return;
     }
     float cached = __ldg(P.res + k);
@@ -136,19 +136,24 @@ __global__ void __launch_bounds__(128) k_scatter(const Params P, PatchPlanes wor
     avg.theta = screen_to_exemplar_angle(P, x, y, avg.x, avg.y, 0);
     float r = test_offset(P, x, y, avg, ia, pc, best);
     if (r < best) { ow = avg; best = r; }
+    if (!head) return;
     if (best < cached) store_patch(work, k, ow);
     else if (write_all) store_patch(work, k, off);
 }
 
 // updateResidualCache_kernel, :661-693
-__global__ void __launch_bounds__(128) k_residual(const Params P, float* out) {
-    PIXEL_XY
-    if (image_culled(P, x, y)) { out[k] = 0.0f; return; }
+__global__ void __launch_bounds__(kCoopThreads) k_residual(const Params P, float* out) {
+    COOP_PIXEL_XY(kCoop, kCoopW, kCoopH)
+    if (image_culled(P, x, y)) {
+        if (head) out[k] = 0.0f;
+        return;
+    }
     PixCtx pc;
     make_pixctx(P, x, y, &pc);
     Patch t = load_patch(P.off, k);
-    if (P.counters) count_eval(P, x, y, pc.temporalF || pc.temporalB);
-    out[k] = energy(P, x, y, t, pc, __int_as_float(0x7fc00000));
+    if (P.counters && head) count_eval(P, x, y, pc.temporalF || pc.temporalB);
+    const float e = energy(P, x, y, t, pc, __int_as_float(0x7fc00000));
+    if (head) out[k] = e;
 }
 
 // base and output exemplar texels interleaved into 32-byte records (the
@@ -507,21 +512,22 @@ using namespace ptk;
 
 static inline dim3 grid2(int w, int h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h + b.y - 1) / b.y); }
 static const dim3 kPix(32, 4);
+static const dim3 kCoopPix(kCoopW, kCoopH);
 static_assert(kResidH == 4 && kTileW == 32, "the canvas kernel gathers the residual's tiles, its own blocks");
 
 #define LAUNCH_CHECK() return cudaGetLastError()
 
 cudaError_t launch_propagate(const Params& P, PatchPlanes work, int jump, int key, cudaStream_t s) {
-    k_propagate<<<grid2(P.lw, P.lh, kPix), kPix, 0, s>>>(P, work, jump, key);
+    k_propagate<<<grid2(P.lw, P.lh, kCoopPix), kCoopThreads, 0, s>>>(P, work, jump, key);
     LAUNCH_CHECK();
 }
 cudaError_t launch_scatter(const Params& P, PatchPlanes work, int write_all, uint32_t pass_id, int key,
                            cudaStream_t s) {
-    k_scatter<<<grid2(P.lw, P.lh, kPix), kPix, 0, s>>>(P, work, write_all, pass_id, key);
+    k_scatter<<<grid2(P.lw, P.lh, kCoopPix), kCoopThreads, 0, s>>>(P, work, write_all, pass_id, key);
     LAUNCH_CHECK();
 }
 cudaError_t launch_residual(const Params& P, float* out, cudaStream_t s) {
-    k_residual<<<grid2(P.lw, P.lh, kPix), kPix, 0, s>>>(P, out);
+    k_residual<<<grid2(P.lw, P.lh, kCoopPix), kCoopThreads, 0, s>>>(P, out);
     LAUNCH_CHECK();
 }
 cudaError_t launch_canvas(const Params& P, float4* canvas, cudaStream_t s) {

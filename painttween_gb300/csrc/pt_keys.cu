@@ -14,6 +14,7 @@ constexpr int kKeyPix = 128;
 constexpr float kEpsilon = 0.000001f;  // EPSILON, types.h:38
 
 dim3 grid_of(int w, int h) { return dim3((w + 31) / 32, (h + 3) / 4); }
+dim3 coop_grid(int w, int h) { return dim3((w + kCoopW - 1) / kCoopW, (h + kCoopH - 1) / kCoopH); }
 
 #define KEY_PIXEL_XY                                    \
     const int x = blockIdx.x * blockDim.x + threadIdx.x; \
@@ -74,53 +75,65 @@ __device__ void ribbon_candidates(const Params& P, const KeyView& K, int x, int 
 }
 
 // propagate_kernel_keys, :984-1110
-__global__ void __launch_bounds__(kKeyPix) k_propagate_keys(const Params P, PatchPlanes work, int jump, int key,
+__global__ void __launch_bounds__(kCoopThreads) k_propagate_keys(const Params P, PatchPlanes work, int jump, int key,
                                                             const KeyView K) {
-    KEY_PIXEL_XY
+    COOP_PIXEL_XY(kDirLanes, kDirW, kDirH)
     if (image_culled(P, x, y)) {
-        store_patch(work, k, make_patch(0, 0, 0, 0, 0, 1.f, 1.f));
+        if (head) store_patch(work, k, make_patch(0, 0, 0, 0, 0, 1.f, 1.f));
         return;
     }
     if (keymask_alpha(P.ex, x, y, key) > 0.0f) {
-        store_patch(work, k, make_patch((float)x, (float)y, 0.f, 1.f, key, 1.f, 1.f));
+        if (head) store_patch(work, k, make_patch((float)x, (float)y, 0.f, 1.f, key, 1.f, 1.f));
         return;
     }
     float best = __ldg(P.res + k);
     const float ia = lay_texel(P.img.base[P.img.cur], P, x, y).w;
-    Patch ow = load_patch(P.off, k);
     PixCtx pc;
     make_pixctx(P, x, y, &pc);
-#pragma unroll 1
-    for (int c = 0; c < 4; c++) {
-        int tx = x, ty = y;
-        if (c == 0) tx = x + jump;
-        else if (c == 1) tx = x - jump;
-        else if (c == 2) ty = y + jump;
-        else ty = y - jump;
-        Patch t = propagate_offset(P, tx, ty, x, y);
-        float r = test_offset(P, x, y, t, ia, pc, best);
-        if (r < best) {
-            ow = t;
-            best = r;
-        }
-        ribbon_candidates<true>(P, K, x, y, t.x, t.y, t.layer, ia, pc, &ow, &best);
+    int tx, ty;
+    propagate_source(threadIdx.x % kDirLanes / kCoop, x, y, jump, &tx, &ty);
+    const Patch t = propagate_offset(P, tx, ty, x, y);
+    Patch mine = t;
+    float r = best;  // the direction's lowest energy, if below the best
+    {
+        const float e = test_offset(P, x, y, t, ia, pc, best);
+        if (e < r) r = e;
     }
-    store_patch(work, k, ow);
+    ribbon_candidates<true>(P, K, x, y, t.x, t.y, t.layer, ia, pc, &mine, &r);
+    const unsigned lanes = ((1u << kDirLanes) - 1u) << (threadIdx.x % 32 / kDirLanes * kDirLanes);
+    int win = -1;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const float rc = __shfl_sync(lanes, r, c * kCoop, kDirLanes);
+        if (rc < best) { win = c; best = rc; }
+    }
+    const int src = (win < 0 ? 0 : win) * kCoop;
+    Patch ow;
+    ow.x = __shfl_sync(lanes, mine.x, src, kDirLanes);
+    ow.y = __shfl_sync(lanes, mine.y, src, kDirLanes);
+    ow.theta = __shfl_sync(lanes, mine.theta, src, kDirLanes);
+    ow.hyst = __shfl_sync(lanes, mine.hyst, src, kDirLanes);
+    ow.layer = __shfl_sync(lanes, mine.layer, src, kDirLanes);
+    ow.su = __shfl_sync(lanes, mine.su, src, kDirLanes);
+    ow.sv = __shfl_sync(lanes, mine.sv, src, kDirLanes);
+    ow.lumy = __shfl_sync(lanes, mine.lumy, src, kDirLanes);
+    ow.luma = __shfl_sync(lanes, mine.luma, src, kDirLanes);
+    if (head) store_patch(work, k, win >= 0 ? ow : load_patch(P.off, k));
 }
 
 // scatter_kernel_keys, :723-839.  randFloat() returns 0 (texSynth_util.h:
 // 155-163): candidate i is (best.x + 0.9*dist_i, best.y) in the best
 // offset's layer, sampleCount / (lastKey - firstKey + 1) of them.
-__global__ void __launch_bounds__(kKeyPix) k_scatter_keys(const Params P, PatchPlanes work, int write_all, int key,
+__global__ void __launch_bounds__(kCoopThreads) k_scatter_keys(const Params P, PatchPlanes work, int write_all, int key,
                                                           const KeyView K) {
-    KEY_PIXEL_XY
+    COOP_PIXEL_XY(kCoop, kCoopW, kCoopH)
     const Patch off = load_patch(P.off, k);
     if (image_culled(P, x, y)) {
-        if (write_all) store_patch(work, k, off);
+        if (write_all && head) store_patch(work, k, off);
         return;
     }
     if (keymask_alpha(P.ex, x, y, key) > 0.0f) {
-        store_patch(work, k, off);
+        if (head) store_patch(work, k, off);
         return;
     }
     const float cached = __ldg(P.res + k);
@@ -148,6 +161,7 @@ __global__ void __launch_bounds__(kKeyPix) k_scatter_keys(const Params P, PatchP
         ribbon_candidates<false>(P, K, x, y, ex, ey, elayer, ia, pc, &ow, &best);
         dist *= factor;
     }
+    if (!head) return;
     if (best < cached) store_patch(work, k, ow);
     else if (write_all) store_patch(work, k, off);
 }
@@ -325,12 +339,12 @@ namespace pt {
 
 cudaError_t launch_propagate_keys(const Params& P, PatchPlanes work, int jump, int key, const KeyView& K,
                                   cudaStream_t s) {
-    ptk::k_propagate_keys<<<ptk::grid_of(P.lw, P.lh), dim3(32, 4), 0, s>>>(P, work, jump, key, K);
+    ptk::k_propagate_keys<<<dim3((P.lw + ptk::kDirW - 1) / ptk::kDirW, (P.lh + ptk::kDirH - 1) / ptk::kDirH), ptk::kCoopThreads, 0, s>>>(P, work, jump, key, K);
     KEY_LAUNCH_CHECK();
 }
 cudaError_t launch_scatter_keys(const Params& P, PatchPlanes work, int write_all, int key, const KeyView& K,
                                 cudaStream_t s) {
-    ptk::k_scatter_keys<<<ptk::grid_of(P.lw, P.lh), dim3(32, 4), 0, s>>>(P, work, write_all, key, K);
+    ptk::k_scatter_keys<<<ptk::coop_grid(P.lw, P.lh), ptk::kCoopThreads, 0, s>>>(P, work, write_all, key, K);
     KEY_LAUNCH_CHECK();
 }
 cudaError_t launch_accumulate_ribbon(const Params& P, int forwards, Ribbon* dest, const Ribbon* src, int time_step,
