@@ -244,6 +244,7 @@ struct pt_ctx {
     int* tile_mark = nullptr;
     int inc_tiles = 0;      // 0: none, 1: the residual's, 2: all
     int inc_kind = 0;       // the pass runs propagate (0) or scatter (1)
+    int inc_canvas = 0;     // the residual kernel writes the canvas
     int inc_fill = 0;       // the next residual computes and stores every tap value
     float* tap_cache = nullptr;  // per-tap residual values, (2r+1)^2 planes
     int tap_cache_k = 0;         // planes allocated

@@ -456,6 +456,13 @@ __device__ __forceinline__ float4 ex_sample_out(const ExView& e, float u, float 
     return bl4(b, __ldg(e.out + r0 + b.x0), __ldg(e.out + r0 + b.x1), __ldg(e.out + r1 + b.x0),
                __ldg(e.out + r1 + b.x1));
 }
+// offsetsToOutput, texSynth_kernel.cu:263-274, of record k
+__device__ __forceinline__ float4 canvas_of(const Params& P, size_t k) {
+    const float4 a = __ldg(P.off.A + k);
+    const float lumy = __ldg(&P.off.B[k].w), luma = __ldg(P.off.C + k);
+    const float4 c = ex_sample_out(P.ex, a.x, a.y, __float_as_int(a.w));
+    return f4(c.x + lumy, c.y + lumy, c.z + lumy, c.w + luma);
+}
 __device__ __forceinline__ float ex_sample_out_alpha(const ExView& e, float u, float v, int layer) {
     if (e.hw && e.tout) return ex_tex(e.tout, e, u, v, layer).w;
     Bl b = bl_setup(u, v, e.w, e.h, e.hw);

@@ -231,7 +231,8 @@ __device__ __forceinline__ bool block_tile(const int* list, int2* tile) {
     return i < n;
 }
 
-// Stages the tile (and halo) of the pixel-side inputs and fills the
+// Stages the tile (and halo) of the pixel-side inputs (`changed`: the records
+// whose canvas is formed here, a bit each by row; plain loads only) and fills the
 // state of pixel `pid` of the tile (several threads of a block of NT >
 // kTileThreads threads may ask for the same pixel).  Returns false for
 // threads whose pixel is outside the level rectangle.  A tile whose halo lies inside the level rectangle, where
@@ -242,7 +243,8 @@ __device__ __forceinline__ bool block_tile(const int* list, int2* tile) {
 // not complete within two bounded waits; the block must then return.
 template <int R, int TM, int NT = kTileThreads, int H = kTileH>
 __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, TileSmem<R, TM, H>& T, int2 tile,
-                                           int pid, PixT* px, bool* abort) {
+                                           int pid, PixT* px, bool* abort,
+                                           const unsigned long long* changed = nullptr) {
     constexpr int TW = TileSmem<R, TM, H>::TW, TH = TileSmem<R, TM, H>::TH, N = TileSmem<R, TM, H>::N;
     const int tid = threadIdx.x + threadIdx.y * kTileW;
     const int lx = pid % kTileW, ly = pid / kTileW;
@@ -274,7 +276,17 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
             int gy = clampi(y0 + q / TW, 0, P.lh - 1);
             size_t k = (size_t)gy * P.W + gx;
             T.base[q] = lin_texel_of(__ldg(ib.p + (size_t)gy * ib.w + gx), P.hwFilter);
-            T.canvas[q] = __ldg(P.canvas + k);
+            if (changed && ((changed[q / TW] >> (q % TW)) & 1)) {
+                // formed here, and written where the record is of this tile;
+                // no block of the launch reads the old value
+                const float4 cv = canvas_of(P, k);
+                const int lx = q % TW - R, ly = q / TW - R;
+                T.canvas[q] = cv;
+                if (lx >= 0 && ly >= 0 && lx < kTileW && ly < H && tile.x * kTileW + lx < P.lw && tile.y * H + ly < P.lh)
+                    const_cast<float4*>(P.canvas)[k] = cv;
+            } else {
+                T.canvas[q] = P.canvas[k];
+            }
             if (TM) {
                 const AdvView& A = P.adv[TM == TM_FWD ? 0 : 1];
                 T.pbase[q] = __ldg(A.base + k);
@@ -1378,7 +1390,8 @@ __global__ void __launch_bounds__(kTileW * H * LPP, ResidShape<LPP, HW>::kBlocks
     }
     PixT px;
     bool abort;
-    stage_tile<R, TM, NT, H>(P, M, T, tile, pid, &px, &abort);  // (synchronises the block)
+    // (synchronises the block)
+    stage_tile<R, TM, NT, H>(P, M, T, tile, pid, &px, &abort, !dense && P.inc.canvas ? E.chg : nullptr);
     if (abort) return;
     bool mine = false;
     LanePix q;

@@ -202,10 +202,7 @@ __global__ void k_canvas(const Params P, float4* canvas) {
         }
     }
     if (!changed) return;
-    float4 a = __ldg(P.off.A + k);
-    float lumy = __ldg(&P.off.B[k].w), luma = __ldg(P.off.C + k);
-    float4 c = ex_sample_out(P.ex, a.x, a.y, __float_as_int(a.w));
-    canvas[k] = f4(c.x + lumy, c.y + lumy, c.z + lumy, c.w + luma);
+    canvas[k] = canvas_of(P, k);
 }
 
 // copyRandomKernel, :2044-2059

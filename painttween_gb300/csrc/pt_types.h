@@ -127,6 +127,7 @@ struct IncView {
     const int* tiles;
     int* rtiles;
     int* rmark;
+    int canvas;  // the residual kernel of this pass also writes the canvas of the changed records
 };
 
 struct Params {
