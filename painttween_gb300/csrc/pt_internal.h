@@ -89,6 +89,8 @@ cudaError_t launch_merge_random(const Params& P, int d, int forwards, float weig
 cudaError_t launch_merge_residual(const Params& P, int d, PatchPlanes work, cudaStream_t s);
 cudaError_t launch_conv(const float* src, float* dst, int w, int h, int pitch, int rows, const ConvKernel& kw,
                         cudaStream_t s);
+// both passes of the separable Gaussian at once (src and dst do not overlap)
+cudaError_t launch_blur(const float* src, float* dst, int w, int h, int pitch, const ConvKernel& kw, cudaStream_t s);
 cudaError_t launch_copy_patch(const Params& P, PatchPlanes dst, PatchPlanes src, cudaStream_t s);
 cudaError_t launch_copy_float(const Params& P, float* dst, const float* src, cudaStream_t s);
 cudaError_t launch_unpack_patch(const Params& P, const pt_patchxf* src, PatchPlanes dst, cudaStream_t s);

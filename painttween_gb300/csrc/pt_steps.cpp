@@ -420,16 +420,22 @@ pt_status pt_convolve_separable(pt_ctx* c, const float* src, float* dst, int w, 
     if (w < 1 || h < 1 || pitch < w || radius < 1 || radius > ptk::kMaxRadius)
         return fail(c, PT_ERR_INVALID, "bad convolution size %dx%d pitch %d radius %d", w, h, pitch, radius);
     CU(cudaSetDevice(c->device));
+    ConvKernel k;
+    k.r = radius;
+    pt::gaussian_weights(radius, true, k.w);
     size_t n = (size_t)pitch * h;
+    // in place (or over each other) the row pass has to be complete first
+    const uintptr_t a = (uintptr_t)src, b = (uintptr_t)dst, bytes = n * sizeof(float);
+    if ((a + bytes <= b || b + bytes <= a) && h <= 262140) {
+        LN(pt::launch_blur(src, dst, w, h, pitch, k, c->stream));
+        return PT_OK;
+    }
     if (n > c->conv_scratch_elems) {
         dfree_t(c, c->conv_scratch);
         c->conv_scratch_elems = 0;
         TRY(dalloc_t(c, &c->conv_scratch, n));
         c->conv_scratch_elems = n;
     }
-    ConvKernel k;
-    k.r = radius;
-    pt::gaussian_weights(radius, true, k.w);
     LN(pt::launch_conv(src, c->conv_scratch, w, h, pitch, 1, k, c->stream));
     LN(pt::launch_conv(c->conv_scratch, dst, w, h, pitch, 0, k, c->stream));
     return PT_OK;
