@@ -64,10 +64,12 @@ pt_status pt_set_style(pt_ctx* c, int style, int w, int h, const float* base, co
     if ((int)c->style_levels.size() != nlev || c->style_levels[0].w != w || c->style_levels[0].h != h) {
         for (auto& L : c->style_levels) {
             dfree_t(c, L.base); dfree_t(c, L.out); dfree_t(c, L.bo); dfree_t(c, L.orient); dfree_t(c, L.dt);
-            dfree_t(c, L.ids); dfree_t(c, L.flags);
+            dfree_t(c, L.ids);
             free_textures(c, &L);
         }
+        if (!c->style_levels.empty()) dfree_t(c, c->style_levels[0].flags);  // (one block for all levels)
         c->style_levels.assign(nlev, ExLevel());
+        TRY(dalloc_t(c, &c->style_levels[0].flags, (size_t)2 * nlev));
         for (int l = 0; l < nlev; l++) {
             ExLevel& L = c->style_levels[l];
             L.w = w >> l;
@@ -79,7 +81,7 @@ pt_status pt_set_style(pt_ctx* c, int style, int w, int h, const float* base, co
             TRY(dalloc_t(c, &L.orient, n));
             TRY(dalloc_t(c, &L.dt, n));
             TRY(dalloc_t(c, &L.ids, n));
-            TRY(dalloc_t(c, &L.flags, (size_t)2));
+            L.flags = c->style_levels[0].flags + 2 * l;
         }
         c->style_set.assign(c->NS, 0);
     }
