@@ -179,7 +179,8 @@ static pt_status propagate_and_scatter(pt_ctx* c, int level, int iterations, boo
         }
     }
     // Levels with more tiles than the GPU holds at once (those of the
-    // residual's narrow shape, more than 8 tiles an SM) list those that have work: a block of an idle tile ends after its checks, but keeps its place
+    // residual's narrow shape, more than 8 tiles an SM) list those that have
+    // work: a block of an idle tile ends after its checks, but keeps its place
     // from another for the time of two or three loads.  Four fifths of a 1080p
     // frame's tiles are culled: propagate 162 -> 149 ms, scatter 49.6 -> 48.1
     // ms over two such frames, propagate of a 1024x1024 still 11.3 -> 10.4 ms;
@@ -188,13 +189,13 @@ static pt_status propagate_and_scatter(pt_ctx* c, int level, int iterations, boo
     int passes = 0;
     if (track) {
         Params P = make_params(c, level);
-        lists = P.lw < 65536 * ptk::kTileW && P.lh < 65536 && !resid_wide(c, P);  // (the list's tiles are the narrow shape's)
+        // (the list's tiles are the narrow shape's)
+        lists = P.lw < 65536 * ptk::kTileW && P.lh < 65536 && !resid_wide(c, P);
         if (lists) {
-            if (!c->tile_mark) {
-                const size_t n = (size_t)((c->W + ptk::kTileW - 1) / ptk::kTileW) * ((c->H + 1) / 2);
-                for (auto& t : c->tile_list) TRY(dalloc_t(c, &t, n + 1));
-                TRY(dalloc_t(c, &c->tile_mark, n));
-            }
+            const size_t n = (size_t)((c->W + ptk::kTileW - 1) / ptk::kTileW) * ((c->H + 1) / 2);
+            for (auto& t : c->tile_list)
+                if (!t) TRY(dalloc_t(c, &t, n + 1));
+            if (!c->tile_mark) TRY(dalloc_t(c, &c->tile_mark, n));
             LN(pt::launch_active_tiles(P, ptk::kPropH, c->tile_list[0], c->stream));
             LN(pt::launch_active_tiles(P, scatter_wide(c, P) ? ptk::kScatHWide : ptk::kScatH, c->tile_list[1], c->stream));
         }
