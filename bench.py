@@ -44,7 +44,7 @@ WORKLOAD = "clip1080p"
 METRIC = "1080p stylized frames/s"
 UNIT = "frames/s"
 
-# DRAM bytes (read + write) per level pixel of one kt_propagate_q launch: the
+# DRAM bytes (read + write) per level pixel of one propagate launch: the
 # ncu capture of a level-0 temporal launch of this workload (1920x1080 level,
 # 340.1 MB read + 64.9 MB written) summarised in
 # profiles/kt_energy_kernels_clip1080p.md.  The exemplar planes stay in L2,
@@ -759,7 +759,7 @@ def main():
     ap.add_argument("--staging", default="tma", choices=["tma", "loads"],
                     help="how the tiled kernels stage interior tiles: tensor copies or plain loads (same results)")
     ap.add_argument("--propagate-lanes", type=int, default=0, choices=[0, 1, 2],
-                    help="propagate's warps per tile row: 0 = autotuned per launch shape (same results)")
+                    help="propagate's lanes per pixel: 1 = two, 2 = four, 0 = autotuned per launch shape (same results)")
     ap.add_argument("--generic-kernels", action="store_true",
                     help="run the generic one-thread-per-pixel kernels instead of the tiled ones (profiling only)")
     args = ap.parse_args()

@@ -552,11 +552,12 @@ static void tile_maps(pt_ctx* c, const Params& P, int tm, int tile_h, TileMaps* 
     M->on = ok ? 1 : 0;
 }
 
-// Propagate's warps per tile row for this launch (0: one, 1: two) and the
+// Propagate's lanes per pixel for this launch (0: two, 1: four) and the
 // variant being timed (-1: none).  Launch shapes are keyed by radius,
 // temporal mode, filter mode and the tile count relative to the SM count,
 // in powers of two (up to a quarter, half, one, 2, 4, 8 SMs' worth, more):
-// the choice depends on how much of the GPU the tiles fill.  Decisions are shared by the contexts of a
+// the choice depends on how much of the GPU the tiles fill.  Decisions are
+// shared by the contexts of a
 // device; until a shape's two variants have been timed, shapes with no
 // more tiles than SMs take two warps.
 static std::mutex g_tune_mutex;

@@ -214,10 +214,10 @@ struct pt_ctx {
     bool adv_written[2] = {false, false};  // advected F/B written since the last reset
     bool use_tiled = true;                 // tiled kernels where an instantiation exists
     bool use_tma = true;                   // interior tiles staged by tensor copies
-    // propagate's warps per tile row: 0 = picked by the autotuner below, 1 or 2
+    // propagate's lanes per pixel: 0 = picked by the autotuner below, 1 = two, 2 = four
     int prop_lanes = 0;
     int sm_count = 0;
-    // autotuner of propagate's warps per tile row, per launch shape (radius,
+    // autotuner of propagate's lanes per pixel, per launch shape (radius,
     // temporal mode, filter mode, tile-count class): one launch of each
     // variant is timed with events (the results are identical), and the
     // faster one is kept, for every context of the device

@@ -5,12 +5,13 @@
 // operation, as the generic kernels in pt_kernels.cu (which restate
 // calculateResidual and its callers, src/PaintTweenCUDA/texSynth_kernel.cu:
 // 537-952), organised for sm_103a:
-//  * a block owns a 32 x 8 pixel tile; the pixel-side inputs of every tap
-//    (input colour, canvas, and for temporal passes the advected colours and
-//    validity) are staged once into shared memory with an R-pixel halo;
-//  * the (2R+1)^2 tap loop is fully unrolled and straight-line: taps outside
-//    the level rectangle are evaluated and then discarded by selects, which
-//    leaves the sums exactly as skipping them would;
+//  * a block owns a tile 32 pixels wide and two or four high; the pixel-side
+//    inputs of every tap (input colour, canvas, and for temporal passes the
+//    advected colours and validity) are staged once into shared memory with an
+//    R-pixel halo;
+//  * several lanes share a pixel: they take its candidates, or the taps of one
+//    candidate, side by side; taps outside the level rectangle count as zeros,
+//    which leaves the sums exactly as skipping them would;
 //  * an exemplar texel is 32 bytes (base RGBA, output RGBA), one sector per
 //    texel of the bilinear footprint; when a candidate's whole footprint lies inside the
 //    exemplar (decided for the whole warp), the wrap and clamp steps -- which

@@ -132,7 +132,8 @@ cudaError_t launch_interleave_texels(const float4* base, const float4* out, cons
 // kind 0 = propagate (arg = jump), 1 = scatter (arg = write_all),
 // 2 = residual (into out); tm 0 = no temporal terms, 1 = forward, 2 = backward;
 // M: the tensor maps of the staged planes (M.on = 0: staged by plain loads);
-// wide: propagate with two warps per tile row (same results)
+// wide: four lanes per pixel instead of two (propagate, scatter) or instead of
+// one or two (residual); same results
 cudaError_t launch_tiled_2(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
                            uint32_t pass_id, float* out, int wide, cudaStream_t s);
 cudaError_t launch_tiled_3(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
