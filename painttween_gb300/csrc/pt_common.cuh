@@ -394,7 +394,7 @@ static __device__ __forceinline__ void propagate_source(int cdx, int x, int y, i
 
 static __device__ Patch propagate_offset(const Params& P, int tx, int ty, int x, int y) {
     size_t kk = pixel_wrap_index(P, tx, ty);
-    float4 a = __ldg(P.off.A + kk);
+    float4 a = P.off.A[kk];
     float2 sc = lvl_texel_lin(P.img.scale, tx, ty, P.hwFilter);
     float2 b0, b1;
     basis(a.z, P.scaleWU * sc.x, P.scaleWV * sc.y, &b0, &b1);

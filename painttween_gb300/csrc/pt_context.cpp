@@ -83,6 +83,7 @@ pt_status dalloc(pt_ctx* c, void** p, size_t bytes) {
         c->allocs[*p] = bytes;
     }
     cudaError_t e = cudaMemsetAsync(*p, 0, bytes, c->stream);
+    c->chained = false;
     if (e != cudaSuccess) return fail(c, PT_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
     return PT_OK;
 }
@@ -646,7 +647,7 @@ int resid_wide(pt_ctx* c, const Params& P) {
 }
 
 cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,
-                         float* out, bool* done) {
+                         float* out, bool dependent, bool* done) {
     *done = false;
     if (!tiled_usable(c)) return cudaSuccess;
     int tm = temporal_mode(c);
@@ -662,11 +663,12 @@ cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work,
     *done = true;
     cudaError_t e;
     switch (P.r) {
-        case 2: e = pt::launch_tiled_2(kind, tm, P, M, work, arg, pass_id, out, wide, c->stream); break;
-        case 3: e = pt::launch_tiled_3(kind, tm, P, M, work, arg, pass_id, out, wide, c->stream); break;
-        default: e = pt::launch_tiled_4(kind, tm, P, M, work, arg, pass_id, out, wide, c->stream); break;
+        case 2: e = pt::launch_tiled_2(kind, tm, P, M, work, arg, pass_id, out, wide, dependent, c->stream); break;
+        case 3: e = pt::launch_tiled_3(kind, tm, P, M, work, arg, pass_id, out, wide, dependent, c->stream); break;
+        default: e = pt::launch_tiled_4(kind, tm, P, M, work, arg, pass_id, out, wide, dependent, c->stream); break;
     }
     if (t) cudaEventRecord(t->ev[2 * probe + 1], c->stream);
+    c->chained = true;
     return e;
 }
 
@@ -685,9 +687,9 @@ pt_status check_tma(pt_ctx* c) {
 pt_status do_residual(pt_ctx* c, int level) {
     Params P = make_params(c, level);
     float* out = c->res[c->res_i];
-    return profiled(c, PT_KERNEL_RESIDUAL, P, [&](const Params& Q) {
+    return profiled(c, PT_KERNEL_RESIDUAL, P, [&](const Params& Q, bool dependent) {
         bool done = false;
-        cudaError_t e = launch_tiled(c, 2, Q, PatchPlanes{}, 0, 0, out, &done);
+        cudaError_t e = launch_tiled(c, 2, Q, PatchPlanes{}, 0, 0, out, dependent, &done);
         return done ? e : pt::launch_residual(Q, out, c->stream);
     });
 }
@@ -718,7 +720,10 @@ pt_status do_sync(pt_ctx* c, int level, int flags) {
         c->inc_canvas = 0;
         return st;
     }
-    TRY(profiled(c, PT_KERNEL_CANVAS, P, [&](const Params& Q) { return pt::launch_canvas(Q, c->canvas, c->stream); }));
+    TRY(profiled(c, PT_KERNEL_CANVAS, P, [&](const Params& Q, bool dependent) {
+        c->chained = true;
+        return pt::launch_canvas(Q, c->canvas, dependent, c->stream);
+    }));
     if (!(flags & PT_DONT_UPDATE_RESIDUAL)) TRY(do_residual(c, level));
     return PT_OK;
 }

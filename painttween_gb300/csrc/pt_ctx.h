@@ -245,6 +245,12 @@ struct pt_ctx {
     int inc_tiles = 0;      // 0: none, 1: the residual's, 2: all
     int inc_kind = 0;       // the pass runs propagate (0) or scatter (1)
     int inc_canvas = 0;     // the residual kernel writes the canvas
+    // The stream's last work is a launch of a kernel that begins with
+    // pdl_start; anything else put on the stream (CU, LN, dalloc) ends the
+    // chain.  Only then is the next such kernel a dependent launch: all that
+    // the chain's kernels read and do not write themselves was complete
+    // before its first one started.
+    bool chained = false;
     int inc_fill = 0;       // the next residual computes and stores every tap value
     float* tap_cache = nullptr;  // per-tap residual values, (2r+1)^2 planes
     int tap_cache_k = 0;         // planes allocated
@@ -261,6 +267,7 @@ struct pt_ctx {
 #define CU(call)                                                                          \
     do {                                                                                  \
         cudaError_t e_ = (call);                                                          \
+        c->chained = false;                                                               \
         if (e_ != cudaSuccess)                                                            \
             return fail(c, PT_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
@@ -300,7 +307,7 @@ PT_HIDDEN void glibc_state(uint32_t seed, uint32_t out[31]);
 PT_HIDDEN const std::vector<uint32_t>& glibc_powers();
 PT_HIDDEN pt_status h2d(pt_ctx* c, void* dst, const void* src, size_t bytes);
 PT_HIDDEN cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,
-                                   float* out, bool* done);
+                                   float* out, bool dependent, bool* done);
 PT_HIDDEN Params make_params(pt_ctx* c, int level);
 PT_HIDDEN cudaEvent_t pool_event(pt_ctx* c);
 PT_HIDDEN pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<float> orient, int nk = 0,
@@ -328,17 +335,24 @@ static void dfree_t(pt_ctx* c, T*& p) {
     dfree(c, (void*)p);
     p = nullptr;
 }
+// launch(P, dependent): a launch of a kernel that begins with pdl_start sets
+// pt_ctx::chained
 template <class F>
 static pt_status profiled(pt_ctx* c, int kernel, Params& P, F&& launch) {
     if (c->profiling & PT_PROFILE_COUNTERS) P.counters = c->counters + 3 * kernel;
-    if (!(c->profiling & PT_PROFILE_TIMING)) {
-        LN(launch(P));
+    auto go = [&]() -> pt_status {
+        const bool dependent = c->chained;
+        c->chained = false;
+        const cudaError_t e = launch(P, dependent);
+        if (e != cudaSuccess) return fail(c, PT_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+        c->launches++;
         return PT_OK;
-    }
+    };
+    if (!(c->profiling & PT_PROFILE_TIMING)) return go();
     cudaEvent_t a = pool_event(c), b = pool_event(c);
     if (!a || !b) return fail(c, PT_ERR_CUDA, "cudaEventCreate failed");
     CU(cudaEventRecord(a, c->stream));
-    LN(launch(P));
+    TRY(go());
     CU(cudaEventRecord(b, c->stream));
     c->ev_pairs[kernel].push_back(std::make_pair(a, b));
     return PT_OK;

@@ -23,7 +23,12 @@ namespace ptk {
 // Programmatic dependent launch: the next kernel of the stream may take its
 // place on the GPU while this one's last blocks run (launch_dependents), and
 // waits before its first access to global memory until this one has ended and
-// its writes are visible (wait).
+// its writes are visible (wait).  What the kernels that begin with this write
+// for one another (offset records, residual, canvas, change tracking, tile
+// lists) they read with plain loads only: a read-only load (__ldg) needs data
+// that nothing writes while the kernel lives, and these are written while the
+// next kernel is already there.  All else is written before the first of a
+// chain of them starts (pt_ctx::chained), so read-only loads serve for it.
 __device__ __forceinline__ void pdl_start() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -210,12 +215,12 @@ __device__ __forceinline__ float4 f4(float x, float y, float z, float w) { retur
 // ---------------------------------------------------------------------------
 
 __device__ __forceinline__ Patch load_patch(const PatchPlanes& p, size_t k) {
-    float4 a = __ldg(p.A + k);
-    float4 b = __ldg(p.B + k);
+    float4 a = p.A[k];
+    float4 b = p.B[k];
     Patch r;
     r.x = a.x; r.y = a.y; r.theta = a.z; r.layer = __float_as_int(a.w);
     r.hyst = b.x; r.su = b.y; r.sv = b.z; r.lumy = b.w;
-    r.luma = __ldg(p.C + k);
+    r.luma = p.C[k];
     return r;
 }
 __device__ __forceinline__ void store_patch(const PatchPlanes& p, size_t k, const Patch& v) {
@@ -458,8 +463,8 @@ __device__ __forceinline__ float4 ex_sample_out(const ExView& e, float u, float 
 }
 // offsetsToOutput, texSynth_kernel.cu:263-274, of record k
 __device__ __forceinline__ float4 canvas_of(const Params& P, size_t k) {
-    const float4 a = __ldg(P.off.A + k);
-    const float lumy = __ldg(&P.off.B[k].w), luma = __ldg(P.off.C + k);
+    const float4 a = P.off.A[k];
+    const float lumy = P.off.B[k].w, luma = P.off.C[k];
     const float4 c = ex_sample_out(P.ex, a.x, a.y, __float_as_int(a.w));
     return f4(c.x + lumy, c.y + lumy, c.z + lumy, c.w + luma);
 }

@@ -227,7 +227,7 @@ __device__ __forceinline__ bool block_tile(const int* list, int2* tile) {
         return true;
     }
     const int i = blockIdx.y * gridDim.x + blockIdx.x;
-    const int n = __ldg(list), id = __ldg(list + 1 + i);  // (the list has room for every tile)
+    const int n = list[0], id = list[1 + i];  // (the list has room for every tile)
     *tile = make_int2(id & 0xffff, id >> 16);
     return i < n;
 }
@@ -893,7 +893,7 @@ __device__ __forceinline__ void propagate_candidates(const Params& P, int x, int
         propagate_source(slot0 + i, x, y, jump, &tx, &ty);
         dx[i] = (float)x - (float)tx;
         dy[i] = (float)y - (float)ty;
-        a[i] = __ldg(P.off.A + pixel_wrap_index(P, tx, ty));
+        a[i] = P.off.A[pixel_wrap_index(P, tx, ty)];
         sc[i] = lvl_texel_lin(P.img.scale, tx, ty, P.hwFilter);
     }
     float eo[CPL];
@@ -951,9 +951,9 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
             for (int i = 0; i < CPL; i++) {
                 int tx, ty;
                 propagate_source(slot0 + i, x, y, jump, &tx, &ty);
-                last[i] = __ldg(P.inc.last + pixel_wrap_index(P, tx, ty));
+                last[i] = P.inc.last[pixel_wrap_index(P, tx, ty)];
             }
-            if (__ldg(P.inc.win + k) < P.inc.prev) {
+            if (P.inc.win[k] < P.inc.prev) {
 #pragma unroll
                 for (int i = 0; i < CPL; i++)
                     if (last[i] < P.inc.prev) skip |= 1u << i;
@@ -990,7 +990,7 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
             }
         } else {
             own = true;
-            best = __ldg(P.res + k);
+            best = P.res[k];
             const float2 scale = lvl_texel_lin(P.img.scale, x, y, P.hwFilter);
             PropCand pc[CPL];
             propagate_candidates<CPL>(P, x, y, slot0, jump, scale, pc);
@@ -1098,7 +1098,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
         const int x = tile.x * kTileW + pid % kTileW, y = tile.y * H + pid / kTileW;
         const bool in = x < P.lw && y < P.lh;
         const size_t k = (size_t)y * P.W + x;
-        stable = in && P.inc.prev != INT_MIN && __ldg(P.inc.win + k) < P.inc.prev;
+        stable = in && P.inc.prev != INT_MIN && P.inc.win[k] < P.inc.prev;
         if (block_idle(P, work, in && !stable, in && head, k, write_all != 0)) return;
     }
     load_tap_list<R>(P, E.L, tid);
@@ -1122,7 +1122,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     // chain state (the reference's loop, :896-937), the same in all of the
     // pixel's lanes
     const float closest = 10.f, factor = 0.9f;
-    const float cached = own ? __ldg(P.res + k) : 0.0f;
+    const float cached = own ? P.res[k] : 0.0f;
     float best = (float)((double)cached + 10e-7);
     float owx = 0.f, owy = 0.f, owt = 0.f;  // running best offset
     int wkind = 0;                           // 0: the pixel's own, 1: a chain candidate, 2: the average
@@ -1133,7 +1133,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
     q.temporal = false;
     q.prev_fast = true;
     if (own) {
-        const float4 a = __ldg(P.off.A + k);
+        const float4 a = P.off.A[k];
         owx = a.x; owy = a.y;
         ia = T.base[px.sidx].w;
         dist = (float)(P.ex.w > P.ex.h ? P.ex.w : P.ex.h);
@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(kTileW * H * LPP, 2)
 #pragma unroll
             for (int j = -1; j <= 1; j++) {
                 if (!in_rect(P, x + i, y + j) || (i == 0 && j == 0)) continue;
-                const float4 nb = __ldg(P.off.A + (size_t)(y + j) * P.W + (x + i));
+                const float4 nb = P.off.A[(size_t)(y + j) * P.W + (x + i)];
                 if (__float_as_int(nb.w) != 0) continue;
                 avgx = avgx + nb.x;
                 avgy = avgy + nb.y;
@@ -1522,7 +1522,7 @@ static cudaError_t allow_smem(F* kernel, size_t smem, std::atomic<uint64_t>& don
 
 template <int R, int TM, int HW, int CPL, int H>
 static cudaError_t launch_propagate_t(const Params& P, const TileMaps& M, PatchPlanes work, int jump,
-                                      cudaStream_t s) {
+                                      bool dependent, cudaStream_t s) {
     constexpr int NP = kTileW * H, NT = NP * 4 / CPL;
     constexpr size_t smem =
         (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(EvalSmem<R, NT / 32, NP, 32 * CPL, 4>);
@@ -1530,12 +1530,13 @@ static cudaError_t launch_propagate_t(const Params& P, const TileMaps& M, PatchP
     const cudaError_t e = allow_smem(kt_propagate<R, TM, HW, CPL, H>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
-    return pt::launch_dependent(kt_propagate<R, TM, HW, CPL, H>, g, dim3(kTileW, NT / kTileW), smem, s, P, M, work, jump);
+    return pt::launch_dependent(dependent, kt_propagate<R, TM, HW, CPL, H>, g, dim3(kTileW, NT / kTileW), smem, s, P, M,
+                                work, jump);
 }
 
 template <int R, int TM, int HW, int LPP, int H>
 static cudaError_t launch_scatter_t(const Params& P, const TileMaps& M, PatchPlanes work, int write_all,
-                                    uint32_t pass_id, cudaStream_t s) {
+                                    uint32_t pass_id, bool dependent, cudaStream_t s) {
     constexpr int NP = kTileW * H, NT = NP * LPP;
     constexpr size_t smem =
         (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(EvalSmem<R, NT / 32, NP, 64, 2 * LPP>);
@@ -1543,38 +1544,40 @@ static cudaError_t launch_scatter_t(const Params& P, const TileMaps& M, PatchPla
     const cudaError_t e = allow_smem(kt_scatter<R, TM, HW, LPP, H>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
-    return pt::launch_dependent(kt_scatter<R, TM, HW, LPP, H>, g, dim3(kTileW, NT / kTileW), smem, s, P, M, work, write_all, pass_id);
+    return pt::launch_dependent(dependent, kt_scatter<R, TM, HW, LPP, H>, g, dim3(kTileW, NT / kTileW), smem, s, P, M,
+                                work, write_all, pass_id);
 }
 
 template <int R, int TM, int HW, int LPP, int H, bool KEEP>
-static cudaError_t launch_residual_t(const Params& P, const TileMaps& M, float* out, cudaStream_t s) {
+static cudaError_t launch_residual_t(const Params& P, const TileMaps& M, float* out, bool dependent, cudaStream_t s) {
     constexpr int NP = kTileW * H, NT = NP * LPP;
     constexpr size_t smem = (sizeof(TileSmem<R, TM, H>) + 127) / 128 * 128 + sizeof(ResidSmem<R, NT / 32, NP, KEEP>);
     static std::atomic<uint64_t> done{0};
     const cudaError_t e = allow_smem(kt_residual<R, TM, HW, LPP, H, KEEP>, smem, done);
     if (e != cudaSuccess) return e;
     const dim3 g((P.lw + kTileW - 1) / kTileW, (P.lh + H - 1) / H);
-    return pt::launch_dependent(kt_residual<R, TM, HW, LPP, H, KEEP>, g, dim3(kTileW, NT / kTileW), smem, s, P, M, out);
+    return pt::launch_dependent(dependent, kt_residual<R, TM, HW, LPP, H, KEEP>, g, dim3(kTileW, NT / kTileW), smem, s,
+                                P, M, out);
 }
 
 template <int R>
 cudaError_t launch_tiled_r(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
-                           uint32_t pass_id, float* out, int wide, cudaStream_t s) {
+                           uint32_t pass_id, float* out, int wide, bool dependent, cudaStream_t s) {
     // the texture-unit kernels fetch through the exemplar's textures, which
     // must be bound
     if (P.ex.hw && (!P.ex.tbase || !P.ex.tout)) return cudaErrorInvalidValue;
-#define PT_TILED_DISPATCH(TMV, HWV)                                                                   \
-    if (kind == 0 && wide) return launch_propagate_t<R, TMV, HWV, 1, kPropH>(P, M, work, arg, s);     \
-    else if (kind == 0) return launch_propagate_t<R, TMV, HWV, 2, kPropH>(P, M, work, arg, s);        \
-    else if (kind == 1 && wide)                                                                        \
-        return launch_scatter_t<R, TMV, HWV, 4, kScatHWide>(P, M, work, arg, pass_id, s);             \
-    else if (kind == 1) return launch_scatter_t<R, TMV, HWV, 2, kScatH>(P, M, work, arg, pass_id, s);  \
-    else if (wide && (P.inc.on || P.inc.fill))                                                         \
-        return launch_residual_t<R, TMV, HWV, 4, kResidHWide, true>(P, M, out, s);                    \
-    else if (wide) return launch_residual_t<R, TMV, HWV, 4, kResidHWide, false>(P, M, out, s);        \
-    else if (P.inc.on || P.inc.fill)                                                                   \
-        return launch_residual_t<R, TMV, HWV, HWV ? 1 : 2, kResidH, true>(P, M, out, s);              \
-    else return launch_residual_t<R, TMV, HWV, HWV ? 1 : 2, kResidH, false>(P, M, out, s);
+#define PT_TILED_DISPATCH(TMV, HWV)                                                                           \
+    if (kind == 0 && wide) return launch_propagate_t<R, TMV, HWV, 1, kPropH>(P, M, work, arg, dependent, s);  \
+    else if (kind == 0) return launch_propagate_t<R, TMV, HWV, 2, kPropH>(P, M, work, arg, dependent, s);     \
+    else if (kind == 1 && wide)                                                                               \
+        return launch_scatter_t<R, TMV, HWV, 4, kScatHWide>(P, M, work, arg, pass_id, dependent, s);          \
+    else if (kind == 1) return launch_scatter_t<R, TMV, HWV, 2, kScatH>(P, M, work, arg, pass_id, dependent, s);\
+    else if (wide && (P.inc.on || P.inc.fill))                                                                \
+        return launch_residual_t<R, TMV, HWV, 4, kResidHWide, true>(P, M, out, dependent, s);                 \
+    else if (wide) return launch_residual_t<R, TMV, HWV, 4, kResidHWide, false>(P, M, out, dependent, s);     \
+    else if (P.inc.on || P.inc.fill)                                                                          \
+        return launch_residual_t<R, TMV, HWV, HWV ? 1 : 2, kResidH, true>(P, M, out, dependent, s);           \
+    else return launch_residual_t<R, TMV, HWV, HWV ? 1 : 2, kResidH, false>(P, M, out, dependent, s);
     if (P.ex.hw) {
         if (tm == TM_NONE) { PT_TILED_DISPATCH(TM_NONE, 1) }
         else if (tm == TM_FWD) { PT_TILED_DISPATCH(TM_FWD, 1) }

@@ -24,8 +24,9 @@ inline void gaussian_weights(int r, bool normalize, float* w) {
 }
 
 #ifdef __CUDACC__
-// A launch whose blocks may start before the stream's previous kernel has
-// ended; the kernel calls pdl_start before it touches global memory.  Measured
+// With `dependent`, a launch whose blocks may start before the stream's
+// previous kernel has ended; the kernel calls pdl_start before it touches
+// global memory, and so does the previous one (pt_ctx::chained).  Measured
 // on whole syntheses: 128x128 still 5.38 -> 5.00 ms, four 512x512 frames 87.7
 // -> 81.6 ms.  Larger grids than these hide a launch behind the last blocks of
 // the one before anyway, and the blocks that wait take places from them: with
@@ -33,7 +34,8 @@ inline void gaussian_weights(int r, bool normalize, float* w) {
 // and 248 with this limit.
 constexpr size_t kDependentBlocks = 3000;
 template <class... K, class... A>
-inline cudaError_t launch_dependent(void (*kernel)(K...), dim3 g, dim3 b, size_t smem, cudaStream_t s, A... args) {
+inline cudaError_t launch_dependent(bool dependent, void (*kernel)(K...), dim3 g, dim3 b, size_t smem, cudaStream_t s,
+                                    A... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -43,7 +45,7 @@ inline cudaError_t launch_dependent(void (*kernel)(K...), dim3 g, dim3 b, size_t
     c.dynamicSmemBytes = smem;
     c.stream = s;
     c.attrs = at;
-    c.numAttrs = (size_t)g.x * g.y <= kDependentBlocks ? 1 : 0;
+    c.numAttrs = dependent && (size_t)g.x * g.y <= kDependentBlocks ? 1 : 0;
     return cudaLaunchKernelEx(&c, kernel, args...);
 }
 #endif
@@ -77,7 +79,7 @@ cudaError_t launch_fill_ribbons(Ribbon* r, size_t n, int layer, cudaStream_t s);
 cudaError_t launch_ribbon_pack(const Ribbon* src, int w, int h, float4* dst, cudaStream_t s);
 cudaError_t launch_ribbon_down(const float4* src, int sw, float4* dst, int w, int h, cudaStream_t s);
 cudaError_t launch_residual(const Params& P, float* out, cudaStream_t s);
-cudaError_t launch_canvas(const Params& P, float4* canvas, cudaStream_t s);
+cudaError_t launch_canvas(const Params& P, float4* canvas, bool dependent, cudaStream_t s);
 // the tiles (kTileW x tile_h) with a pixel that is not culled (IncView::tiles)
 cudaError_t launch_active_tiles(const Params& P, int tile_h, int* list, cudaStream_t s);
 cudaError_t launch_random_offsets(const Params& P, PatchPlanes work, cudaStream_t s);
@@ -133,11 +135,11 @@ cudaError_t launch_interleave_texels(const float4* base, const float4* out, cons
 // 2 = residual (into out); tm 0 = no temporal terms, 1 = forward, 2 = backward;
 // M: the tensor maps of the staged planes (M.on = 0: staged by plain loads);
 // wide: four lanes per pixel instead of two (propagate, scatter) or instead of
-// one or two (residual); same results
+// one or two (residual); same results; dependent: launch_dependent
 cudaError_t launch_tiled_2(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
-                           uint32_t pass_id, float* out, int wide, cudaStream_t s);
+                           uint32_t pass_id, float* out, int wide, bool dependent, cudaStream_t s);
 cudaError_t launch_tiled_3(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
-                           uint32_t pass_id, float* out, int wide, cudaStream_t s);
+                           uint32_t pass_id, float* out, int wide, bool dependent, cudaStream_t s);
 cudaError_t launch_tiled_4(int kind, int tm, const Params& P, const TileMaps& M, PatchPlanes work, int arg,
-                           uint32_t pass_id, float* out, int wide, cudaStream_t s);
+                           uint32_t pass_id, float* out, int wide, bool dependent, cudaStream_t s);
 }  // namespace pt

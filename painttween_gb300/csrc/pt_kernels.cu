@@ -583,8 +583,8 @@ cudaError_t launch_residual(const Params& P, float* out, cudaStream_t s) {
     k_residual<<<grid2(P.lw, P.lh, kCoopPix), kCoopThreads, 0, s>>>(P, out);
     LAUNCH_CHECK();
 }
-cudaError_t launch_canvas(const Params& P, float4* canvas, cudaStream_t s) {
-    return launch_dependent(k_canvas, grid2(P.lw, P.lh, kPix), kPix, 0, s, P, canvas);
+cudaError_t launch_canvas(const Params& P, float4* canvas, bool dependent, cudaStream_t s) {
+    return launch_dependent(dependent, k_canvas, grid2(P.lw, P.lh, kPix), kPix, 0, s, P, canvas);
 }
 cudaError_t launch_active_tiles(const Params& P, int tile_h, int* list, cudaStream_t s) {
     const cudaError_t e = cudaMemsetAsync(list, 0, sizeof(int), s);

@@ -128,10 +128,10 @@ static pt_status propagate_pass(pt_ctx* c, int level, int jump, int key = -1) {
     TRY(writable_work(c, level, &work));
     Params P = make_params(c, level);
     const bool keys = c->params.interpolateKeyFrame != 0;
-    return profiled(c, PT_KERNEL_PROPAGATE, P, [&](const Params& Q) {
+    return profiled(c, PT_KERNEL_PROPAGATE, P, [&](const Params& Q, bool dependent) {
         if (keys) return pt::launch_propagate_keys(Q, work, jump, key, key_view(c), c->stream);
         bool done = false;
-        cudaError_t e = key >= 0 ? cudaSuccess : launch_tiled(c, 0, Q, work, jump, 0, nullptr, &done);
+        cudaError_t e = key >= 0 ? cudaSuccess : launch_tiled(c, 0, Q, work, jump, 0, nullptr, dependent, &done);
         return done ? e : pt::launch_propagate(Q, work, jump, key, c->stream);
     });
 }
@@ -143,10 +143,11 @@ static pt_status scatter_pass(pt_ctx* c, int level, int key = -1) {
     Params P = make_params(c, level);
     uint32_t pass_id = c->pass_counter++;
     const bool keys = c->params.interpolateKeyFrame != 0;
-    return profiled(c, PT_KERNEL_SCATTER, P, [&](const Params& Q) {
+    return profiled(c, PT_KERNEL_SCATTER, P, [&](const Params& Q, bool dependent) {
         if (keys) return pt::launch_scatter_keys(Q, work, aliased ? 1 : 0, key, key_view(c), c->stream);
         bool done = false;
-        cudaError_t e = key >= 0 ? cudaSuccess : launch_tiled(c, 1, Q, work, aliased ? 1 : 0, pass_id, nullptr, &done);
+        cudaError_t e = cudaSuccess;
+        if (key < 0) e = launch_tiled(c, 1, Q, work, aliased ? 1 : 0, pass_id, nullptr, dependent, &done);
         return done ? e : pt::launch_scatter(Q, work, aliased ? 1 : 0, pass_id, key, c->stream);
     });
 }
