@@ -31,7 +31,14 @@ static void destroy_tex_array(TexArray& t) {
     t = TexArray();
 }
 
+// Memory is short: what the context can do without goes, the free blocks and
+// the random level's scratch (unless it is being set up).
 static void release_cache(pt_ctx* c) {
+    if (!c->draws_busy) {
+        dfree_t(c, c->draws);
+        dfree_t(c, c->trials);
+        c->draws_cap = 0;
+    }
     if (c->cache.empty() && c->tex_free.empty()) return;
     cudaStreamSynchronize(c->stream);
     for (auto& kv : c->cache) cudaFree(kv.second);
@@ -759,32 +766,26 @@ static void matmul31(const uint32_t* a, const uint32_t* b, uint32_t* out) {
             out[i * 31 + j] = s;
         }
 }
-// The powers step^(segment steps * 2^b) of the generator's step, each
-// transposed: the jumps to the segments of a stream (k_glibc_states).
-// Computed once a process; streams of up to 2^31 draws need 23.
-static const int kGlibcPowers = 23;
-const std::vector<uint32_t>& glibc_powers() {
-    static const std::vector<uint32_t> all = [] {
-        // one step: s'[i] = s[i+1] (i < 30), s'[30] = s[0] + s[28]
-        std::vector<uint32_t> M(961, 0), R(961, 0), T(961), out;
-        for (int i = 0; i < 30; i++) M[i * 31 + i + 1] = 1;
-        M[30 * 31 + 0] = 1;
-        M[30 * 31 + 28] += 1;
-        for (int i = 0; i < 31; i++) R[i * 31 + i] = 1;
-        for (int n = pt::glibc_segment_steps(); n; n >>= 1) {
-            if (n & 1) { matmul31(R.data(), M.data(), T.data()); R.swap(T); }
-            matmul31(M.data(), M.data(), T.data());
-            M.swap(T);
-        }
-        for (int b = 0; b < kGlibcPowers; b++) {
-            for (int k = 0; k < 31; k++)
-                for (int i = 0; i < 31; i++) out.push_back(R[i * 31 + k]);
-            matmul31(R.data(), R.data(), T.data());
-            R.swap(T);
-        }
-        return out;
-    }();
-    return all;
+// (jumps to the segments of a stream, k_glibc_states)
+std::vector<uint32_t> pt::glibc_powers(int segment, int count) {
+    // one step: s'[i] = s[i+1] (i < 30), s'[30] = s[0] + s[28]
+    std::vector<uint32_t> M(961, 0), R(961, 0), T(961), out;
+    for (int i = 0; i < 30; i++) M[i * 31 + i + 1] = 1;
+    M[30 * 31 + 0] = 1;
+    M[30 * 31 + 28] += 1;
+    for (int i = 0; i < 31; i++) R[i * 31 + i] = 1;
+    for (int n = segment; n; n >>= 1) {
+        if (n & 1) { matmul31(R.data(), M.data(), T.data()); R.swap(T); }
+        matmul31(M.data(), M.data(), T.data());
+        M.swap(T);
+    }
+    for (int b = 0; b < count; b++) {
+        for (int k = 0; k < 31; k++)
+            for (int i = 0; i < 31; i++) out.push_back(R[i * 31 + k]);
+        matmul31(R.data(), R.data(), T.data());
+        R.swap(T);
+    }
+    return out;
 }
 
 // ---------------------------------------------------------------------------
@@ -861,7 +862,7 @@ pt_status pt_create(int device, size_t budget, pt_ctx** out) {
         return PT_ERR_CUDA;
     }
     pt_default_params(&c->params);
-    if (dalloc_t(c, &c->flag, 4) != PT_OK || dalloc_t(c, &c->tma_err, 1) != PT_OK) {
+    if (dalloc_t(c, &c->flag, 64) != PT_OK || dalloc_t(c, &c->tma_err, 1) != PT_OK) {
         cudaStreamDestroy(c->stream);
         delete c;
         return PT_ERR_OOM;

@@ -183,14 +183,13 @@ struct pt_ctx {
     size_t stage_bytes = 0;
     float* conv_scratch = nullptr;
     size_t conv_scratch_elems = 0;
-    // random levels: the generator's matrix powers, and the scratch of one
-    // level (segment states, draws, trials, starts, how far they sufficed)
-    uint32_t* glibc_mats = nullptr;
-    uint32_t* states = nullptr;
+    // random levels: the draws of a window of the stream, their trials
     uint32_t* draws = nullptr;
     uint8_t* trials = nullptr;
-    int* starts = nullptr;
-    size_t states_cap = 0, draws_cap = 0, starts_cap = 0;
+    size_t draws_cap = 0;
+    bool draws_busy = false;
+    // 64 words: [0, 1] counts of unpainted texels, [4 ...] the random level's
+    // Walk, [8 ...] the state of its last segment
     int* flag = nullptr;
 
     // resident working set
@@ -304,7 +303,6 @@ PT_HIDDEN void free_frames(pt_ctx* c);
 PT_HIDDEN void free_store(pt_ctx* c);
 PT_HIDDEN void free_textures(pt_ctx* c, ExLevel* L);
 PT_HIDDEN void glibc_state(uint32_t seed, uint32_t out[31]);
-PT_HIDDEN const std::vector<uint32_t>& glibc_powers();
 PT_HIDDEN pt_status h2d(pt_ctx* c, void* dst, const void* src, size_t bytes);
 PT_HIDDEN cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,
                                    float* out, bool dependent, bool* done);

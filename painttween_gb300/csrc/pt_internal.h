@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "pt_types.h"
 
@@ -113,18 +114,22 @@ struct RandomLevel {
     int nk, first_key;
 };
 using ptk::GlibcState;
-// segments of a stream of `draws` draws, and the generator's steps of one
-size_t glibc_segments(size_t draws);
-int glibc_segment_steps();
-// pixels that cannot retry: four draws each.  mats: the transposed powers
-// step^(segment steps * 2^b); states: 31 words a segment
-cudaError_t launch_random_level(const RandomLevel& L, const GlibcState& s0, const uint32_t* mats, uint32_t* states,
+using ptk::Walk;
+// the powers step^(segment * 2^b), b < count, of glibc's generator, each transposed (31 x 31)
+std::vector<uint32_t> glibc_powers(int segment, int count);
+// Pixels that cannot retry: four draws each, no scratch but `last` (31 words).
+// *launches grows by the kernels launched.
+cudaError_t launch_random_level(const RandomLevel& L, const GlibcState& s0, uint32_t* last, int* launches,
                                 cudaStream_t s);
-// with retries or keys, from a stream of n draws (n > 1000; what it does not
-// suffice for is drawn serially); trials: n bytes, starts: w * h, done: 2
-cudaError_t launch_random_level_retry(const RandomLevel& L, const GlibcState& s0, const uint32_t* mats,
-                                      uint32_t* states, uint32_t* draws, size_t n, uint8_t* trials, int* starts,
-                                      int* done, cudaStream_t s);
+// With retries or keys: windows of the stream up to `total` draws in all (what
+// these do not suffice for is drawn serially); draws and trials: `window`
+// elements, a size that random_window gave, or null (all is drawn serially);
+// last: 31 words.
+constexpr size_t kRandomWindow = 1 << 20;  // 5 MB of scratch
+size_t random_window(size_t n);
+cudaError_t launch_random_level_retry(const RandomLevel& L, const GlibcState& s0, size_t total, uint32_t* draws,
+                                      uint8_t* trials, size_t window, uint32_t* last, Walk* walk, int* launches,
+                                      cudaStream_t s);
 cudaError_t launch_random_level_counter(const RandomLevel& L, uint32_t seed, cudaStream_t s);
 cudaError_t launch_count_transparent(const float4* out, size_t n, int* count, cudaStream_t s);
 cudaError_t launch_interleave_texels(const float4* base, const float4* out, const float* dt, float4* bo, int* flags,

@@ -7,7 +7,8 @@
 // trials), then two draws for the fractions.  Here the stream is cut into
 // segments that are generated in parallel, each from its state, which the
 // powers of the generator's step matrix give (k_glibc_states, k_glibc_draws).
-// Without retries pixel k's draws are the k-th four.  With them:
+// Without retries pixel k's draws are the k-th four.  With them, window by
+// window of the stream, so that the scratch stays small (5 bytes a draw):
 //  * k_trials: for every place in the stream, how many trials an opaque pixel
 //    that starts there takes;
 //  * k_starts: the one serial part, a warp that follows the places from
@@ -18,6 +19,10 @@
 // 1 ms of host work and a synchronisation less), a 192x160 level of an
 // exemplar with a fifth of it unpainted 18.6 -> 0.84 ms, bounded by k_starts'
 // chain of about 60 cycles a retry.
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 #include "pt_common.cuh"
 #include "pt_device.cuh"
 #include "pt_internal.h"
@@ -25,6 +30,12 @@
 namespace ptk {
 
 constexpr int kSegment = 496;  // draws of a segment: 16 turns of the 31-word state
+
+// The powers step^(kSegment 2^b) of the generator's step, each transposed, in
+// the library's own device memory (no context's budget pays for them), filled
+// once a device.  Streams of up to 2^31 draws need 23.
+constexpr int kPowers = 23;
+__device__ uint32_t g_powers[kPowers * 961];
 
 struct RandParams {
     int w, h, mx, my;
@@ -67,18 +78,26 @@ __device__ __forceinline__ bool opaque_pixel(const RandParams& R, int k) {
     return __ldg(R.img.p + (size_t)y * R.img.w + x).w > kAlphaThreshold;
 }
 
-// The state at the start of each segment: segment g starts g * kSegment
-// steps on, so its state is the product of the powers mats[b] = step^(kSegment
-// 2^b) (transposed) of g's bits with the seed's state.  A warp a segment;
-// word i of segment g goes to states[i * segments + g].
-__global__ void __launch_bounds__(256) k_glibc_states(const GlibcState s0, const uint32_t* __restrict__ mats,
-                                                      int segments, uint32_t* states) {
-    const int g = blockIdx.x * 8 + threadIdx.x / 32, i = threadIdx.x % 32;
-    if (g >= segments) return;
+// The state at the start of each segment: segment g of the stream starts g *
+// kSegment steps on, so its state is the product of the powers of g's bits
+// with the seed's state.  A warp a segment.  The states lie where the draws
+// will be, each at its segment's start; the last segment's, whose draws may
+// be fewer than 31, in `last`.
+__device__ __forceinline__ uint32_t* segment_state(uint32_t* draws, uint32_t* last, int segments, int i) {
+    return i == segments - 1 ? last : draws + (size_t)i * kSegment;
+}
+// (walk: with retries; nothing is left to do once every pixel has its place)
+__device__ __forceinline__ bool walk_done(const Walk* walk, int px) { return walk && walk->next >= px; }
+
+__global__ void __launch_bounds__(256) k_glibc_states(const GlibcState s0, int first, int segments, uint32_t* draws,
+                                                      uint32_t* last, const Walk* walk, int px) {
+    const int seg = blockIdx.x * 8 + threadIdx.x / 32, i = threadIdx.x % 32;
+    if (seg >= segments || walk_done(walk, px)) return;
+    const int g = first + seg;
     uint32_t s = i < 31 ? s0.s[i] : 0u;
     for (int b = 0; g >> b; b++) {
         if (!((g >> b) & 1)) continue;
-        const uint32_t* M = mats + (size_t)b * 961;
+        const uint32_t* M = g_powers + (size_t)b * 961;
         uint32_t acc = 0;
 #pragma unroll
         for (int k = 0; k < 31; k++) {
@@ -87,19 +106,22 @@ __global__ void __launch_bounds__(256) k_glibc_states(const GlibcState s0, const
         }
         s = acc;
     }
-    if (i < 31) states[(size_t)i * segments + g] = s;
+    if (i < 31) segment_state(draws, last, segments, seg)[i] = s;
 }
 
 // The draws of each segment, a thread a segment with the 31-word state of
 // r[i] = r[i-31] + r[i-3] in registers; each turn's 31 words go through
 // shared memory so that a warp writes whole runs.
-__global__ void __launch_bounds__(32) k_glibc_draws(const uint32_t* __restrict__ states, int segments, size_t n,
-                                                    uint32_t* draws) {
+__global__ void __launch_bounds__(32) k_glibc_draws(int segments, size_t n, uint32_t* draws, uint32_t* last,
+                                                    const Walk* walk, int px) {
     __shared__ uint32_t out[32][33];
     const int lane = threadIdx.x, g0 = blockIdx.x * 32, g = g0 + lane;
+    if (walk_done(walk, px)) return;
+    const uint32_t* state = segment_state(draws, last, segments, min(g, segments - 1));
     uint32_t r[31];
 #pragma unroll
-    for (int i = 0; i < 31; i++) r[i] = g < segments ? __ldg(states + (size_t)i * segments + g) : 0u;
+    for (int i = 0; i < 31; i++) r[i] = state[i];
+    __syncwarp();  // (the warp's draws go over its segments' states)
 #pragma unroll 1
     for (int turn = 0; turn < kSegment / 31; turn++) {
 #pragma unroll
@@ -128,9 +150,9 @@ __global__ void __launch_bounds__(256) k_texels_plain(const RandParams R) {
 // trials of an opaque pixel that starts at draw a (draws past n count as
 // painted: k_starts does not go there)
 __global__ void __launch_bounds__(256) k_trials(const RandParams R, const uint32_t* __restrict__ draws, int n,
-                                                uint8_t* trials) {
+                                                uint8_t* trials, const Walk* walk) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n) return;
+    if (a >= n || walk_done(walk, R.w * R.h)) return;
     int t = 1;
     if (R.lead || !(a & 1)) {  // (without keys every pixel starts at an even place)
         const float4* L = layer_out(R, R.lead ? style_of(R, draws[a]) : 0);
@@ -143,20 +165,25 @@ __global__ void __launch_bounds__(256) k_trials(const RandParams R, const uint32
     trials[a] = (uint8_t)t;
 }
 
-// The place in the stream at which each pixel starts.  One block; its first
-// warp walks, the others help to stage the windows of `trials` and of the
-// pixels' opacity.  A lane takes a pixel as if those before it in the step
-// had no retry; the step ends at the first that has one.  done[0]: the pixels
-// that the n draws sufficed for.
+// The place among the window's n draws at which each pixel starts, left in
+// the bits of its texel's first word.  One block; its first warp walks, the
+// others help to stage parts of `trials` and of the pixels' opacity.  A lane
+// takes a pixel as if those before it in the step had no retry; the step ends
+// at the first that has one.  The walk goes on from the window before, whose
+// draws began `back` places earlier; it ends with less than a reserve of
+// draws left, and windows overlap by a segment, which is more, so the place
+// it ends at is one of the next window's.
 constexpr int kWalkWindow = 1 << 15, kWalkReserve = 1 + 2 * 50 + 2 + 5 * 32;
+static_assert(kSegment >= kWalkReserve + 31, "the next window holds the walk's place and the 31 draws before it");
 __global__ void __launch_bounds__(512) k_starts(const RandParams R, const uint8_t* __restrict__ trials, int n,
-                                                int* starts, int* done) {
+                                                int back, Walk* walk) {
     __shared__ __align__(16) uint8_t T[kWalkWindow];
     __shared__ uint32_t O[kWalkWindow / 4 / 32 + 1];
     __shared__ int at[2];  // the next pixel and its place
     const int px = R.w * R.h, c = R.lead + 4, tid = threadIdx.x, lane = tid % 32;
-    int k = 0, a = 0;
-    while (true) {
+    const int k0 = walk->next;
+    int k = k0, a = walk->place - back;
+    while (k < px) {
         const int count = min(n - a, kWalkWindow), pixels = min(px - k, kWalkWindow / 4);
         for (int i = tid; i < count; i += blockDim.x) T[i] = trials[a + i];
         for (int i = tid; i < (pixels + 31) / 32 * 32; i += blockDim.x) {
@@ -173,7 +200,7 @@ __global__ void __launch_bounds__(512) k_starts(const RandParams R, const uint8_
                 const int t = in && ((O[j / 32] >> (j % 32)) & 1) ? T[da + c * lane] : 1;
                 const unsigned retry = __ballot_sync(0xffffffffu, t != 1);
                 const int s = retry ? __ffs(retry) - 1 : m - 1;  // the step's last pixel
-                if (lane <= s) starts[k + j] = a + da + c * lane;
+                if (lane <= s) R.out[k + j].x = __int_as_float(a + da + c * lane);
                 da += c * s + R.lead + 2 + 2 * __shfl_sync(0xffffffffu, t, s);
                 dk += s + 1;
             }
@@ -188,37 +215,36 @@ __global__ void __launch_bounds__(512) k_starts(const RandParams R, const uint8_
         const bool stuck = k1 == k;  // fewer than a reserve of draws left
         k = k1;
         a = a1;
-        if (k >= px || stuck) break;
+        if (stuck) break;
     }
+    __syncthreads();  // (all have read the walk)
     if (tid == 0) {
-        done[0] = k;
-        done[1] = a;
+        walk->first = k0;
+        walk->next = k;
+        walk->place = k < px ? a : back;
     }
 }
 
-// every pixel that k_starts placed, from its place
+// every pixel that k_starts placed in this window, from its place
 __global__ void __launch_bounds__(256) k_texels(const RandParams R, const uint32_t* __restrict__ draws,
-                                                const uint8_t* __restrict__ trials, const int* __restrict__ starts,
-                                                const int* __restrict__ done) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= R.w * R.h || k >= __ldg(done)) return;
-    const int a = starts[k], t = opaque_pixel(R, k) ? trials[a] : 1;
+                                                const uint8_t* __restrict__ trials, const Walk* walk) {
+    const int k = walk->first + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k >= walk->next) return;
+    const int a = __float_as_int(R.out[k].x), t = opaque_pixel(R, k) ? trials[a] : 1;
     const uint32_t* d = draws + a + R.lead + 2 * (t - 1);
     R.out[k] = random_texel(R, k % R.w, k / R.w, R.lead ? style_of(R, draws[a]) : 0, d[0], d[1], d[2], d[3]);
 }
 
-// The pixels that the draws did not suffice for (an exemplar with hardly a
-// painted texel), one thread on from where k_starts ended: the stream goes on
-// from its last 31 draws.
-__global__ void k_rest(const RandParams R, const uint32_t* draws, const int* done) {
+// The pixels that the windows' draws did not suffice for (an exemplar with
+// hardly a painted texel), one thread on from where k_starts ended: the 31
+// draws before that place in the last window are the state there.  Without
+// any draws (no scratch to be had), the whole level from the seed.
+__global__ void k_rest(const RandParams R, const GlibcState s0, const uint32_t* draws, const Walk* walk) {
     const int px = R.w * R.h;
-    int k = done[0];
+    int k = draws ? walk->next : 0;
     if (k >= px) return;
-    // the 31 draws before place a are the state there; k_starts leaves at
-    // least that many behind it or starts at the stream's seed (place 0)
-    const int a = done[1];
     uint32_t ring[31];
-    for (int i = 0; i < 31; i++) ring[i] = draws[a - 31 + i];
+    for (int i = 0; i < 31; i++) ring[i] = draws ? draws[walk->place - 31 + i] : s0.s[i];
     int head = 0;
     auto next = [&]() -> uint32_t {
         int h28 = head + 28;
@@ -297,38 +323,77 @@ static RandParams rand_params(const RandomLevel& L) {
     return R;
 }
 
-size_t glibc_segments(size_t draws) { return (draws + kSegment - 1) / kSegment; }
-int glibc_segment_steps() { return kSegment; }
+// g_powers of the current device
+static cudaError_t powers_ready(cudaStream_t s) {
+    static std::mutex m;
+    static uint64_t done = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(m);
+    if (dev < 64 && (done >> dev & 1)) return cudaSuccess;
+    const std::vector<uint32_t> all = glibc_powers(kSegment, kPowers);
+    e = cudaMemcpyToSymbolAsync(g_powers, all.data(), all.size() * sizeof(uint32_t), 0, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // (other contexts' streams read them next)
+    if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
+    return e;
+}
 
-static cudaError_t draw_stream(const GlibcState& s0, const uint32_t* mats, size_t n, uint32_t* states,
-                               uint32_t* draws, cudaStream_t s) {
-    const int seg = (int)glibc_segments(n);
-    k_glibc_states<<<(seg + 7) / 8, 256, 0, s>>>(s0, mats, seg, states);
-    k_glibc_draws<<<(seg + 31) / 32, 32, 0, s>>>(states, seg, n, draws);
+// n draws of the stream from segment `first` on
+static cudaError_t draw_stream(const GlibcState& s0, int first, size_t n, uint32_t* draws, uint32_t* last,
+                               const Walk* walk, int px, cudaStream_t s) {
+    const int seg = (int)((n + kSegment - 1) / kSegment);
+    k_glibc_states<<<(seg + 7) / 8, 256, 0, s>>>(s0, first, seg, draws, last, walk, px);
+    k_glibc_draws<<<(seg + 31) / 32, 32, 0, s>>>(seg, n, draws, last, walk, px);
     return cudaGetLastError();
 }
 
-cudaError_t launch_random_level(const RandomLevel& L, const GlibcState& s0, const uint32_t* mats, uint32_t* states,
+cudaError_t launch_random_level(const RandomLevel& L, const GlibcState& s0, uint32_t* last, int* launches,
                                 cudaStream_t s) {
     const RandParams R = rand_params(L);
     const size_t px = (size_t)L.w * L.h;
-    const cudaError_t e = draw_stream(s0, mats, 4 * px, states, (uint32_t*)L.out, s);
+    cudaError_t e = powers_ready(s);
+    if (e == cudaSuccess) e = draw_stream(s0, 0, 4 * px, (uint32_t*)L.out, last, nullptr, 0, s);
     if (e != cudaSuccess) return e;
     k_texels_plain<<<(unsigned)((px + 255) / 256), 256, 0, s>>>(R);
+    *launches += 3;
     return cudaGetLastError();
 }
 
-cudaError_t launch_random_level_retry(const RandomLevel& L, const GlibcState& s0, const uint32_t* mats,
-                                      uint32_t* states, uint32_t* draws, size_t n, uint8_t* trials, int* starts,
-                                      int* done, cudaStream_t s) {
+size_t random_window(size_t n) {
+    const size_t least = 8, most = (kRandomWindow + kSegment - 1) / kSegment;
+    return std::min(std::max((n + kSegment - 1) / kSegment, least), most) * kSegment;
+}
+
+cudaError_t launch_random_level_retry(const RandomLevel& L, const GlibcState& s0, size_t total, uint32_t* draws,
+                                      uint8_t* trials, size_t window, uint32_t* last, Walk* walk, int* launches,
+                                      cudaStream_t s) {
     const RandParams R = rand_params(L);
-    const size_t px = (size_t)L.w * L.h;
-    const cudaError_t e = draw_stream(s0, mats, n, states, draws, s);
+    const int px = L.w * L.h, n = (int)window;
+    if (!draws) {
+        k_rest<<<1, 1, 0, s>>>(R, s0, nullptr, nullptr);
+        *launches += 1;
+        return cudaGetLastError();
+    }
+    cudaError_t e = powers_ready(s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(walk, 0, sizeof(Walk), s);
+    // (at least four draws a pixel)
+    const unsigned texels = (unsigned)((std::min(px, n / 4 + 1) + 255) / 256);
+    int back = 0;
+    for (size_t at = 0; e == cudaSuccess; at += back) {
+        e = draw_stream(s0, (int)(at / kSegment), n, draws, last, walk, px, s);
+        if (e != cudaSuccess) return e;
+        k_trials<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(R, draws, n, trials, walk);
+        k_starts<<<1, 512, 0, s>>>(R, trials, n, back, walk);
+        k_texels<<<texels, 256, 0, s>>>(R, draws, trials, walk);
+        *launches += 5;
+        e = cudaGetLastError();
+        back = n - kSegment;
+        if (at + n >= total) break;
+    }
     if (e != cudaSuccess) return e;
-    k_trials<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(R, draws, (int)n, trials);
-    k_starts<<<1, 512, 0, s>>>(R, trials, (int)n, starts, done);
-    k_texels<<<(unsigned)((px + 255) / 256), 256, 0, s>>>(R, draws, trials, starts, done);
-    k_rest<<<1, 1, 0, s>>>(R, draws, done);
+    k_rest<<<1, 1, 0, s>>>(R, s0, draws, walk);
+    *launches += 1;
     return cudaGetLastError();
 }
 

@@ -18,15 +18,27 @@ static pt_status ensure_transparency_known(pt_ctx* c) {
     return PT_OK;
 }
 
-// scratch of at least n elements
-template <class T>
-static pt_status ensure_scratch(pt_ctx* c, T** p, size_t* cap, size_t n) {
-    if (*cap >= n) return PT_OK;
-    dfree_t(c, *p);
-    *cap = 0;
-    TRY(dalloc_t(c, p, n));
-    *cap = n;
-    return PT_OK;
+// Scratch for a window of a stream of n draws; its size, 0 if there is none to
+// be had.  A context short of memory takes smaller windows: the level needs
+// none of it, and other allocations of the context take it back.
+static size_t draw_scratch(pt_ctx* c, size_t n) {
+    for (size_t want = pt::random_window(n);; want = pt::random_window(want / 4)) {
+        if (c->draws_cap >= want) return want;
+        dfree_t(c, c->draws);
+        dfree_t(c, c->trials);
+        c->draws_cap = 0;
+        c->draws_busy = true;
+        const bool ok = dalloc_t(c, &c->draws, want) == PT_OK && dalloc_t(c, &c->trials, want) == PT_OK;
+        c->draws_busy = false;
+        if (ok) {
+            c->draws_cap = want;
+            return want;
+        }
+        if (want == pt::random_window(1)) break;
+    }
+    dfree_t(c, c->draws);
+    dfree_t(c, c->trials);
+    return 0;
 }
 
 // SynthesisFrame::createRandomPyramid, synthesisFrame.cpp:66-150, over the
@@ -66,15 +78,11 @@ pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<fl
     TRY(ensure_transparency_known(c));
     pt::GlibcState s0;
     glibc_state((uint32_t)(frame * level), s0.s);
-    if (!c->glibc_mats) {
-        const std::vector<uint32_t>& m = glibc_powers();
-        TRY(dalloc_t(c, &c->glibc_mats, m.size()));
-        TRY(h2d(c, c->glibc_mats, m.data(), m.size() * sizeof(uint32_t)));
-    }
+    uint32_t* last = (uint32_t*)c->flag + 8;
+    int launches = 0;
     if (nk == 0 && (c->params.transparencyOk || !c->ex->transparent)) {
-        TRY(ensure_scratch(c, &c->states, &c->states_cap, 31 * pt::glibc_segments(4 * px)));
-        LN(pt::launch_random_level(L, s0, c->glibc_mats, c->states, c->stream));
-        c->launches += 2;
+        CU(pt::launch_random_level(L, s0, last, &launches, c->stream));
+        c->launches += launches;
         return PT_OK;
     }
     // the draws that the pixels take on average, and eight deviations more
@@ -82,20 +90,11 @@ pt_status random_level(pt_ctx* c, int level, int frame, Arr<float4> rgba, Arr<fl
     const double f = std::min((double)(nk ? c->ex->transparent_all : c->ex->transparent) / texels, 0.98);
     const double mean = (nk ? 1.0 : 0.0) + 2.0 + 2.0 / (1.0 - f), dev = 2.0 * std::sqrt(f) / (1.0 - f);
     const double want = std::min(1.05 * mean, 64.0) * (double)px + 8.0 * dev * std::sqrt((double)px) + 4096.0;
-    const size_t n = (size_t)std::min(want, (double)(1u << 30));
-    if (n > c->draws_cap) {
-        dfree_t(c, c->draws);
-        dfree_t(c, c->trials);
-        c->draws_cap = 0;
-        TRY(dalloc_t(c, &c->draws, n));
-        TRY(dalloc_t(c, &c->trials, n));
-        c->draws_cap = n;
-    }
-    TRY(ensure_scratch(c, &c->states, &c->states_cap, 31 * pt::glibc_segments(n)));
-    TRY(ensure_scratch(c, &c->starts, &c->starts_cap, px));
-    LN(pt::launch_random_level_retry(L, s0, c->glibc_mats, c->states, c->draws, n, c->trials, c->starts, c->flag + 2,
-                                     c->stream));
-    c->launches += 5;
+    const size_t total = (size_t)std::min(want, (double)(1u << 30));
+    const size_t window = draw_scratch(c, total);
+    CU(pt::launch_random_level_retry(L, s0, total, window ? c->draws : nullptr, c->trials, window, last,
+                                     (pt::Walk*)(c->flag + 4), &launches, c->stream));
+    c->launches += launches;
     return PT_OK;
 }
 

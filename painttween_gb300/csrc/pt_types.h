@@ -177,6 +177,12 @@ struct GlibcState {
     uint32_t s[31];
 };
 
+// How far the random level's pixels have their places in the stream: this
+// window's first pixel, the next pixel, and its place among the window's draws.
+struct Walk {
+    int first, next, place;
+};
+
 struct ConvKernel {
     int r;
     float w[2 * kMaxRadius + 1];
