@@ -31,9 +31,15 @@ static void destroy_tex_array(TexArray& t) {
     t = TexArray();
 }
 
-// Memory is short: what the context can do without goes, the free blocks and
-// the random level's scratch (unless it is being set up).
+void free_tile_lists(pt_ctx* c) {
+    for (auto& t : c->tile_list) dfree_t(c, t);
+    dfree_t(c, c->tile_mark);
+}
+// Memory is short: what the context can do without goes, the free blocks, the
+// random level's scratch (unless it is being set up) and the tile lists
+// (unless a loop uses them).
 static void release_cache(pt_ctx* c) {
+    if (!c->lists_held) free_tile_lists(c);
     if (!c->draws_busy) {
         dfree_t(c, c->draws);
         dfree_t(c, c->trials);
@@ -995,8 +1001,7 @@ pt_status pt_initialize(pt_ctx* c, int iw, int ih, int sw, int sh, int ns) {
     dfree_t(c, c->chg); dfree_t(c, c->stamp_last); dfree_t(c, c->stamp_win);
     dfree_t(c, c->tap_cache);
     c->tap_cache_k = 0;
-    for (auto& t : c->tile_list) dfree_t(c, t);
-    dfree_t(c, c->tile_mark);
+    free_tile_lists(c);
     free_store(c);
     c->initialized = false;
     c->W = iw; c->H = ih; c->SW = sw; c->SH = sh; c->NS = ns;

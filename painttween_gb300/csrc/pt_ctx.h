@@ -241,6 +241,7 @@ struct pt_ctx {
     // the residual's with its marks; inc_tiles: the lists of this pass
     int* tile_list[3] = {nullptr, nullptr, nullptr};
     int* tile_mark = nullptr;
+    bool lists_held = false;  // in use: not given back when memory is short
     int inc_tiles = 0;      // 0: none, 1: the residual's, 2: all
     int inc_kind = 0;       // the pass runs propagate (0) or scatter (1)
     int inc_canvas = 0;     // the residual kernel writes the canvas
@@ -302,6 +303,7 @@ PT_HIDDEN pt_status fail(pt_ctx* c, pt_status s, const char* fmt, ...);
 PT_HIDDEN void free_frames(pt_ctx* c);
 PT_HIDDEN void free_store(pt_ctx* c);
 PT_HIDDEN void free_textures(pt_ctx* c, ExLevel* L);
+PT_HIDDEN void free_tile_lists(pt_ctx* c);
 PT_HIDDEN void glibc_state(uint32_t seed, uint32_t out[31]);
 PT_HIDDEN pt_status h2d(pt_ctx* c, void* dst, const void* src, size_t bytes);
 PT_HIDDEN cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work, int arg, uint32_t pass_id,

@@ -133,6 +133,20 @@ static pt_status load_last_saved_offsets(pt_ctx* c, int frame, int level) {
     return store_load_offsets(c, level, frame, pass);
 }
 
+// The lists of active tiles and their marks, if there is memory for them: a
+// loop runs without them too, and other allocations take them back.
+static bool take_tile_lists(pt_ctx* c) {
+    const size_t n = (size_t)((c->W + ptk::kTileW - 1) / ptk::kTileW) * ((c->H + 1) / 2);
+    const bool held = c->lists_held;
+    c->lists_held = true;
+    bool ok = true;
+    for (auto& t : c->tile_list) ok = ok && (t || dalloc_t(c, &t, n + 1) == PT_OK);
+    ok = ok && (c->tile_mark || dalloc_t(c, &c->tile_mark, n) == PT_OK);
+    c->lists_held = held;
+    if (!ok) free_tile_lists(c);
+    return ok;
+}
+
 // SynthesisFrame::propagateAndScatter, synthesisFrame.cpp:483-508
 //
 // With change tracking (tiled kernels), every pass of the loop is numbered.
@@ -191,15 +205,17 @@ static pt_status propagate_and_scatter(pt_ctx* c, int level, int iterations, boo
         Params P = make_params(c, level);
         // (the list's tiles are the narrow shape's)
         lists = P.lw < 65536 * ptk::kTileW && P.lh < 65536 && !resid_wide(c, P);
+        if (lists) lists = take_tile_lists(c);
         if (lists) {
-            const size_t n = (size_t)((c->W + ptk::kTileW - 1) / ptk::kTileW) * ((c->H + 1) / 2);
-            for (auto& t : c->tile_list)
-                if (!t) TRY(dalloc_t(c, &t, n + 1));
-            if (!c->tile_mark) TRY(dalloc_t(c, &c->tile_mark, n));
             LN(pt::launch_active_tiles(P, ptk::kPropH, c->tile_list[0], c->stream));
             LN(pt::launch_active_tiles(P, scatter_wide(c, P) ? ptk::kScatHWide : ptk::kScatH, c->tile_list[1], c->stream));
         }
     }
+    struct Hold {  // the lists stay while the loop uses them
+        pt_ctx* c;
+        ~Hold() { c->lists_held = false; }
+    } hold{c};
+    c->lists_held = lists;
     std::map<int, int> last_pass;  // jump (0 = scatter) -> index of its last pass
     auto run = [&](int jump) -> pt_status {
         if (fill_after_first) {
