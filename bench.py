@@ -44,12 +44,13 @@ WORKLOAD = "clip1080p"
 METRIC = "1080p stylized frames/s"
 UNIT = "frames/s"
 
-# DRAM bytes (read + write) per level pixel of one propagate launch: the
-# ncu capture of a level-0 temporal launch of this workload (1920x1080 level,
-# 340.1 MB read + 64.9 MB written) summarised in
-# profiles/kt_energy_kernels_clip1080p.md.  The exemplar planes stay in L2,
-# so DRAM traffic follows the staged pixel-side planes, i.e. the level area.
-PROPAGATE_DRAM_BYTES_PER_PIXEL = (340.1e6 + 64.9e6) / (1920 * 1080)
+# DRAM bytes (read + write) per level pixel of one propagate launch: the mean
+# of three temporal launches in a row on the 1920x1080 level of this workload
+# (104.4 MB read + 11.3 MB written), captured with ncu and summarised in
+# profiles/kt_kernels_clip1080p.md.  The exemplar stays in L2 and idle tiles
+# are left out, so DRAM traffic follows the pixel-side planes of the others,
+# i.e. the level area at this workload's culling.
+PROPAGATE_DRAM_BYTES_PER_PIXEL = (104.4e6 + 11.3e6) / (1920 * 1080)
 
 
 def peaks():
@@ -362,7 +363,7 @@ def run_ours(args, dist):
     s = Synthesizer(device=device)
     s.setup(p, cfg["w"], cfg["h"], cfg["ew"], cfg["eh"], 1)
     if args.generic_kernels:
-        s.set_tiled_kernels(False)  # same results, one-thread-per-pixel kernels (profiling them)
+        s.set_tiled_kernels(False)  # same results, generic kernels (profiling them)
     s.set_tma_staging(args.staging == "tma")
     s.set_propagate_lanes(args.propagate_lanes)
     s.set_style(0, ex["base"], ex["output"], ex["orient_tensor"], ex["dist_trans"], ex["object_ids"])
@@ -483,7 +484,7 @@ def run_ours(args, dist):
                    "iterations": p.iterations, "scheme": "FMBM_RM", "histogram": True,
                    "kernels": "generic" if args.generic_kernels else "tiled",
                    "staging": args.staging,
-                   "propagate_warps_per_row": args.propagate_lanes or "autotuned",
+                   "propagate_lanes": {1: "two", 2: "four"}.get(args.propagate_lanes, "autotuned"),
                    "filter": args.filter,
                    "parallelism": "replicas" if dist.ws > 1 else "single",
                    "l2": "inputs larger than L2 (%.1f GB of resident frame pyramids per step)"
@@ -761,7 +762,7 @@ def main():
     ap.add_argument("--propagate-lanes", type=int, default=0, choices=[0, 1, 2],
                     help="propagate's lanes per pixel: 1 = two, 2 = four, 0 = autotuned per launch shape (same results)")
     ap.add_argument("--generic-kernels", action="store_true",
-                    help="run the generic one-thread-per-pixel kernels instead of the tiled ones (profiling only)")
+                    help="run the generic kernels instead of the tiled ones (profiling only)")
     args = ap.parse_args()
     dist = Dist()
     try:

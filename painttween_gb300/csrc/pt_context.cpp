@@ -570,10 +570,12 @@ static void tile_maps(pt_ctx* c, const Params& P, int tm, int tile_h, TileMaps* 
 // variant being timed (-1: none).  Launch shapes are keyed by radius,
 // temporal mode, filter mode and the tile count relative to the SM count,
 // in powers of two (up to a quarter, half, one, 2, 4, 8 SMs' worth, more):
-// the choice depends on how much of the GPU the tiles fill.  Decisions are
-// shared by the contexts of a
-// device; until a shape's two variants have been timed, shapes with no
-// more tiles than SMs take two warps.
+// the choice depends on how much of the GPU the tiles fill.  (Tiles are
+// counted here as kTileW x kTuneH pixels, twice the kernel's.)  Decisions are
+// shared by the contexts of a device; until a shape's two variants have been
+// timed, shapes with no more such tiles than SMs take four lanes.  Each variant
+// is timed on one launch, the two launches being successive passes of a loop,
+// so the choice is an estimate; results do not depend on it.
 static std::mutex g_tune_mutex;
 static std::map<std::tuple<int, int, int, int, int>, int> g_tune;  // (device, shape) -> choice
 
@@ -589,7 +591,7 @@ int sm_count(pt_ctx* c) {
 
 static std::tuple<int, int, int, int> tune_key(pt_ctx* c, const Params& P, int tm, int* blocks) {
     const int sms = sm_count(c);
-    *blocks = ((P.lw + ptk::kTileW - 1) / ptk::kTileW) * ((P.lh + ptk::kTileH - 1) / ptk::kTileH);
+    *blocks = ((P.lw + ptk::kTileW - 1) / ptk::kTileW) * ((P.lh + ptk::kTuneH - 1) / ptk::kTuneH);
     int cls = 0;
     while (cls < 6 && 4 * (long long)*blocks > ((long long)sms << cls)) cls++;
     return std::make_tuple(P.r, tm, P.ex.hw, cls);
@@ -666,9 +668,19 @@ cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work,
     int tm = temporal_mode(c);
     if (P.r < 2 || P.r > 4) return cudaSuccess;
     int probe = -1;
-    const int wide = kind == 0 ? propagate_variant(c, P, tm, &probe) : kind == 1 ? scatter_wide(c, P) : resid_wide(c, P);
+    int wide, tile_h;
+    if (kind == 0) {
+        wide = propagate_variant(c, P, tm, &probe);
+        tile_h = ptk::kPropH;
+    } else if (kind == 1) {
+        wide = scatter_wide(c, P);
+        tile_h = wide ? ptk::kScatHWide : ptk::kScatH;
+    } else {
+        wide = resid_wide(c, P);
+        tile_h = wide ? ptk::kResidHWide : ptk::kResidH;
+    }
     TileMaps M;
-    tile_maps(c, P, tm, kind == 2 ? (wide ? ptk::kResidHWide : ptk::kResidH) : kind == 0 ? ptk::kPropH : wide ? ptk::kScatHWide : ptk::kScatH, &M);
+    tile_maps(c, P, tm, tile_h, &M);
     if (kind == 2 && P.inc.canvas) M.on = 0;  // (its canvas tile is not a plain copy)
     int blocks = 0;
     pt_ctx::Tune* t = probe >= 0 ? &c->tune[tune_key(c, P, tm, &blocks)] : nullptr;

@@ -26,8 +26,6 @@
 
 namespace ptk {
 
-constexpr int kTileThreads = kTileW * kTileH;
-
 // Propagate's blocks per SM, which set its registers: the kernel waits for its
 // fetches, so more warps help until they spill.  Measured (summed launches):
 // without temporal terms three blocks of two candidates a lane (80 registers)
@@ -49,7 +47,7 @@ enum { TM_NONE = 0, TM_FWD = 1, TM_BWD = 2 };
 
 // The staged planes start on 128-byte boundaries (tensor copies write
 // there); a tile row is TW texels, as a tensor copy's box row is.
-template <int R, int TM, int H = kTileH>
+template <int R, int TM, int H>
 struct TileSmem {
     static constexpr int TW = kTileW + 2 * R;
     static constexpr int TH = H + 2 * R;
@@ -234,15 +232,15 @@ __device__ __forceinline__ bool block_tile(const int* list, int2* tile) {
 
 // Stages the tile (and halo) of the pixel-side inputs (`changed`: the records
 // whose canvas is formed here, a bit each by row; plain loads only) and fills the
-// state of pixel `pid` of the tile (several threads of a block of NT >
-// kTileThreads threads may ask for the same pixel).  Returns false for
+// state of pixel `pid` of the tile (several threads of the block's NT may ask
+// for the same pixel).  Returns false for
 // threads whose pixel is outside the level rectangle.  A tile whose halo lies inside the level rectangle, where
 // the clamps are no-ops, is copied by tensor copies when the maps are on
 // (one thread issues them; the texture mode's flush of subnormal input
 // colours follows in shared memory); the others load texel by texel with
 // the clamp rules.  *abort is set (for the whole block) when the copies did
 // not complete within two bounded waits; the block must then return.
-template <int R, int TM, int NT = kTileThreads, int H = kTileH>
+template <int R, int TM, int NT, int H>
 __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, TileSmem<R, TM, H>& T, int2 tile,
                                            int pid, PixT* px, bool* abort,
                                            const unsigned long long* changed = nullptr) {
@@ -283,7 +281,8 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const TileMaps& M, T
                 const float4 cv = canvas_of(P, k);
                 const int lx = q % TW - R, ly = q / TW - R;
                 T.canvas[q] = cv;
-                if (lx >= 0 && ly >= 0 && lx < kTileW && ly < H && tile.x * kTileW + lx < P.lw && tile.y * H + ly < P.lh)
+                if (lx >= 0 && ly >= 0 && lx < kTileW && ly < H && tile.x * kTileW + lx < P.lw &&
+                    tile.y * H + ly < P.lh)
                     const_cast<float4*>(P.canvas)[k] = cv;
             } else {
                 T.canvas[q] = P.canvas[k];
@@ -406,7 +405,7 @@ __device__ __forceinline__ LanePix lane_pix(const Params& P, const PixT& px) {
 }
 
 // the pixel contexts of a tile of NP pixels in shared memory
-template <int NP = kTileThreads>
+template <int NP>
 struct PixShared {
     float4 a[NP];  // sum0, sumW, prev x, prev y
     float4 b[NP];  // prev basis
@@ -423,7 +422,7 @@ __device__ __forceinline__ void put_pix(PixShared<NP>& S, int pid, const LanePix
 
 template <int R, int TM, int NP>
 __device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>& S, int2 tile, int pid) {
-    constexpr int TW = TileSmem<R, TM>::TW;
+    constexpr int TW = TileSmem<R, TM, NP / kTileW>::TW;
     LanePix q;
     const int lx = pid % kTileW, ly = pid / kTileW;
     q.x = tile.x * kTileW + lx;
@@ -458,13 +457,13 @@ __device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>&
 //  * The front pass (front_taps) takes the heaviest taps, the 3 x 3 in the
 //    middle, for all of a lane's candidates of its pixel at once: the
 //    pixel-side texels and the previous frame's samples of a tap are read
-//    once for them.  Measured over the taps that reject: 82-90 % of the
-//    candidates end here at radius 2, 66-68 % at radius 3, 46 % at radius 4.
+//    once for them.  Measured on whole syntheses: 82-89 % of the candidates end
+//    here at radius 2, 66-68 % at radius 3, 45-57 % at radius 4.
 //  * The survivors of a warp are packed into a queue of its own (WarpQueue),
 //    from which groups of eight lanes take one candidate each (eval_queue):
 //    eight further taps at a time in the order of their weight, the bound
 //    tested after each eight.  Every tap's value is kept, so that a candidate
-//    that no bound rejects (5-8 %) has its energy summed from them in the
+//    that no bound rejects (5-9 %) has its energy summed from them in the
 //    reference's order: no tap is fetched again for the exact sum.
 // Before this, each candidate was summed in the reference's order from the
 // first column on, whose taps are the lightest, and left at the threshold:
@@ -472,9 +471,10 @@ __device__ __forceinline__ LanePix get_pix(const Params& P, const PixShared<NP>&
 // 12.0 / 24.6), each with its own read of the pixel side.  Measured, summed
 // launches: propagate of a 1024x1024 still (radius 2) 21.5 -> 11.6 ms, of two
 // 1080p frames (radius 3) 288 -> 167 ms, of a 128x128 still 5.5 -> 2.5 ms.
-// What bounds it now: the texture unit's share of its peak fell from 74 to
-// 27 % while the fetches fell 2.4 times, and warps wait for the fetches of one
-// tap at a time (5.3 of 10.4 cycles per instruction); hence as many warps as
+// What bounds it now (launches of the finest level, three in a row): warps wait
+// for the fetches of one tap at a time, 4.8 of 10.2 cycles an instruction on a
+// 1080p level and 6.3 of 11.8 on a 1024x1024 one, with the texture unit's data
+// pipe at 33-45 and 26-40 % of its peak (74 % before); hence as many warps as
 // the registers allow (PropShape).  Groups of 4 lanes measured the same, of 16
 // 7 % slower; a front of 5 taps 1-7 % slower than 9.
 // ---------------------------------------------------------------------------
@@ -1009,7 +1009,8 @@ __global__ void __launch_bounds__(kTileW * H * 4 / CPL, PropShape<CPL, TM, HW>::
                            __float_as_uint(c[h].y) == __float_as_uint(c[i].y) &&
                            __float_as_uint(pc[h].theta) == __float_as_uint(pc[i].theta) && c[h].layer == c[i].layer;
                 if (!((skip >> i) & 1) && !dup) {
-                    bool ok = !culls || !(ex_texel_dt(ex_mode<HW>(P.ex), (int)c[i].x, (int)c[i].y, c[i].layer) > P.exCull);
+                    bool ok = !culls ||
+                              !(ex_texel_dt(ex_mode<HW>(P.ex), (int)c[i].x, (int)c[i].y, c[i].layer) > P.exCull);
                     if (ok && !opaque && ia > kAlphaThreshold)
                         ok = !(ex_sample_out_alpha(ex_mode<HW>(P.ex), c[i].x, c[i].y, c[i].layer) < kAlphaThreshold);
                     if (ok) {

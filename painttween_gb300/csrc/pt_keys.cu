@@ -339,7 +339,8 @@ namespace pt {
 
 cudaError_t launch_propagate_keys(const Params& P, PatchPlanes work, int jump, int key, const KeyView& K,
                                   cudaStream_t s) {
-    ptk::k_propagate_keys<<<dim3((P.lw + ptk::kDirW - 1) / ptk::kDirW, (P.lh + ptk::kDirH - 1) / ptk::kDirH), ptk::kCoopThreads, 0, s>>>(P, work, jump, key, K);
+    const dim3 g((P.lw + ptk::kDirW - 1) / ptk::kDirW, (P.lh + ptk::kDirH - 1) / ptk::kDirH);
+    ptk::k_propagate_keys<<<g, ptk::kCoopThreads, 0, s>>>(P, work, jump, key, K);
     KEY_LAUNCH_CHECK();
 }
 cudaError_t launch_scatter_keys(const Params& P, PatchPlanes work, int write_all, int key, const KeyView& K,

@@ -12,7 +12,7 @@ namespace ptk {
 
 constexpr int kMaxRadius = 15;  // taps per axis <= 31
 constexpr int kTileW = 32;      // pixel tile of the tiled kernels
-constexpr int kTileH = 8;
+constexpr int kTuneH = 8;       // rows of the tiles that propagate's autotuner counts
 constexpr int kPropH = 4;       // tile height of propagate
 constexpr int kScatH = 4;       // of scatter with two lanes per pixel
 constexpr int kScatHWide = 2;   // and with four

@@ -117,6 +117,7 @@ class TexSynth:
         self._check(lib().pt_set_tiled_kernels(self.h, int(on)), "pt_set_tiled_kernels")
 
     def set_propagate_lanes(self, warps_per_row):
+        """1: two lanes a pixel, 2: four, 0: the autotuner's choice."""
         self._check(lib().pt_set_propagate_lanes(self.h, int(warps_per_row)), "pt_set_propagate_lanes")
 
     def set_tma_staging(self, on):
