@@ -344,7 +344,10 @@ static pt_status profiled(pt_ctx* c, int kernel, Params& P, F&& launch) {
         const bool dependent = c->chained;
         c->chained = false;
         const cudaError_t e = launch(P, dependent);
-        if (e != cudaSuccess) return fail(c, PT_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            c->chained = false;
+            return fail(c, PT_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+        }
         c->launches++;
         return PT_OK;
     };
