@@ -693,7 +693,6 @@ cudaError_t launch_tiled(pt_ctx* c, int kind, const Params& P, PatchPlanes work,
         default: e = pt::launch_tiled_4(kind, tm, P, M, work, arg, pass_id, out, wide, dependent, c->stream); break;
     }
     if (t) cudaEventRecord(t->ev[2 * probe + 1], c->stream);
-    c->chained = true;
     return e;
 }
 
@@ -746,7 +745,6 @@ pt_status do_sync(pt_ctx* c, int level, int flags) {
         return st;
     }
     TRY(profiled(c, PT_KERNEL_CANVAS, P, [&](const Params& Q, bool dependent) {
-        c->chained = true;
         return pt::launch_canvas(Q, c->canvas, dependent, c->stream);
     }));
     if (!(flags & PT_DONT_UPDATE_RESIDUAL)) TRY(do_residual(c, level));

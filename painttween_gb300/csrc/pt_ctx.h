@@ -245,11 +245,12 @@ struct pt_ctx {
     int inc_tiles = 0;      // 0: none, 1: the residual's, 2: all
     int inc_kind = 0;       // the pass runs propagate (0) or scatter (1)
     int inc_canvas = 0;     // the residual kernel writes the canvas
-    // The stream's last work is a launch of a kernel that begins with
-    // pdl_start; anything else put on the stream (CU, LN, dalloc) ends the
-    // chain.  Only then is the next such kernel a dependent launch: all that
-    // the chain's kernels read and do not write themselves was complete
-    // before its first one started.
+    // The stream's last work is a propagate, scatter, residual or canvas
+    // launch; anything else put on the stream (CU, LN, dalloc) ends the chain.
+    // Only then is the next of them that begins with pdl_start a dependent
+    // launch: all that the chain's kernels read and do not write themselves
+    // was complete before its first one started.  (The generic kernels of a
+    // chain are plain launches, which wait for all before them.)
     bool chained = false;
     int inc_fill = 0;       // the next residual computes and stores every tap value
     float* tap_cache = nullptr;  // per-tap residual values, (2r+1)^2 planes
@@ -335,8 +336,8 @@ static void dfree_t(pt_ctx* c, T*& p) {
     dfree(c, (void*)p);
     p = nullptr;
 }
-// launch(P, dependent): a launch of a kernel that begins with pdl_start sets
-// pt_ctx::chained
+// launch(P, dependent): dependent, if the kernel begins with pdl_start
+// (pt_ctx::chained)
 template <class F>
 static pt_status profiled(pt_ctx* c, int kernel, Params& P, F&& launch) {
     if (c->profiling & PT_PROFILE_COUNTERS) P.counters = c->counters + 3 * kernel;
@@ -344,10 +345,8 @@ static pt_status profiled(pt_ctx* c, int kernel, Params& P, F&& launch) {
         const bool dependent = c->chained;
         c->chained = false;
         const cudaError_t e = launch(P, dependent);
-        if (e != cudaSuccess) {
-            c->chained = false;
-            return fail(c, PT_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
-        }
+        if (e != cudaSuccess) return fail(c, PT_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+        c->chained = true;
         c->launches++;
         return PT_OK;
     };

@@ -27,8 +27,8 @@ inline void gaussian_weights(int r, bool normalize, float* w) {
 #ifdef __CUDACC__
 // With `dependent`, a launch whose blocks may start before the stream's
 // previous kernel has ended; the kernel calls pdl_start before it touches
-// global memory, and so does the previous one (pt_ctx::chained).  Measured
-// on whole syntheses: 128x128 still 5.38 -> 5.00 ms, four 512x512 frames 87.7
+// global memory, and the previous one is of the same chain (pt_ctx::chained).
+// Measured on whole syntheses: 128x128 still 5.38 -> 5.00 ms, four 512x512 frames 87.7
 // -> 81.6 ms.  Larger grids than these hide a launch behind the last blocks of
 // the one before anyway, and the blocks that wait take places from them: with
 // all launches dependent two 1080p frames took 257 ms against 251 with none
