@@ -28,11 +28,11 @@ inline void gaussian_weights(int r, bool normalize, float* w) {
 // With `dependent`, a launch whose blocks may start before the stream's
 // previous kernel has ended; the kernel calls pdl_start before it touches
 // global memory, and the previous one is of the same chain (pt_ctx::chained).
-// Measured on whole syntheses: 128x128 still 5.38 -> 5.00 ms, four 512x512 frames 87.7
-// -> 81.6 ms.  Larger grids than these hide a launch behind the last blocks of
-// the one before anyway, and the blocks that wait take places from them: with
-// all launches dependent two 1080p frames took 257 ms against 251 with none
-// and 248 with this limit.
+// Measured on whole syntheses: 128x128 still 5.38 -> 5.00 ms, four 512x512
+// frames 87.7 -> 81.6 ms.  Larger grids than these hide a launch behind the
+// last blocks of the one before anyway, and the blocks that wait take places
+// from them: with all launches dependent two 1080p frames took 257 ms against
+// 251 with none and 248 with this limit.
 constexpr size_t kDependentBlocks = 3000;
 template <class... K, class... A>
 inline cudaError_t launch_dependent(bool dependent, void (*kernel)(K...), dim3 g, dim3 b, size_t smem, cudaStream_t s,
